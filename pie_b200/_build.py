@@ -27,20 +27,20 @@ OUT = ROOT / "_C"
 KERNEL_LIB = OUT / "libpie_kernels.so"
 
 # sources whose kernels a latent-attention model launches
-LATENT_SOURCES = ("attention_tc", "elementwise", "gemm2_tcgen05", "gemm_tcgen05", "latent",
+LATENT_SOURCES = ("attention_tc", "elementwise", "gemm2_tcgen05", "gemm_skinny", "gemm_tcgen05", "latent",
                   "latent_attn", "latent_attn_tc", "sampling")
 
 # sources whose kernels sandwich-normed blocks with linear attention launch
-SANDWICH_SOURCES = ("attention_bias", "elementwise", "gdn", "gemm2_tcgen05", "gemm_tcgen05", "latent", "latent_attn", "linear_attn", "moe",
-                    "sampling")
+SANDWICH_SOURCES = ("attention_bias", "elementwise", "gdn", "gemm2_tcgen05", "gemm_skinny", "gemm_tcgen05", "latent",
+                    "latent_attn", "linear_attn", "moe", "sampling")
 
 # sources whose kernels blocks normed on the way out (grouped and latent attention, matrix memory) launch
-POST_NORM_SOURCES = ("attention", "attention_gqa", "attention_tc", "elementwise", "gdn", "gemm2_tcgen05", "gemm_tcgen05", "latent",
-                     "latent_attn", "latent_attn_tc", "linear_attn", "moe", "sampling")
+POST_NORM_SOURCES = ("attention", "attention_gqa", "attention_tc", "elementwise", "gdn", "gemm2_tcgen05", "gemm_skinny",
+                     "gemm_tcgen05", "latent", "latent_attn", "latent_attn_tc", "linear_attn", "moe", "sampling")
 
 # sources whose kernels blocks that read the stream through a layer norm and a convolution launch
-LAYER_NORM_SOURCES = ("attention_gqa", "attention_pool", "attention_tc", "delta_rule", "elementwise", "gdn", "gemm2_tcgen05", "gemm_tcgen05",
-                      "latent", "latent_attn", "linear_attn", "sampling", "stream_conv")
+LAYER_NORM_SOURCES = ("attention_gqa", "attention_pool", "attention_tc", "delta_rule", "elementwise", "gdn", "gemm2_tcgen05",
+                      "gemm_skinny", "gemm_tcgen05", "latent", "latent_attn", "linear_attn", "sampling", "stream_conv")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

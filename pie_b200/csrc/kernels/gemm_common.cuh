@@ -18,14 +18,6 @@ enum GemmEpilogue : int {
     EPI_STREAM = 5,    // out32 = res32 + acc + bias: a 32-bit residual stream; C = the same in bf16
     EPI_CLAMP_GLU = 6, // as EPI_SWIGLU with g = min(gate, limit), u = clamp(up, +-limit): g * sigmoid(1.702 g) * (u + 1)
     EPI_GEGLU = 7,     // as EPI_SWIGLU with the tanh form of GELU on the gate
-    // Swapped operands (small batches): the kernel computes C^T = W * A^T, so its rows are output
-    // features and its columns tokens; these epilogues write the tile back transposed. EPI_STORE_T is the first of them.
-    EPI_STORE_T = 8,
-    EPI_RESIDUAL_T = 9,
-    EPI_SWIGLU_T = 10,
-    EPI_XIELU_T = 11,
-    EPI_STREAM_T = 12,
-    EPI_GEGLU_T = 13,
 };
 
 // Operands of the epilogues with a bias. xIELU(z) = a z^2 + z / 2 for z > 0, b (e^z - 1 - z) + z / 2 below, with
@@ -47,7 +39,7 @@ __device__ __forceinline__ float glu_value(float g, float u, float limit) {
         return g / (1.f + __expf(-1.702f * g)) * (u + 1.f);
     }
     // (1 + tanh(y)) / 2 = sigmoid(2 y)
-    if (EPI == EPI_GEGLU || EPI == EPI_GEGLU_T) return g / (1.f + __expf(-1.5957691216057308f * (g + 0.044715f * g * g * g))) * u;
+    if (EPI == EPI_GEGLU) return g / (1.f + __expf(-1.5957691216057308f * (g + 0.044715f * g * g * g))) * u;
     return g / (1.f + __expf(-g)) * u;
 }
 
@@ -336,85 +328,6 @@ __device__ __forceinline__ void epilogue_store_64(const uint32_t (&v0)[32], cons
             dst = C + (size_t)row * ldc + col;
         }
         *reinterpret_cast<bf16x8*>(dst) = *slot(r, c);
-    }
-    __syncwarp();
-}
-
-// Transposed epilogue of the swapped-operand launch: thread `lane` holds output feature
-// (feat0 + lane), v0 / v1 its values for tokens tok0..+31 / +32..+63. The output is C[token][feature].
-// Values are staged as bf16 in the warp's 4 KB tile as [64 tokens][32 features] (64 B per token; for
-// SwiGLU [64 tokens][16 outputs]) and leave in 16-byte stores, 8 (16) token rows per warp store.
-//   F       : number of output features of the GEMM (rows of the swapped problem)
-//   tok_end : tokens at or past tok_end are not stored
-template <int EPI>
-__device__ __forceinline__ void epilogue_store_64_t(const uint32_t (&v0)[32], const uint32_t (&v1)[32],
-                                                    uint8_t* stage, int feat0, int tok0, int F, int tok_end,
-                                                    bf16* __restrict__ C, int ldc, const bf16* __restrict__ R,
-                                                    int ldr, const EpiArgs& ex = EpiArgs(), const XieluCoef* act = nullptr) {
-    const int lane = threadIdx.x & 31;
-    bf16* st = reinterpret_cast<bf16*>(stage);
-    const int feat = feat0 + lane;
-    if (EPI == EPI_SWIGLU_T || EPI == EPI_GEGLU_T) {
-        // even lanes hold gate_j, odd lanes up_j of output j = feat / 2
-#pragma unroll
-        for (int t = 0; t < 64; ++t) {
-            const float mine = __uint_as_float(t < 32 ? v0[t] : v1[t - 32]);
-            const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            if (!(lane & 1)) st[t * 16 + (lane >> 1)] = __float2bfloat16(glu_value<EPI>(mine, other, 0.f));
-        }
-        __syncwarp();
-        const int oc0 = feat0 >> 1;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = i * 16 + (lane >> 1), c = lane & 1;
-            const int tok = tok0 + t;
-            if (tok < tok_end && 2 * (oc0 + c * 8) < F)
-                *reinterpret_cast<bf16x8*>(C + (size_t)tok * ldc + oc0 + c * 8) = *reinterpret_cast<const bf16x8*>(st + t * 16 + c * 8);
-        }
-        __syncwarp();
-        return;
-    }
-    float bias = 0.f;
-    if constexpr (EPI == EPI_XIELU_T || EPI == EPI_STREAM_T) bias = ex.bias && feat < F ? __bfloat162float(ex.bias[feat]) : 0.f;
-    if constexpr (EPI == EPI_STREAM_T) {
-        // the warp's 32 features of a token are 128 bytes of its stream row; all loads of a batch leave before its stores,
-        // which may be to the same addresses
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            float x[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int tok = tok0 + b * 16 + i;
-                x[i] = tok < tok_end && feat < F ? ex.res32[(size_t)tok * ex.ld32 + feat] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int t = b * 16 + i, tok = tok0 + t;
-                x[i] += __uint_as_float(t < 32 ? v0[t] : v1[t - 32]) + bias;
-                if (tok < tok_end && feat < F) ex.out32[(size_t)tok * ex.ld32 + feat] = x[i];
-                st[t * 32 + lane] = __float2bfloat16(x[i]);
-            }
-        }
-        if (!C) return;
-    }
-#pragma unroll
-    for (int t = 0; t < 64; ++t) {
-        if constexpr (EPI == EPI_STREAM_T) break;
-        float o = __uint_as_float(t < 32 ? v0[t] : v1[t - 32]);
-        if constexpr (EPI == EPI_XIELU_T) o = (*act)(o + bias);
-        if (EPI == EPI_RESIDUAL_T) {
-            const int tok = tok0 + t;
-            if (tok < tok_end && feat < F) o += __bfloat162float(R[(size_t)tok * ldr + feat]);
-        }
-        st[t * 32 + lane] = __float2bfloat16(o);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = i * 8 + (lane >> 2), c = lane & 3;
-        const int tok = tok0 + t;
-        if (tok < tok_end && feat0 + c * 8 < F)
-            *reinterpret_cast<bf16x8*>(C + (size_t)tok * ldc + feat0 + c * 8) = *reinterpret_cast<const bf16x8*>(st + t * 32 + c * 8);
     }
     __syncwarp();
 }

@@ -45,6 +45,10 @@ struct GemmCfg {
 // BN is the widest tile the instantiation has room for (ring slots, TMEM columns); the launch
 // picks the actual width bn <= BN, a multiple of 16, so that the tile count fills the machine's
 // waves; the W tensor map's box has bn rows.
+// bm: rows of A in a tile and of its tensor map's box (at most 128). The box ends with the batch where it can: a row past
+// the end costs the TMA more than one inside it (it is filled with zeros row by row). With 128-row boxes a 28672 x 4096
+// product took 71 us for 1 row against 50 us for 128; with boxes of the batch's rows 47 us. Rows of a tile past its box are
+// whatever shared memory held; an accumulator row depends on its own operand row alone, and these are not stored.
 // GROUPED: mixture-of-experts form. A holds token rows sorted by expert in 128-row tiles,
 // tile_expert[m_tile] names the expert whose weights ([E*N, K] under tma_b) the tile multiplies,
 // or -1 for an unused tile, which every role skips. Whole-tile scheduling only.
@@ -53,10 +57,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, OCC)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  bf16* __restrict__ C, const bf16* __restrict__ R, int M, int N, int K, int ldc,
                  int ldr, int* status, const __grid_constant__ TpArgs tp, const StreamKArgs sk,
-                 const int* __restrict__ tile_expert, int bn, const __grid_constant__ EpiArgs ex) {
+                 const int* __restrict__ tile_expert, int bn, int bm, const __grid_constant__ EpiArgs ex) {
     using Cfg = GemmCfg<BN, OCC>;
     constexpr int STAGES = Cfg::STAGES;
-    constexpr bool SWAPPED = EPI >= EPI_STORE_T;   // tma_a walks the weights, tma_b the activation
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t tiles = (raw + 1023u) & ~1023u;
@@ -70,10 +73,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * STAGES + 4);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_m = (M + GEMM_BM - 1) / GEMM_BM;
+    const int tiles_m = (M + bm - 1) / bm;
     const int tiles_n = (N + bn - 1) / bn;
     const int num_tiles = tiles_m * tiles_n;
-    const uint32_t stage_tx = Cfg::A_BYTES + (uint32_t)bn * (GEMM_KSTEP * 2);
+    const uint32_t stage_tx = (uint32_t)(bm + bn) * (GEMM_KSTEP * 2);
     const int num_kb = (K + GEMM_KSTEP - 1) / GEMM_KSTEP;
 
     if (threadIdx.x == 0) {
@@ -117,17 +120,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             auto resolve = [&]() {
                 pdl_wait();
                 for (int j = 0; j < pending && ok; ++j) {
-                    if (tp.gated) ok = ag_gate_wait_rows(tp, status, q_row[j], SWAPPED ? bn : GEMM_BM, seen);
+                    if (tp.gated) ok = ag_gate_wait_rows(tp, status, q_row[j], bm, seen);
                     if (!ok) break;
 #pragma unroll
-                    for (int u = 0; u < Cfg::KSUB; ++u) {
-                        if (SWAPPED)
-                            tma_load_2d(tiles + q_stage[j] * Cfg::STAGE_BYTES + Cfg::A_BYTES + u * Cfg::B_SUB, &tma_b,
-                                        full_bar(q_stage[j]), q_kb[j] * GEMM_KSTEP + u * GEMM_BK, q_row[j]);
-                        else
-                            tma_load_2d(tiles + q_stage[j] * Cfg::STAGE_BYTES + u * Cfg::A_SUB, &tma_a, full_bar(q_stage[j]),
-                                        q_kb[j] * GEMM_KSTEP + u * GEMM_BK, q_row[j]);
-                    }
+                    for (int u = 0; u < Cfg::KSUB; ++u)
+                        tma_load_2d(tiles + q_stage[j] * Cfg::STAGE_BYTES + u * Cfg::A_SUB, &tma_a, full_bar(q_stage[j]),
+                                    q_kb[j] * GEMM_KSTEP + u * GEMM_BK, q_row[j]);
                 }
                 pending = 0;
                 dep_ready = true;
@@ -154,36 +152,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
                     const uint32_t a_dst = tiles + s * Cfg::STAGE_BYTES;
                     if (PIE_DIAG(sk.dbg & 6)) {   // diagnostics: 2 = no activation loads, 4 = no weight loads, 6 = neither
-                        const uint32_t tx = ((sk.dbg & 2) ? 0u : Cfg::A_BYTES) + ((sk.dbg & 4) ? 0u : (uint32_t)bn * (GEMM_KSTEP * 2));
+                        const uint32_t tx = (uint32_t)(((sk.dbg & 2) ? 0 : bm) + ((sk.dbg & 4) ? 0 : bn)) * (GEMM_KSTEP * 2);
                         mbar_arrive_expect_tx(full_bar(s), tx);
                         for (int u = 0; u < Cfg::KSUB; ++u) {
                             if (!(sk.dbg & 4))
                                 tma_load_2d(a_dst + Cfg::A_BYTES + u * Cfg::B_SUB, &tma_b, full_bar(s), kb * GEMM_KSTEP + u * GEMM_BK, b_row);
                             if (!(sk.dbg & 2))
-                                tma_load_2d(a_dst + u * Cfg::A_SUB, &tma_a, full_bar(s), kb * GEMM_KSTEP + u * GEMM_BK, m_blk * GEMM_BM);
+                                tma_load_2d(a_dst + u * Cfg::A_SUB, &tma_a, full_bar(s), kb * GEMM_KSTEP + u * GEMM_BK, m_blk * bm);
                         }
                         continue;
                     }
                     if (dep_ready && tp.gated &&
-                        !ag_gate_wait_rows(tp, status, SWAPPED ? b_row : m_blk * GEMM_BM, SWAPPED ? bn : GEMM_BM, seen)) {
+                        !ag_gate_wait_rows(tp, status, m_blk * bm, bm, seen)) {
                         ok = false;
                         break;
                     }
                     mbar_arrive_expect_tx(full_bar(s), stage_tx);
-                    // the operand that holds the weights goes first; the activation operand (tma_a, or
-                    // tma_b of a swapped launch) waits for its producer
-                    if (!SWAPPED || dep_ready) {
+                    // the weights go first; the activation waits for its producer
+#pragma unroll
+                    for (int u = 0; u < Cfg::KSUB; ++u)
+                        tma_load_2d(a_dst + Cfg::A_BYTES + u * Cfg::B_SUB, &tma_b, full_bar(s), kb * GEMM_KSTEP + u * GEMM_BK, b_row);
+                    if (dep_ready) {
 #pragma unroll
                         for (int u = 0; u < Cfg::KSUB; ++u)
-                            tma_load_2d(a_dst + Cfg::A_BYTES + u * Cfg::B_SUB, &tma_b, full_bar(s), kb * GEMM_KSTEP + u * GEMM_BK, b_row);
-                    }
-                    if (SWAPPED || dep_ready) {
-#pragma unroll
-                        for (int u = 0; u < Cfg::KSUB; ++u)
-                            tma_load_2d(a_dst + u * Cfg::A_SUB, &tma_a, full_bar(s), kb * GEMM_KSTEP + u * GEMM_BK, m_blk * GEMM_BM);
+                            tma_load_2d(a_dst + u * Cfg::A_SUB, &tma_a, full_bar(s), kb * GEMM_KSTEP + u * GEMM_BK, m_blk * bm);
                     }
                     if (!dep_ready) {
-                        q_kb[pending] = kb; q_row[pending] = SWAPPED ? b_row : m_blk * GEMM_BM; q_stage[pending] = s;
+                        q_kb[pending] = kb; q_row[pending] = m_blk * bm; q_stage[pending] = s;
                         ++pending;
                     }
                 }
@@ -241,7 +236,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         SegmentWalk walk(sk.enabled != 0, num_tiles, num_kb, blockIdx.x, gridDim.x);
         Segment seg;
         const long long total_units = (long long)num_tiles * num_kb;
-        const XieluCoef act((EPI == EPI_XIELU || EPI == EPI_XIELU_T) ? ex.act : nullptr);
+        const XieluCoef act(EPI == EPI_XIELU ? ex.act : nullptr);
         for (; walk.next(seg); ++tcount) {
             const int m_blk = seg.tile % tiles_m, n_blk = seg.tile / tiles_m;
             if (GROUPED && tile_expert[m_blk] < 0) { --tcount; continue; }
@@ -250,11 +245,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             if (!__all_sync(0xffffffffu, got)) break;
             if (warp == 2 && lane == 0) trace_stamp(sk.trace, tcount == 0 ? 4 : 5);
             tc_fence_after();
-            const int row = m_blk * GEMM_BM + q * 32 + lane;
+            const int row_end = min(M, (m_blk + 1) * bm);
             const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
             const bool partial = seg.kb0 != 0 || seg.kb1 != num_kb;
-            // a 32-row quarter that lies wholly past M has nothing to park, reduce or store
-            const bool rows_valid = m_blk * GEMM_BM + q * 32 < M;
+            // a 32-row quarter that lies wholly past the tile's rows has nothing to park, reduce or store
+            const bool rows_valid = m_blk * bm + q * 32 < row_end;
             bool finalise = rows_valid;
             int c_first = 0, c_last = -1;
             if (partial && rows_valid) {
@@ -305,7 +300,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                                                   (size_t)q * (32 * BN / 4) + (size_t)c * 16 * 32 + lane;
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
-                                const float4 a4 = __ldcg(other + j * 32), b4 = __ldcg(other + (8 + j) * 32);
+                                const float4 a4 = __ldcg(other + j * 32);
+                                const float4 b4 = c * 64 + 32 < bn ? __ldcg(other + (8 + j) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
                                 v0[4 * j] = __float_as_uint(__uint_as_float(v0[4 * j]) + a4.x);
                                 v0[4 * j + 1] = __float_as_uint(__uint_as_float(v0[4 * j + 1]) + a4.y);
                                 v0[4 * j + 2] = __float_as_uint(__uint_as_float(v0[4 * j + 2]) + a4.z);
@@ -317,19 +313,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                             }
                         }
                     }
-                    if constexpr (EPI >= EPI_STORE_T)
-                        epilogue_store_64_t<EPI>(v0, v1, stage, m_blk * GEMM_BM + q * 32, n_blk * bn + c * 64, M,
-                                                 min(N, (n_blk + 1) * bn), C, ldc, R, ldr, ex, &act);
-                    else
-                        epilogue_store_64<EPI>(v0, v1, stage, m_blk * GEMM_BM + q * 32, n_blk * bn + c * 64, M, N, C,
-                                               ldc, R, ldr, tp, min(N, (n_blk + 1) * bn), ex, &act);
+                    epilogue_store_64<EPI>(v0, v1, stage, m_blk * bm + q * 32, n_blk * bn + c * 64, row_end, N, C,
+                                           ldc, R, ldr, tp, min(N, (n_blk + 1) * bn), ex, &act);
                 }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty_bar(acc));
             // one arrival per (tile, quarter): the finaliser's for a valid quarter, the owner of the
-            // tile's last k-block for a quarter past M
+            // tile's last k-block for a quarter past the tile's rows
             if (EPI == EPI_RS && (rows_valid ? finalise : seg.kb1 == num_kb)) {
                 // publish: this warp's rows of the tile are in the owners' buffers
                 __threadfence_system();
@@ -440,10 +432,10 @@ PIE_API int pie_set_pdl(int enabled) { g_pie_pdl = enabled; return 0; }
 static int g_gemm_pairs = 1;
 PIE_API int pie_gemm_set_pairs(int enabled) { g_gemm_pairs = enabled; return 0; }
 
-// Batches of up to this many rows run with swapped operands (0: never): the weight rows take the
-// 128-row side of the MMA and the batch the narrow side, so each CTA streams a [128 x K-slice]
-// block of the weights against the whole (small) activation instead of re-reading the activation
-// once per narrow weight tile.
+// Batches of up to this many rows take the kernel for small batches (0: never; 1000: whatever the shape), where N >= 128 and
+// K >= 512: below, a weight tile's worth of set-up outweighs the streaming. Measured, 1 / 64 / 128 rows: 6144 x 4096 12 / 14 /
+// 17 us against 21 / 22 / 22 us on whole tiles here, 4096 x 14336 22 / 28 / 33 us against 46 / 49 / 53 us, 28672 x 4096
+// 37 / 47 / 55 us against 48 / 50 / 51 us; the last column is the price of one summation order for all batches of a tile.
 static int g_gemm_swap_max_m = 128;
 PIE_API int pie_gemm_set_swap(int max_m) { g_gemm_swap_max_m = max_m; return 0; }
 
@@ -451,6 +443,9 @@ int pie_gemm2_dispatch(const void* A, const void* W, void* C, const void* R, int
                        int ldw, int ldc, int ldr, int epilogue, int* status, int num_sms, cudaStream_t st,
                        const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, int* handled,
                        const EpiArgs& ex = EpiArgs());
+
+int pie_gemm_skinny(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda, int ldw, int ldc, int ldr,
+                    int epilogue, int* status, int num_sms, cudaStream_t st, const EpiArgs& ex);
 
 struct GemmPlan {
     int bn;        // tile width of the launch (multiple of 16)
@@ -543,9 +538,16 @@ PIE_API int pie_gemm_plan(int M, int N, int K, int num_sms, int with_workspace, 
     return 0;
 }
 
+// Rows of a tile: the batch spread evenly over its 128-row tiles, whole where one tile holds it.
+static int tile_rows(int M) {
+    if (M <= GEMM_BM) return M;
+    const int tiles = (M + GEMM_BM - 1) / GEMM_BM;
+    return std::min(GEMM_BM, ((M + tiles - 1) / tiles + 7) / 8 * 8);
+}
+
 template <int BN, int EPI>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, void* C, const void* R, int M,
-                       int N, int K, int ldc, int ldr, int* status, const GemmPlan& plan,
+                       int N, int K, int ldc, int ldr, int* status, const GemmPlan& plan, int bm,
                        const GemmWorkspace& w, cudaStream_t st, const TpArgs& tp = TpArgs{}, const EpiArgs& ex = EpiArgs()) {
     using Cfg = GemmCfg<BN>;
     auto kern = gemm_bf16_kernel<BN, EPI>;
@@ -554,7 +556,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, void* C, co
     if (e != cudaSuccess) return (int)e;
     StreamKArgs sk{w.ws, w.cnt, plan.streamk, g_gemm_dbg, g_gemm_trace};
     e = launch_pdl(kern, dim3(plan.grid), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, ta, tb, (bf16*)C, (const bf16*)R,
-                   M, N, K, ldc, ldr, status, tp, sk, (const int*)nullptr, plan.bn, ex);
+                   M, N, K, ldc, ldr, status, tp, sk, (const int*)nullptr, plan.bn, bm, ex);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
@@ -582,52 +584,24 @@ static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M
                                           nullptr, w.ws, w.ws_floats, w.cnt, w.cnt_ints, &handled, ex);
         if (handled || rc) return rc;
     }
-    if (force_bn == 0 && M <= (g_gemm_swap_max_m >= 1000 ? 128 : g_gemm_swap_max_m) && M <= 128 && N >= 128 && K >= 512) {
-        // C^T = W * A^T: rows of the launch are output features, its one column tile the batch
-        const int bt = M <= 64 ? 64 : 128;
-        const GemmPlan plan = plan_gemm(N, bt, K, num_sms, bt, w, true);
-        // Measured (Llama-3.1-8B shapes, 8 to 128 rows): the swapped launch wins where its 128-row
-        // feature tiles cannot fill the machine by themselves and K is long enough that each CTA of
-        // the K split keeps 20 or more k-blocks (qkv 31 -> 27 us, down 59 -> 47 us at 64 rows); with
-        // shorter splits the fix-up of the partial tiles costs more than the narrow direct tiles. Up to 128 rows the
-        // decode step still gains (96 requests 8.41 -> 7.96 ms, 128 requests 9.20 -> 8.99 ms).
-        const long s_tiles = (N + GEMM_BM - 1) / GEMM_BM, s_kb = (K + GEMM_KSTEP - 1) / GEMM_KSTEP;
-        const bool take = g_gemm_swap_max_m >= 1000 ||
-                          (plan.streamk && s_tiles <= num_sms && s_tiles * s_kb >= 20L * plan.grid);
-        CUtensorMap ta, tb;
-        if (!take) goto direct;
-        if (pie_make_tma_2d_bf16(&ta, W, N, K, ldw, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
-        if (pie_make_tma_2d_bf16(&tb, A, M, K, lda, bt) != 0) return (int)cudaErrorInvalidValue;
-#define GO_T(BN_)                                                                                   \
-    switch (epilogue) {                                                                           \
-        case EPI_STORE: return launch_gemm<BN_, EPI_STORE_T>(ta, tb, C, R, N, M, K, ldc, ldr, status, plan, w, st); \
-        case EPI_RESIDUAL: return launch_gemm<BN_, EPI_RESIDUAL_T>(ta, tb, C, R, N, M, K, ldc, ldr, status, plan, w, st); \
-        case EPI_SWIGLU: return launch_gemm<BN_, EPI_SWIGLU_T>(ta, tb, C, R, N, M, K, ldc, ldr, status, plan, w, st); \
-        case EPI_GEGLU: return launch_gemm<BN_, EPI_GEGLU_T>(ta, tb, C, R, N, M, K, ldc, ldr, status, plan, w, st); \
-        case EPI_XIELU: return launch_gemm<BN_, EPI_XIELU_T>(ta, tb, C, R, N, M, K, ldc, ldr, status, plan, w, st, TpArgs{}, ex); \
-        case EPI_STREAM: return launch_gemm<BN_, EPI_STREAM_T>(ta, tb, C, R, N, M, K, ldc, ldr, status, plan, w, st, TpArgs{}, ex); \
-        default: return (int)cudaErrorInvalidValue;                                               \
-    }
-        if (bt == 64) { GO_T(64) } else { GO_T(128) }
-#undef GO_T
-    }
-direct:
+    if (force_bn == 0 && M <= GEMM_BM && (g_gemm_swap_max_m >= 1000 || (M <= g_gemm_swap_max_m && N >= 128 && K >= 512)))
+        return pie_gemm_skinny(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, status, num_sms, st, ex);
     bool allow_sk = true;
     if (force_bn < 0) { allow_sk = false; force_bn = -force_bn == 1 ? 0 : -force_bn; }  // negative: whole-tile only
     if (force_bn > 256 || force_bn % 16) return (int)cudaErrorInvalidValue;
     const GemmPlan plan = plan_gemm(M, N, K, num_sms, force_bn, w, allow_sk);
-    const int bn = plan.bn_t();
+    const int bn = plan.bn_t(), bm = tile_rows(M);
     CUtensorMap ta, tb;
-    if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
+    if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, bm) != 0) return (int)cudaErrorInvalidValue;
     if (pie_make_tma_2d_bf16(&tb, W, N, K, ldw, plan.bn) != 0) return (int)cudaErrorInvalidValue;
 #define GO(BN_)                                                                                   \
     switch (epilogue) {                                                                           \
-        case EPI_STORE: return launch_gemm<BN_, EPI_STORE>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, w, st); \
-        case EPI_RESIDUAL: return launch_gemm<BN_, EPI_RESIDUAL>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, w, st); \
-        case EPI_SWIGLU: return launch_gemm<BN_, EPI_SWIGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, w, st); \
-        case EPI_GEGLU: return launch_gemm<BN_, EPI_GEGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, w, st); \
-        case EPI_XIELU: return launch_gemm<BN_, EPI_XIELU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, w, st, TpArgs{}, ex); \
-        case EPI_STREAM: return launch_gemm<BN_, EPI_STREAM>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, w, st, TpArgs{}, ex); \
+        case EPI_STORE: return launch_gemm<BN_, EPI_STORE>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
+        case EPI_RESIDUAL: return launch_gemm<BN_, EPI_RESIDUAL>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
+        case EPI_SWIGLU: return launch_gemm<BN_, EPI_SWIGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
+        case EPI_GEGLU: return launch_gemm<BN_, EPI_GEGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
+        case EPI_XIELU: return launch_gemm<BN_, EPI_XIELU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
+        case EPI_STREAM: return launch_gemm<BN_, EPI_STREAM>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
         default: return (int)cudaErrorInvalidValue;                                               \
     }
     if (bn == 256) { GO(256) }
@@ -706,15 +680,15 @@ PIE_API int pie_gemm_bf16_tp(const void* A, const void* W, void* C, int M, int N
     }
     if (force_bn < 0 || force_bn > 256 || force_bn % 16) return (int)cudaErrorInvalidValue;
     const GemmPlan plan = plan_gemm(M, N, K, num_sms, force_bn, w);
-    const int bn = plan.bn_t();
+    const int bn = plan.bn_t(), bm = M < GEMM_BM ? M : GEMM_BM;       // tiles of 128 rows: owners hold multiples of 32
     CUtensorMap ta, tb;
-    if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
+    if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, bm) != 0) return (int)cudaErrorInvalidValue;
     if (pie_make_tma_2d_bf16(&tb, W, N, K, ldw, plan.bn) != 0) return (int)cudaErrorInvalidValue;
 #define GO(BN_)                                                                                    \
     switch (epilogue) {                                                                            \
-        case EPI_STORE: return launch_gemm<BN_, EPI_STORE>(ta, tb, C, nullptr, M, N, K, ldc, 0, status, plan, w, st, tp);   \
-        case EPI_SWIGLU: return launch_gemm<BN_, EPI_SWIGLU>(ta, tb, C, nullptr, M, N, K, ldc, 0, status, plan, w, st, tp); \
-        case EPI_RS: return launch_gemm<BN_, EPI_RS>(ta, tb, C, nullptr, M, N, K, ldc, 0, status, plan, w, st, tp);         \
+        case EPI_STORE: return launch_gemm<BN_, EPI_STORE>(ta, tb, C, nullptr, M, N, K, ldc, 0, status, plan, bm, w, st, tp);   \
+        case EPI_SWIGLU: return launch_gemm<BN_, EPI_SWIGLU>(ta, tb, C, nullptr, M, N, K, ldc, 0, status, plan, bm, w, st, tp); \
+        case EPI_RS: return launch_gemm<BN_, EPI_RS>(ta, tb, C, nullptr, M, N, K, ldc, 0, status, plan, bm, w, st, tp);         \
         default: return (int)cudaErrorInvalidValue;                                                \
     }
     if (bn == 256) { GO(256) }
@@ -749,7 +723,7 @@ static int grouped_gemm(const void* A, const void* W, void* C, const int* tile_e
                                              (int)GemmCfg<BN_>::SMEM_BYTES);                              \
         if (e != cudaSuccess) return (int)e;                                                              \
         e = launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), GemmCfg<BN_>::SMEM_BYTES, st, ta, tb, (bf16*)C, \
-                       (const bf16*)nullptr, M, N, K, ldc, 0, status, tp, sk, tile_expert, bn, ex);    \
+                       (const bf16*)nullptr, M, N, K, ldc, 0, status, tp, sk, tile_expert, bn, GEMM_BM, ex);    \
         return (int)(e != cudaSuccess ? e : cudaGetLastError());                                          \
     }
     if (epilogue == EPI_STORE) {

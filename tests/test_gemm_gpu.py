@@ -130,3 +130,29 @@ def test_gemm_swapped_operands_small_batch(m, n, k, epi):
     check(y, ref, k)
     check(y0, ref, k)
     ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("m", [1, 3, 17, 127, 129, 130, 200, 255, 257, 300])
+@pytest.mark.parametrize("n,k,epi", [(1024, 4096, "store"), (28672, 512, "swiglu"), (1000, 520, "residual")])
+def test_gemm_tiles_of_no_more_rows_than_the_batch_has(m, n, k, epi):
+    """A tile's box ends with its rows; what shared memory holds beyond them (here infinities of the product before)
+    reaches no stored row."""
+    x, w = bf(m, k, seed=41), bf(n, k, scale=0.03, seed=42)
+    r = bf(m, n, seed=43) if epi == "residual" else None
+    e = {"store": ops.EPI_STORE, "residual": ops.EPI_RESIDUAL, "swiglu": ops.EPI_SWIGLU}[epi]
+    want = x.float() @ w.float().t()
+    if epi == "residual":
+        want = want + r.float()
+    if epi == "swiglu":
+        want = ref.swiglu_interleaved(want)
+    wild = torch.full((128, k), float("inf"), dtype=torch.bfloat16, device=DEV)
+    for swap in (0, 128, 1000):
+        ops.set_gemm_swap(swap)
+        try:
+            ops.gemm(wild, w)
+            ops.set_gemm_pairs(swap != 0)
+            y = ops.gemm(x, w, residual=r, epilogue=e)
+        finally:
+            ops.set_gemm_swap(128)
+            ops.set_gemm_pairs(True)
+        check(y, want, k)
