@@ -740,3 +740,44 @@ def test_mamba2_mixer_matches_reference_over_chunks(heads, head_dim, state, grou
         close(got.cpu(), want, 3e-2)
         assert torch.allclose(dev_cache.rec_state.cpu(), cpu_cache.rec_state, atol=2e-2, rtol=2e-2)
         assert torch.allclose(dev_cache.conv_state.cpu(), cpu_cache.conv_state, atol=1e-6)
+
+
+@pytest.mark.parametrize("vocab", [8, 4096, 4104, 32768, 151936, 151944, 800008, 1600000])
+def test_sample_over_cluster_sizes(vocab):
+    """Rows at the edges of a CTA's share and of the cluster's size, and rows too long to be kept: the drawn token's Gumbel score
+    in 64 bits is the best one's up to the error of the kernel's fast logarithms (2^-22 absolute near 1: relative to -log u),
+    filters keep to their set, and greedy is the arg-max."""
+    rows = 3
+    lg = bf(rows, vocab, scale=2.5, seed=vocab)
+    seeds = torch.arange(7, 7 + rows, dtype=torch.int64)
+    u64 = (1 << 64) - 1
+
+    def splitmix(x):
+        x = (x + 0x9E3779B97F4A7C15) & u64
+        x = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & u64
+        x = ((x ^ (x >> 27)) * 0x94D049BB133111EB) & u64
+        return x ^ (x >> 31)
+
+    idx, m32 = torch.arange(vocab, device=DEV), 0xFFFFFFFF
+    for k, p, mp in ((0, 1.0, 0.0), (5, 1.0, 0.0), (0, 0.3, 0.0), (0, 1.0, 0.2)):
+        got = ops.sample(lg, *_params(rows, 1.0, k, p, mp, seed0=7)).long()
+        for r in range(rows):
+            s = splitmix(int(seeds[r]))
+            h = ((idx + (s & m32) + 7 * 0x632BE5AB) & m32) * 0x9E3779B1 & m32 ^ (s >> 32)
+            h = (h ^ (h >> 16)) * 0x85EBCA6B & m32
+            h = (h ^ (h >> 13)) * 0xC2B2AE35 & m32
+            u = (((h ^ (h >> 16)) >> 8).float() + 0.5).mul(2.0 ** -24).double()
+            x = lg[r].double()
+            keep = ref.kept_set(lg[r], 1.0, k, p, mp)
+            score = torch.where(keep, x - x.max() - torch.log(-torch.log(u)), -math.inf)
+            assert bool(keep[got[r]])
+            err = 1e-4 + 4e-7 / -math.log(min(float(u[got[r]]), 1 - 2.0 ** -25)) + 4e-7 / -math.log(min(float(u[score.argmax()]), 1 - 2.0 ** -25))
+            assert float(score[got[r]]) >= float(score.max()) - err
+    got = ops.sample(lg, *_params(rows, 0.0, 0, 1.0, 0.0))
+    first = torch.stack([(lg[r] == lg[r].max()).nonzero()[0, 0] for r in range(rows)])
+    assert torch.equal(got.long(), first)
+    # nothing but -inf, and rows of the lowest finite value
+    lg[0] = -math.inf
+    lg[1] = torch.finfo(torch.bfloat16).min
+    got = ops.sample(lg, *_params(rows, 1.0, 0, 0.9, 0.0))
+    assert int(got[0]) == 0 and 0 <= int(got[1]) < vocab
