@@ -139,27 +139,6 @@ struct DeltaSmem {
     float2 dots[2][DELTA_CT];              // r . (a * u), r . k
 };
 
-// Sums of NV values over LPC lanes: halves change hands until a lane is left with one value (of index `which`, the lane's own
-// number in bits from the top); further lanes then add up copies of it.
-template <int NV, int LPC>
-__device__ __forceinline__ float halving_sum(float (&x)[NV], int g) {
-    if constexpr (NV == 1) {
-        float y = x[0];
-#pragma unroll
-        for (int o = LPC / 2; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-        return y;
-    } else {
-        const bool up = g & (LPC / 2);
-        float y[NV / 2];
-#pragma unroll
-        for (int i = 0; i < NV / 2; ++i) {
-            const float keep = up ? x[i + NV / 2] : x[i], give = up ? x[i] : x[i + NV / 2];
-            y[i] = keep + __shfl_xor_sync(0xffffffffu, give, LPC / 2);
-        }
-        return halving_sum<NV / 2, LPC / 2>(y, g);
-    }
-}
-
 // Lane g of a column group holds the rows 4 (g + LPC i) + e.
 template <typename T, int R, int LPC, int CPT>
 __global__ void __launch_bounds__(DELTA_WARPS * 32) delta_portion_kernel(const DeltaArgs a) {

@@ -58,7 +58,8 @@ _SIGNATURES = {
     "pie_row_stats": [p, i64, i32, i32, p, p],
     "pie_feed_tokens": [p, p, p, i32, p],
     "pie_validate_indices": [p, i32, i32, i32, i32, p, p],
-    "pie_gdn_mixer": [p, i32, p, p, p, p, p, p, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, i32, f32, p],
+    "pie_gdn_coef_elems": [i32, i32, i32, i32],
+    "pie_gdn_mixer": [p, i32, p, p, p, p, p, p, p, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, i32, f32, p],
     "pie_gdn_copy_slot": [p, i64, i64, i32, i32, i32, p],
     "pie_mamba2_mixer": [p, i32, p, p, p, p, p, p, p, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, p],
     "pie_stream_embed": [p, p, p, i32, i32, i32, i32, f32, i32, p],
@@ -124,7 +125,7 @@ _SIGNATURES = {
     "pie_moe_permute": [p, i32, p, p, p, i32, i32, i32, p, p, p],
     "pie_moe_combine": [p, p, p, p, i32, i32, i32, i32, p, i32, p],
 }
-_RESTYPES = {"pie_decode_attn_scratch_floats": i64}
+_RESTYPES = {"pie_decode_attn_scratch_floats": i64, "pie_gdn_coef_elems": i64}
 
 
 class KernelLibraryError(RuntimeError):

@@ -781,3 +781,38 @@ def test_sample_over_cluster_sizes(vocab):
     lg[1] = torch.finfo(torch.bfloat16).min
     got = ops.sample(lg, *_params(rows, 1.0, 0, 0.9, 0.0))
     assert int(got[0]) == 0 and 0 <= int(got[1]) < vocab
+
+
+@pytest.mark.parametrize("dk,dv,hk,hv,lens", [
+    (128, 128, 2, 4, [1, 2, 3, 4, 5, 15, 16, 17, 33]),       # walk: groups of four, stages of sixteen
+    (128, 128, 2, 4, [1, 2, 1, 3, 1, 0]),                    # step: up to two tokens per request on average
+    (128, 128, 1, 32, [7] * 10),                             # walk with four columns per lane
+    (128, 32, 1, 3, [1, 1]), (64, 96, 3, 3, [1, 6, 1]), (32, 256, 1, 2, [19]), (64, 128, 2, 2, [1, 1, 2])])
+def test_gdn_mixer_routes_match_reference(dk, dv, hk, hv, lens):
+    """Every route of the mixer against the reference, from a state that is not zero, with one request reset, over two fires."""
+    from pie_b200.driver.recurrent import RecurrentStateCache
+    from pie_b200.models.config import ModelConfig
+    torch.manual_seed(dk * 7 + dv + len(lens))
+    cfg = ModelConfig(model_type="qwen3_5", num_hidden_layers=1, layer_types=["linear_attention"], linear_num_key_heads=hk,
+                      linear_num_value_heads=hv, linear_key_head_dim=dk, linear_value_head_dim=dv)
+    c, f, n = cfg.gdn_conv_channels, cfg.gdn_in_features, len(lens)
+    bf32 = lambda t: t.to(torch.bfloat16).float()
+    lw = {"gdn_conv": bf32(torch.randn(c, 4) * 0.3), "gdn_A_log": torch.randn(hv) * 0.5, "gdn_dt_bias": torch.randn(hv) * 0.5,
+          "gdn_norm": bf32(1 + torch.randn(dv) * 0.1)}
+    lw_d = {k: v.to(DEV, torch.bfloat16 if k in ("gdn_conv", "gdn_norm") else torch.float32) for k, v in lw.items()}
+    dev_cache, cpu_cache = RecurrentStateCache(cfg, n + 1, DEV), RecurrentStateCache(cfg, n + 1, "cpu")
+    cpu_cache.rec_state.normal_(0, 0.3)
+    cpu_cache.conv_state.normal_()
+    dev_cache.rec_state.copy_(cpu_cache.rec_state)
+    dev_cache.conv_state.copy_(cpu_cache.conv_state)
+    qo = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    slots = np.random.default_rng(1).permutation(n + 1)[:n].astype(np.int32)
+    for reset in ([0] * (n - 1) + [1], [0] * n):
+        mix = bf32(torch.randn(int(qo[-1]), f) * 1.5)
+        want = ref.gdn_mixer(mix, lw["gdn_conv"], lw["gdn_A_log"], lw["gdn_dt_bias"], lw["gdn_norm"], 1e-5, hk, hv, dk, dv,
+                             qo.tolist(), cpu_cache.conv_state[0], cpu_cache.rec_state[0], slots.tolist(), reset)
+        got = ops.gdn_mixer(mix.to(DEV, torch.bfloat16), lw_d, cfg, dev_cache.inputs(qo, slots, np.asarray(reset, np.int32)), 0)
+        torch.cuda.synchronize()
+        close(got.cpu(), want, 2e-3, rtol=1e-2)                       # bf16 results of 32-bit sums
+        assert torch.allclose(dev_cache.rec_state.cpu(), cpu_cache.rec_state, atol=1e-4, rtol=1e-4)
+        assert torch.equal(dev_cache.conv_state.cpu(), cpu_cache.conv_state)
