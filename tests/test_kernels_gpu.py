@@ -816,3 +816,10 @@ def test_gdn_mixer_routes_match_reference(dk, dv, hk, hv, lens):
         close(got.cpu(), want, 2e-3, rtol=1e-2)                       # bf16 results of 32-bit sums
         assert torch.allclose(dev_cache.rec_state.cpu(), cpu_cache.rec_state, atol=1e-4, rtol=1e-4)
         assert torch.equal(dev_cache.conv_state.cpu(), cpu_cache.conv_state)
+
+
+@pytest.mark.parametrize("n,k", [(1, 16), (3, 1008), (7, 1024), (5, 1040), (300, 5120), (2, 25600), (9000, 144)])
+def test_fp8_dequant_row_lengths(n, k):
+    w8 = (torch.randn(n, k, device=DEV) * 100).clamp(-448, 448).to(torch.float8_e4m3fn)
+    q = ops.Fp8Linear(w8, torch.rand(n, (k + 127) // 128, device=DEV) + 0.1)
+    assert torch.equal(ops.dequant_fp8(q), (w8.float() * q.scale.repeat_interleave(128, 1)[:, :k]).to(torch.bfloat16))
