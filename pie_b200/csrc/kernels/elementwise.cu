@@ -138,7 +138,7 @@ __global__ void glu_interleaved_kernel(const bf16* __restrict__ gu, bf16* __rest
 }
 
 // -------------------------------------------- q/k norm + rope + paged KV write
-// One warp per (token, head) of the packed qkv row [Hq*d | Hkv*d | Hkv*d].
+// One block per token of the packed qkv rows [Hq*d | Hkv*d | Hkv*d], D / 16 lanes per head, each with 8 elements of both halves.
 // q heads: optional RMSNorm over the head (weight qn[d]) then rotate-half RoPE,
 // written to q_out[t, h, :]. k heads: same with kn, written to the K half of
 // the token's KV slot. v heads: copied to the V half.
@@ -146,98 +146,139 @@ __global__ void glu_interleaved_kernel(const bf16* __restrict__ gu, bf16* __rest
 // A negative slot skips the KV write (padding tokens of a graph bucket).
 // KV8: the K and V rows are stored as e4m3 bytes with one fp32 scale per (token, KV head) row,
 // scale = max|x| / 448 (kv_layer then addresses bytes, kv_scale [pages][2][Hkv][page_size] floats).
-template <int D, bool KV8>
+// VEC: everything lies on 16-byte boundaries; else elements are read and written one by one.
+// Bound by memory. The token's sines and cosines are worked out once and not by every head's warp again, and rows move in
+// 16-byte pieces. 8300 tokens of 32 + 2 x 8 heads of 128, inputs cold: 91 us with a warp per head, 51 us like this (4.0 TB/s);
+// 512 tokens 12.3 and 10.2 us.
+template <int D, bool KV8, bool VEC>
 __global__ void __launch_bounds__(256)
 qk_norm_rope_kvwrite_kernel(const bf16* __restrict__ qkv, const int* __restrict__ positions,
                             const int* __restrict__ slots, const float* __restrict__ inv_freq,
                             const bf16* __restrict__ qn, const bf16* __restrict__ kn,
-                            bf16* __restrict__ q_out, bf16* __restrict__ kv_layer, int n_tokens,
+                            bf16* __restrict__ q_out, bf16* __restrict__ kv_layer,
                             int hq, int hkv, int page_size, float eps, int qkv_stride,
                             float* __restrict__ kv_scale, const bf16* __restrict__ bias) {
-    constexpr int EP = D / 64;  // elements per lane per half
+    constexpr int LPH = D / 16, HEADS = 256 / LPH;      // lanes of a head, heads at a time
+    __shared__ __align__(16) float s_cos[D / 2], s_sin[D / 2];
     pdl_trigger();
+    const int t = blockIdx.x, g = threadIdx.x % LPH, heads = hq + 2 * hkv;
     pdl_wait();
-    const int heads = hq + 2 * hkv;
-    const long gw = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (gw >= (long)n_tokens * heads) return;
-    const int t = (int)(gw / heads);
-    const int h = (int)(gw - (long)t * heads);
-    const bf16* src = qkv + (size_t)t * qkv_stride + (size_t)h * D;
-    float lo[EP], hi[EP];
+    auto load8 = [](const bf16* p, float (&f)[8]) {
+        if (VEC) {
+            unpack8(*reinterpret_cast<const bf16x8*>(p), f);
+        } else {
 #pragma unroll
-    for (int e = 0; e < EP; ++e) {
-        lo[e] = __bfloat162float(src[lane * EP + e]);
-        hi[e] = __bfloat162float(src[D / 2 + lane * EP + e]);
-    }
-    if (bias) {     // projection bias (Qwen2): added here instead of by a pass of its own over the packed rows, rounded as that pass would
-        const bf16* bp = bias + (size_t)h * D;
-#pragma unroll
-        for (int e = 0; e < EP; ++e) {
-            lo[e] = __bfloat162float(__float2bfloat16(lo[e] + __bfloat162float(bp[lane * EP + e])));
-            hi[e] = __bfloat162float(__float2bfloat16(hi[e] + __bfloat162float(bp[D / 2 + lane * EP + e])));
+            for (int e = 0; e < 8; ++e) f[e] = __bfloat162float(p[e]);
         }
-    }
-    const bool is_q = h < hq;
-    const bool is_k = !is_q && h < hq + hkv;
-    if (is_q || is_k) {
-        const bf16* nw = is_q ? qn : kn;
-        if (nw) {
-            float ss = 0.f;
+    };
+    float lo[8], hi[8];
+    auto load = [&](int h) {
+        const bf16* src = qkv + (size_t)t * qkv_stride + (size_t)min(h, heads - 1) * D + g * 8;
+        load8(src, lo);
+        load8(src + D / 2, hi);
+    };
+    load(threadIdx.x / LPH);
+    if (threadIdx.x < D / 2) sincosf((float)positions[t] * inv_freq[threadIdx.x], &s_sin[threadIdx.x], &s_cos[threadIdx.x]);
+    const int slot = slots[t], page = slot / page_size, off = slot - page * page_size;
+    __syncthreads();
+    for (int h0 = 0; h0 < heads; h0 += HEADS) {
+        const int h = h0 + threadIdx.x / LPH;
+        if (h0) load(h);
+        if (bias) {     // projection bias (Qwen2): added here instead of by a pass of its own over the packed rows, rounded as that pass would
+            float b[8];
+            const bf16* bp = bias + (size_t)min(h, heads - 1) * D + g * 8;
+            load8(bp, b);
 #pragma unroll
-            for (int e = 0; e < EP; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
-            ss = warp_sum(ss);
-            const float inv = rsqrtf(ss / (float)D + eps);
+            for (int e = 0; e < 8; ++e) lo[e] = __bfloat162float(__float2bfloat16(lo[e] + b[e]));
+            load8(bp + D / 2, b);
 #pragma unroll
-            for (int e = 0; e < EP; ++e) {
+            for (int e = 0; e < 8; ++e) hi[e] = __bfloat162float(__float2bfloat16(hi[e] + b[e]));
+        }
+        const bool is_q = h < hq, is_k = !is_q && h < hq + hkv;
+        if (qn || kn) {                                 // by all lanes of the warp, whatever their heads
+            // pairs of squares as 32 lanes of D / 64 pairs would add them up, halving outwards in
+            constexpr int EP = D / 64, NP = 8 / EP;
+            float part[NP];
+#pragma unroll
+            for (int i = 0; i < NP; ++i) {
+                part[i] = 0.f;
+#pragma unroll
+                for (int e = i * EP; e < (i + 1) * EP; ++e) part[i] += lo[e] * lo[e] + hi[e] * hi[e];
+            }
+#pragma unroll
+            for (int o = LPH / 2; o; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < NP; ++i) part[i] += __shfl_xor_sync(0xffffffffu, part[i], o);
+#pragma unroll
+            for (int o = NP / 2; o; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < o; ++i) part[i] += part[i + o];
+            const bf16* nw = is_q ? qn : is_k ? kn : nullptr;
+            if (nw) {
+                const float inv = rsqrtf(part[0] / (float)D + eps);
+                float w[8];
+                load8(nw + g * 8, w);
                 // round to bf16 after the norm as a separate norm kernel would
-                lo[e] = __bfloat162float(__float2bfloat16(
-                    lo[e] * inv * __bfloat162float(nw[lane * EP + e])));
-                hi[e] = __bfloat162float(__float2bfloat16(
-                    hi[e] * inv * __bfloat162float(nw[D / 2 + lane * EP + e])));
+#pragma unroll
+                for (int e = 0; e < 8; ++e) lo[e] = __bfloat162float(__float2bfloat16(lo[e] * inv * w[e]));
+                load8(nw + D / 2 + g * 8, w);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) hi[e] = __bfloat162float(__float2bfloat16(hi[e] * inv * w[e]));
             }
         }
-        const float pos = (float)positions[t];
+        if (is_q || is_k) {
 #pragma unroll
-        for (int e = 0; e < EP; ++e) {
-            float s, c;
-            sincosf(pos * inv_freq[lane * EP + e], &s, &c);
-            const float a = lo[e], b = hi[e];
-            lo[e] = a * c - b * s;
-            hi[e] = b * c + a * s;
+            for (int e = 0; e < 8; ++e) {
+                const float s = s_sin[g * 8 + e], c = s_cos[g * 8 + e], a = lo[e], b = hi[e];
+                lo[e] = a * c - b * s;
+                hi[e] = b * c + a * s;
+            }
         }
-    }
-    bf16* dst;
-    if (is_q) {
-        dst = q_out + ((size_t)t * hq + h) * D;
-    } else {
-        const int slot = slots[t];
-        if (slot < 0) return;
-        const int page = slot / page_size, off = slot - page * page_size;
-        const int kvh = is_k ? (h - hq) : (h - hq - hkv);
-        const size_t row = (((size_t)page * 2 + (is_k ? 0 : 1)) * hkv + kvh) * page_size + off;
+        float scale = 0.f;
         if (KV8) {
             float amax = 0.f;
 #pragma unroll
-            for (int e = 0; e < EP; ++e) amax = fmaxf(amax, fmaxf(fabsf(lo[e]), fabsf(hi[e])));
-            amax = warp_max(amax);
-            const float scale = fmaxf(amax, 1e-12f) * (1.0f / 448.0f);
-            const float inv = 1.0f / scale;
-            uint8_t* d8 = reinterpret_cast<uint8_t*>(kv_layer) + row * D;
+            for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fmaxf(fabsf(lo[e]), fabsf(hi[e])));
 #pragma unroll
-            for (int e = 0; e < EP; ++e) {
-                d8[lane * EP + e] = (uint8_t)__nv_cvt_float_to_fp8(lo[e] * inv, __NV_SATFINITE, __NV_E4M3);
-                d8[D / 2 + lane * EP + e] = (uint8_t)__nv_cvt_float_to_fp8(hi[e] * inv, __NV_SATFINITE, __NV_E4M3);
-            }
-            if (lane == 0) kv_scale[row] = scale;
-            return;
+            for (int o = LPH / 2; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            scale = fmaxf(amax, 1e-12f) * (1.0f / 448.0f);
         }
-        dst = kv_layer + row * D;
-    }
+        if (h >= heads || (!is_q && slot < 0)) continue;
+        const int kvh = is_k ? h - hq : h - hq - hkv;
+        const size_t row = (((size_t)page * 2 + (is_k ? 0 : 1)) * hkv + kvh) * page_size + off;
+        if (KV8 && !is_q) {
+            const float inv = 1.0f / scale;
+            union { uint8_t b[8]; uint2 v; } p[2];
 #pragma unroll
-    for (int e = 0; e < EP; ++e) {
-        dst[lane * EP + e] = __float2bfloat16(lo[e]);
-        dst[D / 2 + lane * EP + e] = __float2bfloat16(hi[e]);
+            for (int e = 0; e < 8; ++e) {
+                p[0].b[e] = (uint8_t)__nv_cvt_float_to_fp8(lo[e] * inv, __NV_SATFINITE, __NV_E4M3);
+                p[1].b[e] = (uint8_t)__nv_cvt_float_to_fp8(hi[e] * inv, __NV_SATFINITE, __NV_E4M3);
+            }
+            uint8_t* d8 = reinterpret_cast<uint8_t*>(kv_layer) + row * D + g * 8;
+            if (VEC) {
+                *reinterpret_cast<uint2*>(d8) = p[0].v;
+                *reinterpret_cast<uint2*>(d8 + D / 2) = p[1].v;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    d8[e] = p[0].b[e];
+                    d8[D / 2 + e] = p[1].b[e];
+                }
+            }
+            if (g == 0) kv_scale[row] = scale;
+            continue;
+        }
+        bf16* dst = (is_q ? q_out + ((size_t)t * hq + h) * D : kv_layer + row * D) + g * 8;
+        if (VEC) {
+            *reinterpret_cast<bf16x8*>(dst) = pack8(lo);
+            *reinterpret_cast<bf16x8*>(dst + D / 2) = pack8(hi);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                dst[e] = __float2bfloat16(lo[e]);
+                dst[D / 2 + e] = __float2bfloat16(hi[e]);
+            }
+        }
     }
 }
 
@@ -512,12 +553,13 @@ PIE_API int pie_qk_bias_norm_rope_kvwrite(const void* qkv, const void* qkv_bias,
                                           int hkv, int head_dim, int page_size, float eps, int qkv_stride,
                                           cudaStream_t st) {
     if (n_tokens <= 0) return 0;
-    const long warps = (long)n_tokens * (hq + 2 * hkv);
-    const int blocks = (int)((warps + 7) / 8);
+    const uintptr_t all = (uintptr_t)qkv | (uintptr_t)qkv_bias | (uintptr_t)q_norm_w | (uintptr_t)k_norm_w | (uintptr_t)q_out | (uintptr_t)kv_layer;
+    const bool vec = qkv_stride % 8 == 0 && all % 16 == 0;
 #define LAUNCH(D, KV8)                                                                           \
-    launch_pdl(qk_norm_rope_kvwrite_kernel<D, KV8>, dim3(blocks), dim3(256), 0, st,             \
+    launch_pdl(vec ? qk_norm_rope_kvwrite_kernel<D, KV8, true> : qk_norm_rope_kvwrite_kernel<D, KV8, false>, \
+        dim3(n_tokens), dim3(256), 0, st,                                                       \
         (const bf16*)qkv, positions, slots, inv_freq, (const bf16*)q_norm_w,                    \
-        (const bf16*)k_norm_w, (bf16*)q_out, (bf16*)kv_layer, n_tokens, hq, hkv, page_size, eps, \
+        (const bf16*)k_norm_w, (bf16*)q_out, (bf16*)kv_layer, hq, hkv, page_size, eps,          \
         qkv_stride, kv_scale, (const bf16*)qkv_bias)
     if (kv_scale) {
         if (head_dim == 64) LAUNCH(64, true);

@@ -818,6 +818,25 @@ def test_gdn_mixer_routes_match_reference(dk, dv, hk, hv, lens):
         assert torch.equal(dev_cache.conv_state.cpu(), cpu_cache.conv_state)
 
 
+@pytest.mark.parametrize("d,hq,hkv", [(64, 3, 1), (128, 32, 8), (128, 5, 1), (256, 17, 2)])
+def test_rope_kvwrite_of_unaligned_rows(d, hq, hkv):
+    """Rows on odd boundaries take the element-wise form of the kernel: the same numbers, and the reference's."""
+    n, page, width = 9, 4, (hq + 2 * hkv) * d
+    packed, kn = bf(n, width, seed=5), bf(d, seed=6) + 1
+    odd = torch.zeros(n, width + 3, dtype=torch.bfloat16, device=DEV)[:, 1:width + 1]
+    odd.copy_(packed)
+    pos = torch.tensor([0, 1, 7, 100, 4095, 8, 9, 10, 131071], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([3, 0, -1, 11, 5, 6, 7, 8, 9], dtype=torch.int32, device=DEV)
+    freq = 500000.0 ** (-torch.arange(0, d, 2, device=DEV).float() / d)
+    kv = [torch.zeros(3, 2, hkv, page, d, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+    for norm in (None, kn):
+        got = [ops.qk_norm_rope_kvwrite(q, pos, slots, freq, norm, norm, k, hq, hkv, d, page, 1e-5) for q, k in ((packed, kv[0]), (odd, kv[1]))]
+        want = ref.qk_norm_rope_kvwrite(packed, pos, slots, freq, norm, norm, kv[2], hq, hkv, d, page, 1e-5)
+        assert torch.equal(got[0], got[1]) and torch.equal(kv[0], kv[1])
+        close(got[0].view(n, -1), want.reshape(n, -1), 3e-2)
+        close(kv[0], kv[2], 3e-2)
+
+
 @pytest.mark.parametrize("n,k", [(1, 16), (3, 1008), (7, 1024), (5, 1040), (300, 5120), (2, 25600), (9000, 144)])
 def test_fp8_dequant_row_lengths(n, k):
     w8 = (torch.randn(n, k, device=DEV) * 100).clamp(-448, 448).to(torch.float8_e4m3fn)
