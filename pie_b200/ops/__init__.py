@@ -480,6 +480,7 @@ class MoeBuffers:
         self.counts_out = torch.zeros(num_experts, **i32)
         self.seg_start = torch.empty(num_experts, **i32)
         self.tile_expert = torch.empty(self.max_mtiles, **i32)
+        self.tile_list = torch.zeros(1 + self.max_mtiles, **i32)
         self.xs = torch.zeros(rows, hidden, dtype=dtype, device=device)
         self.act = torch.zeros(rows, inter, dtype=dtype, device=device)
         self.ys = torch.zeros(rows, hidden, dtype=dtype, device=device)
@@ -496,7 +497,7 @@ def moe_route(logits, k: int, renorm: bool, buf: "MoeBuffers", e_lo: int = 0):
 
 def moe_align(buf: "MoeBuffers", max_mtiles: int = 0):
     check(fn("pie_moe_align")(ptr(buf.counts), buf.E, max_mtiles or buf.max_mtiles, ptr(buf.seg_start),
-                              ptr(buf.tile_expert), ptr(buf.counts_out), stream_ptr()), "moe_align")
+                              ptr(buf.tile_expert), ptr(buf.tile_list), ptr(buf.counts_out), stream_ptr()), "moe_align")
 
 
 def moe_permute(x, buf: "MoeBuffers", weighted: bool = False):
@@ -510,11 +511,12 @@ def moe_permute(x, buf: "MoeBuffers", weighted: bool = False):
                                 ptr(buf.xs), ptr(buf.slot_of), stream_ptr()), "moe_permute")
 
 
-def grouped_gemm(a, w, tile_expert, out, max_mtiles: int, epilogue: int = EPI_STORE):
-    """out[tile rows] = a[tile rows] @ w[tile_expert[tile]].T for every used 128-row tile. w [E,N,K]."""
+def grouped_gemm(a, w, tile_expert, out, max_mtiles: int, epilogue: int = EPI_STORE, tile_list=None):
+    """out[tile rows] = a[tile rows] @ w[tile_expert[tile]].T for every used 128-row tile. w [E,N,K]. `tile_list` (as `moe_align`
+    writes it) limits the work to the rows in use; other rows of `out` are left alone."""
     e, n, k = w.shape
     assert w.is_contiguous() and a.shape[1] == k and a.shape[0] >= max_mtiles * MOE_TILE
-    check(fn("pie_grouped_gemm_bf16")(ptr(a), ptr(w), ptr(out), ptr(tile_expert), max_mtiles, e, n, k, a.stride(0),
+    check(fn("pie_grouped_gemm_bf16")(ptr(a), ptr(w), ptr(out), ptr(tile_expert), ptr(tile_list), max_mtiles, e, n, k, a.stride(0),
                                       out.stride(0), epilogue, ptr(kernel_status(a.device)), num_sms(a.device),
                                       stream_ptr()), "grouped_gemm_bf16")
     return out
@@ -554,8 +556,8 @@ def moe_experts(x, logits, w_gate_up, w_down, k: int, renorm: bool, buf: "MoeBuf
     moe_route(logits, k, renorm, buf, e_lo)
     moe_align(buf, mt)
     moe_permute(x, buf)
-    grouped_gemm(buf.xs, w_gate_up, buf.tile_expert, buf.act, mt, EPI_SWIGLU)
-    grouped_gemm(buf.act, w_down, buf.tile_expert, buf.ys, mt, EPI_STORE)
+    grouped_gemm(buf.xs, w_gate_up, buf.tile_expert, buf.act, mt, EPI_SWIGLU, buf.tile_list)
+    grouped_gemm(buf.act, w_down, buf.tile_expert, buf.ys, mt, EPI_STORE, buf.tile_list)
     if rs is not None:
         check(fn("pie_moe_combine_rs")(ptr(buf.ys), ptr(buf.slot_of), ptr(buf.w), n, buf.H, k, rs[0], rs[1],
                                        stream_ptr()), "moe_combine_rs")

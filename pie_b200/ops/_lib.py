@@ -112,16 +112,16 @@ _SIGNATURES = {
     "pie_biased_prefill": [p, i32, p, p],
     "pie_moe_route_scored": [p, i32, i64, i32, i32, i32, i32, i32, p, p, p, p, p, p],
     "pie_moe_combine_identity": [p, p, p, p, i32, i32, i32, i32, p, i32, p],
-    "pie_grouped_gemm_clamp_glu": [p, p, p, p, i32, i32, i32, i32, i32, i32, f32, p, i32, p],
+    "pie_grouped_gemm_clamp_glu": [p, p, p, p, p, i32, i32, i32, i32, i32, i32, f32, p, i32, p],
     "pie_gemm_set_workspace": [i32, p, i64, p, i32],
     "pie_gemm_set_pairs": [i32],
     "pie_gemm_set_swap": [i32],
     "pie_set_pdl": [i32],
     "pie_gemm_bf16": [p, p, p, p, i32, i32, i32, i32, i32, i32, i32, i32, i32, p, i32, p],
-    "pie_grouped_gemm_bf16": [p, p, p, p, i32, i32, i32, i32, i32, i32, i32, p, i32, p],
+    "pie_grouped_gemm_bf16": [p, p, p, p, p, i32, i32, i32, i32, i32, i32, i32, p, i32, p],
     "pie_moe_route": [p, i32, i32, i32, i32, i32, i32, i32, i32, p, p, p, p, p],
     "pie_moe_combine_rs": [p, p, p, i32, i32, i32, p, i32, p],
-    "pie_moe_align": [p, i32, i32, p, p, p, p],
+    "pie_moe_align": [p, i32, i32, p, p, p, p, p],
     "pie_moe_permute": [p, i32, p, p, p, i32, i32, i32, p, p, p],
     "pie_moe_combine": [p, p, p, p, i32, i32, i32, i32, p, i32, p],
 }
