@@ -31,11 +31,11 @@ LATENT_SOURCES = ("attention_tc", "elementwise", "gemm2_tcgen05", "gemm_skinny",
                   "latent_attn", "latent_attn_tc", "sampling")
 
 # sources whose kernels sandwich-normed blocks with linear attention launch
-SANDWICH_SOURCES = ("attention_bias", "elementwise", "gdn", "gemm2_tcgen05", "gemm_skinny", "gemm_tcgen05", "latent",
+SANDWICH_SOURCES = ("attention_bias", "elementwise", "gdn", "gemm2_tcgen05", "gemm_grouped", "gemm_skinny", "gemm_tcgen05", "latent",
                     "latent_attn", "linear_attn", "moe", "sampling")
 
 # sources whose kernels blocks normed on the way out (grouped and latent attention, matrix memory) launch
-POST_NORM_SOURCES = ("attention", "attention_gqa", "attention_tc", "elementwise", "gdn", "gemm2_tcgen05", "gemm_skinny",
+POST_NORM_SOURCES = ("attention", "attention_gqa", "attention_tc", "elementwise", "gdn", "gemm2_tcgen05", "gemm_grouped", "gemm_skinny",
                      "gemm_tcgen05", "latent", "latent_attn", "latent_attn_tc", "linear_attn", "moe", "sampling")
 
 # sources whose kernels blocks that read the stream through a layer norm and a convolution launch

@@ -25,60 +25,8 @@ constexpr int SKINNY_MAX_STAGES = 8;
 constexpr uint32_t SKINNY_RING = 108 * 1024;                   // two CTAs per SM
 constexpr uint32_t SKINNY_SMEM = SKINNY_RING + 1024 /*align*/ + 256 /*barriers*/;
 
-// 32 lanes x 16 columns of fp32 accumulators: thread = TMEM lane, v[j] = column j.
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
-// Stores 16 tokens' values of one output feature per thread (a warp holds 32 consecutive features): 64 B of a token's row
-// per store. GLU epilogues pair neighbouring lanes (gate, up).
-template <int EPI>
-__device__ __forceinline__ void skinny_store(const float (&v)[16], int feat, int tok0, int F, int tok_end, bf16* __restrict__ C, int ldc,
-                                             const bf16* __restrict__ R, int ldr, const EpiArgs& ex, const XieluCoef& act) {
-    const bool live = feat < F;
-    if constexpr (EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_CLAMP_GLU) {
-        const bool even = !(threadIdx.x & 1);
-#pragma unroll
-        for (int t = 0; t < 16; ++t) {
-            const float other = __shfl_xor_sync(0xffffffffu, v[t], 1);
-            if (live && even && tok0 + t < tok_end)
-                C[(size_t)(tok0 + t) * ldc + (feat >> 1)] = __float2bfloat16(glu_value<EPI>(v[t], other, ex.limit));
-        }
-        return;
-    }
-    if (!live) return;
-    float add[16];
-    const float bias = (EPI == EPI_XIELU || EPI == EPI_STREAM) && ex.bias ? __bfloat162float(ex.bias[feat]) : 0.f;
-    if constexpr (EPI == EPI_RESIDUAL || EPI == EPI_STREAM) {      // all loads before the first store: it may be to the same row
-#pragma unroll
-        for (int t = 0; t < 16; ++t) {
-            const int tok = tok0 + t;
-            if (EPI == EPI_RESIDUAL) add[t] = tok < tok_end ? __bfloat162float(R[(size_t)tok * ldr + feat]) : 0.f;
-            else add[t] = tok < tok_end ? ex.res32[(size_t)tok * ex.ld32 + feat] : 0.f;
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < 16; ++t) {
-        const int tok = tok0 + t;
-        if (tok >= tok_end) break;
-        float o = v[t];
-        if constexpr (EPI == EPI_RESIDUAL) o += add[t];
-        if constexpr (EPI == EPI_XIELU) o = act(o + bias);
-        if constexpr (EPI == EPI_STREAM) {
-            o = add[t] + o + bias;
-            ex.out32[(size_t)tok * ex.ld32 + feat] = o;
-            if (!C) continue;
-        }
-        C[(size_t)tok * ldc + feat] = __float2bfloat16(o);
-    }
 }
 
 // tma_w walks the weights in boxes of 128 rows, tma_x the batch in boxes of all its rows.

@@ -49,15 +49,12 @@ struct GemmCfg {
 // the end costs the TMA more than one inside it (it is filled with zeros row by row). With 128-row boxes a 28672 x 4096
 // product took 71 us for 1 row against 50 us for 128; with boxes of the batch's rows 47 us. Rows of a tile past its box are
 // whatever shared memory held; an accumulator row depends on its own operand row alone, and these are not stored.
-// GROUPED: mixture-of-experts form. A holds token rows sorted by expert in 128-row tiles,
-// tile_expert[m_tile] names the expert whose weights ([E*N, K] under tma_b) the tile multiplies,
-// or -1 for an unused tile, which every role skips. Whole-tile scheduling only.
-template <int BN, int EPI, bool GROUPED = false, int OCC = 1>
+template <int BN, int EPI, int OCC = 1>
 __global__ void __launch_bounds__(GEMM_THREADS, OCC)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  bf16* __restrict__ C, const bf16* __restrict__ R, int M, int N, int K, int ldc,
                  int ldr, int* status, const __grid_constant__ TpArgs tp, const StreamKArgs sk,
-                 const int* __restrict__ tile_expert, int bn, int bm, const __grid_constant__ EpiArgs ex) {
+                 int bn, int bm, const __grid_constant__ EpiArgs ex) {
     using Cfg = GemmCfg<BN, OCC>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -134,13 +131,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             Segment seg;
             while (ok && walk.next(seg)) {
                 const int m_blk = seg.tile % tiles_m, n_blk = seg.tile / tiles_m;
-                int b_row = n_blk * bn;
-                if (GROUPED) {
-                    if (!dep_ready) resolve();       // the tile table itself comes from the previous kernel
-                    const int e = tile_expert[m_blk];
-                    if (e < 0) continue;
-                    b_row += e * N;
-                }
+                const int b_row = n_blk * bn;
                 // Every tile walks K in ascending order: an output element then sees the same
                 // summation order whatever tile shape the plan picked (rotating the start per tile
                 // was measured and did not help).
@@ -198,9 +189,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             bool ok = true;
             SegmentWalk walk(sk.enabled != 0, num_tiles, num_kb, blockIdx.x, gridDim.x);
             Segment seg;
-            if (GROUPED) pdl_wait();
             for (; ok && walk.next(seg); ++tcount) {
-                if (GROUPED && tile_expert[seg.tile % tiles_m] < 0) { --tcount; continue; }
                 const uint32_t acc = tcount & 1u, aph = (tcount >> 1) & 1u;
                 if (!mbar_wait(tempty_bar(acc), aph ^ 1u, status, PIE_ERR_WAIT_EPILOGUE)) break;
                 tc_fence_after();
@@ -239,7 +228,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const XieluCoef act(EPI == EPI_XIELU ? ex.act : nullptr);
         for (; walk.next(seg); ++tcount) {
             const int m_blk = seg.tile % tiles_m, n_blk = seg.tile / tiles_m;
-            if (GROUPED && tile_expert[m_blk] < 0) { --tcount; continue; }
             const uint32_t acc = tcount & 1u, aph = (tcount >> 1) & 1u;
             const bool got = mbar_wait(tfull_bar(acc), aph, status, PIE_ERR_WAIT_MMA);
             if (!__all_sync(0xffffffffu, got)) break;
@@ -556,7 +544,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, void* C, co
     if (e != cudaSuccess) return (int)e;
     StreamKArgs sk{w.ws, w.cnt, plan.streamk, g_gemm_dbg, g_gemm_trace};
     e = launch_pdl(kern, dim3(plan.grid), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, ta, tb, (bf16*)C, (const bf16*)R,
-                   M, N, K, ldc, ldr, status, tp, sk, (const int*)nullptr, plan.bn, bm, ex);
+                   M, N, K, ldc, ldr, status, tp, sk, plan.bn, bm, ex);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
@@ -696,59 +684,4 @@ PIE_API int pie_gemm_bf16_tp(const void* A, const void* W, void* C, int M, int N
     else if (bn == 64) { GO(64) }
 #undef GO
     return (int)cudaErrorInvalidValue;
-}
-
-// Grouped (mixture-of-experts) GEMM: A [max_mtiles*128, K] holds token rows sorted by expert in
-// 128-row tiles; W is [E, N, K] contiguous; tile_expert [max_mtiles] (device) gives each tile's
-// expert or -1. C [max_mtiles*128, N] (or N/2 with the SwiGLU epilogue). Graph-safe: the launch
-// shape depends only on max_mtiles.
-static int grouped_gemm(const void* A, const void* W, void* C, const int* tile_expert, int max_mtiles, int num_experts, int N, int K,
-                        int lda, int ldc, int epilogue, int* status, int num_sms, cudaStream_t st, const EpiArgs& ex) {
-    if (max_mtiles <= 0 || N <= 0 || num_experts <= 0) return 0;
-    if (K <= 0 || K % 8 || N % 8 || ldc % 8) return (int)cudaErrorInvalidValue;
-    if ((epilogue == EPI_SWIGLU || epilogue == EPI_CLAMP_GLU) && N % 32) return (int)cudaErrorInvalidValue;
-    const int M = max_mtiles * GEMM_BM;
-    const int bn = N >= 128 ? 128 : 64;
-    CUtensorMap ta, tb;
-    if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
-    if (pie_make_tma_2d_bf16(&tb, W, (long)num_experts * N, K, K, bn) != 0) return (int)cudaErrorInvalidValue;
-    const long tiles = (long)max_mtiles * ((N + bn - 1) / bn);
-    const int grid = (int)(tiles < num_sms ? tiles : num_sms);
-    StreamKArgs sk{nullptr, nullptr, 0, 0, nullptr};
-    TpArgs tp{};
-#define GO(BN_, EPI_)                                                                                     \
-    {                                                                                                     \
-        auto kern = gemm_bf16_kernel<BN_, EPI_, true>;                                                    \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                                             (int)GemmCfg<BN_>::SMEM_BYTES);                              \
-        if (e != cudaSuccess) return (int)e;                                                              \
-        e = launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), GemmCfg<BN_>::SMEM_BYTES, st, ta, tb, (bf16*)C, \
-                       (const bf16*)nullptr, M, N, K, ldc, 0, status, tp, sk, tile_expert, bn, GEMM_BM, ex);    \
-        return (int)(e != cudaSuccess ? e : cudaGetLastError());                                          \
-    }
-    if (epilogue == EPI_STORE) {
-        if (bn == 128) GO(128, EPI_STORE) else GO(64, EPI_STORE)
-    } else if (epilogue == EPI_SWIGLU) {
-        if (bn == 128) GO(128, EPI_SWIGLU) else GO(64, EPI_SWIGLU)
-    } else if (epilogue == EPI_CLAMP_GLU) {
-        if (bn == 128) GO(128, EPI_CLAMP_GLU) else GO(64, EPI_CLAMP_GLU)
-    }
-#undef GO
-    return (int)cudaErrorInvalidValue;
-}
-
-PIE_API int pie_grouped_gemm_bf16(const void* A, const void* W, void* C, const int* tile_expert, int max_mtiles,
-                                  int num_experts, int N, int K, int lda, int ldc, int epilogue, int* status,
-                                  int num_sms, cudaStream_t st) {
-    if (epilogue != EPI_STORE && epilogue != EPI_SWIGLU) return (int)cudaErrorInvalidValue;
-    return grouped_gemm(A, W, C, tile_expert, max_mtiles, num_experts, N, K, lda, ldc, epilogue, status, num_sms, st, EpiArgs());
-}
-
-// The clamped GLU of experts without biases in the epilogue: C [max_mtiles*128, N/2], see EPI_CLAMP_GLU.
-PIE_API int pie_grouped_gemm_clamp_glu(const void* A, const void* W, void* C, const int* tile_expert, int max_mtiles,
-                                       int num_experts, int N, int K, int lda, int ldc, float limit, int* status,
-                                       int num_sms, cudaStream_t st) {
-    EpiArgs ex;
-    ex.limit = limit;
-    return grouped_gemm(A, W, C, tile_expert, max_mtiles, num_experts, N, K, lda, ldc, EPI_CLAMP_GLU, status, num_sms, st, ex);
 }

@@ -1,7 +1,7 @@
-// Mixture-of-experts plumbing around the grouped tcgen05 GEMM (gemm_tcgen05.cu, GROUPED form):
+// Mixture-of-experts plumbing around the grouped tcgen05 GEMM (gemm_grouped.cu):
 //   pie_moe_route    softmax over E router logits, top-k, optional renormalisation; every route
 //                    (token, j) takes a position inside its expert's segment with one atomic
-//   pie_moe_align    per-expert segments padded to 128-row tiles: seg_start[e], tile_expert[tile]
+//   pie_moe_align    per-expert segments padded to 128-row tiles: seg_start[e], tile_expert[tile], and the list of work tiles
 //   pie_moe_permute  token rows -> expert-sorted rows
 //   pie_moe_combine  out[t] = residual[t] + sum_j w[t,j] * y[slot(t,j)]; the _rs form stores this
 //                    rank's partial rows into the row owners' receive buffers (peer stores)
@@ -107,32 +107,61 @@ __global__ void moe_route_kernel(const T* __restrict__ logits, int ld, int n, in
 
 // Single block. counts [E] -> seg_start [E] (row of the expert's first slot), tile_expert
 // [max_mtiles]; counts are copied to counts_out (may be null) and zeroed for the next call.
+// tile_list (may be null): the work tiles of the grouped GEMM, [0] their number, then (first 128-row tile << 9 | rows) with up
+// to 256 rows of one expert each.
 __global__ void moe_align_kernel(int* __restrict__ counts, int E, int max_mtiles, int* __restrict__ seg_start,
-                                 int* __restrict__ tile_expert, int* __restrict__ counts_out) {
-    __shared__ int tiles_of[MOE_MAX_E];
-    __shared__ int start_of[MOE_MAX_E + 1];
+                                 int* __restrict__ tile_expert, int* __restrict__ tile_list, int* __restrict__ counts_out) {
+    __shared__ int count_of[MOE_MAX_E];
+    __shared__ int start_of[MOE_MAX_E + 1], work_of[MOE_MAX_E + 1];       // first 128-row tile, first work tile
+    constexpr int PER = MOE_MAX_E / 32;
     const int tid = threadIdx.x;
-    for (int e = tid; e < E; e += blockDim.x) {
-        const int c = counts[e];
-        tiles_of[e] = (c + MOE_TILE - 1) / MOE_TILE;
-        if (counts_out) counts_out[e] = c;
-        counts[e] = 0;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        int acc = 0;
-        for (int e = 0; e < E; ++e) {
-            start_of[e] = acc;
-            acc += tiles_of[e];
+    for (int e = tid; e < MOE_MAX_E; e += blockDim.x) {
+        const int c = e < E ? counts[e] : 0;
+        count_of[e] = c;
+        if (e < E) {
+            if (counts_out) counts_out[e] = c;
+            counts[e] = 0;
         }
-        start_of[E] = acc;
+    }
+    __syncthreads();
+    if (tid < 32) {                          // a lane adds up its experts, the warp the lanes
+        int tiles = 0, works = 0;
+        for (int i = 0; i < PER; ++i) {
+            const int c = count_of[tid * PER + i];
+            tiles += (c + MOE_TILE - 1) / MOE_TILE;
+            works += (c + 2 * MOE_TILE - 1) / (2 * MOE_TILE);
+        }
+        int t = tiles, w = works;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int tt = __shfl_up_sync(0xffffffffu, t, o), ww = __shfl_up_sync(0xffffffffu, w, o);
+            if (tid >= o) { t += tt; w += ww; }
+        }
+        t -= tiles;
+        w -= works;
+        for (int i = 0; i < PER; ++i) {
+            const int e = tid * PER + i, c = count_of[e];
+            start_of[e] = t;
+            work_of[e] = w;
+            t += (c + MOE_TILE - 1) / MOE_TILE;
+            w += (c + 2 * MOE_TILE - 1) / (2 * MOE_TILE);
+        }
+        if (tid == 31) {
+            start_of[MOE_MAX_E] = t;
+            work_of[MOE_MAX_E] = w;
+        }
     }
     __syncthreads();
     for (int e = tid; e < E; e += blockDim.x) {
-        seg_start[e] = start_of[e] * MOE_TILE;
-        for (int t = start_of[e]; t < start_of[e + 1] && t < max_mtiles; ++t) tile_expert[t] = e;
+        const int first = start_of[e], c = count_of[e];
+        seg_start[e] = first * MOE_TILE;
+        for (int t = first; t < start_of[e + 1] && t < max_mtiles; ++t) tile_expert[t] = e;
+        if (!tile_list) continue;
+        for (int j = 0; j * 2 * MOE_TILE < c && work_of[e] + j < max_mtiles; ++j)
+            tile_list[1 + work_of[e] + j] = (first + 2 * j) << 9 | min(c - j * 2 * MOE_TILE, 2 * MOE_TILE);
     }
-    for (int t = start_of[E] + tid; t < max_mtiles; t += blockDim.x) tile_expert[t] = -1;
+    if (tile_list && tid == 0) tile_list[0] = work_of[MOE_MAX_E];
+    for (int t = start_of[MOE_MAX_E] + tid; t < max_mtiles; t += blockDim.x) tile_expert[t] = -1;
 }
 
 // One block per route: xs[slot] = x[token], times the route's weight with `scale`; routes of experts that are not local (ids < 0) take
@@ -244,10 +273,10 @@ PIE_API int pie_moe_route_sigmoid(const float* logits, int splits, long split_st
     return (int)cudaGetLastError();
 }
 
-PIE_API int pie_moe_align(int* counts, int E, int max_mtiles, int* seg_start, int* tile_expert, int* counts_out,
+PIE_API int pie_moe_align(int* counts, int E, int max_mtiles, int* seg_start, int* tile_expert, int* tile_list, int* counts_out,
                           cudaStream_t st) {
     if (E > MOE_MAX_E || E <= 0) return (int)cudaErrorInvalidValue;
-    moe_align_kernel<<<1, 256, 0, st>>>(counts, E, max_mtiles, seg_start, tile_expert, counts_out);
+    moe_align_kernel<<<1, 256, 0, st>>>(counts, E, max_mtiles, seg_start, tile_expert, tile_list, counts_out);
     return (int)cudaGetLastError();
 }
 

@@ -233,8 +233,8 @@ def sigmoid_experts(x, router, gate_up, down, spec, buf, shared=None):
     mt = ops.moe_max_mtiles(n, spec.top, spec.experts)
     ops.moe_align(buf, mt)
     ops.moe_permute(x, buf, weighted=True)
-    ops.grouped_gemm(buf.xs, gate_up, buf.tile_expert, buf.act, mt, ops.EPI_SWIGLU)
-    ops.grouped_gemm(buf.act, down, buf.tile_expert, buf.ys, mt, ops.EPI_STORE)
+    ops.grouped_gemm(buf.xs, gate_up, buf.tile_expert, buf.act, mt, ops.EPI_SWIGLU, buf.tile_list)
+    ops.grouped_gemm(buf.act, down, buf.tile_expert, buf.ys, mt, ops.EPI_STORE, buf.tile_list)
     return ops.moe_combine(buf, n, shared, weighted=False)
 
 
@@ -252,10 +252,10 @@ def scored_experts(x, router, correction, gate_up, down, spec, buf):
     ops.moe_align(buf, mt)
     ops.moe_permute(x, buf)
     ne, n2, k = gate_up.shape
-    check(fn("pie_grouped_gemm_clamp_glu")(ptr(buf.xs), ptr(gate_up), ptr(buf.act), ptr(buf.tile_expert), mt, ne, n2, k, buf.xs.stride(0),
-                                           buf.act.stride(0), spec.limit, ptr(ops.kernel_status(dev)), ops.num_sms(dev), stream_ptr()),
+    check(fn("pie_grouped_gemm_clamp_glu")(ptr(buf.xs), ptr(gate_up), ptr(buf.act), ptr(buf.tile_expert), ptr(buf.tile_list), mt, ne, n2, k,
+                                           buf.xs.stride(0), buf.act.stride(0), spec.limit, ptr(ops.kernel_status(dev)), ops.num_sms(dev), stream_ptr()),
           "grouped_gemm_clamp_glu")
-    ops.grouped_gemm(buf.act, down, buf.tile_expert, buf.ys, mt, ops.EPI_STORE)
+    ops.grouped_gemm(buf.act, down, buf.tile_expert, buf.ys, mt, ops.EPI_STORE, buf.tile_list)
     out = torch.empty(n, buf.H, dtype=x.dtype, device=dev)
     check(fn("pie_moe_combine_identity")(ptr(buf.ys), ptr(buf.slot_of), ptr(buf.w), ptr(x), x.stride(0), n, buf.H, spec.top, ptr(out),
                                          out.stride(0), stream_ptr()), "moe_combine_identity")

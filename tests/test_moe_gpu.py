@@ -84,3 +84,36 @@ def test_moe_block_in_cuda_graph_and_model():
         top2 = torch.topk(logits[-1].float(), 2).values
         if (top2[0] - top2[1]) > 0.05:                   # only compare when the oracle is not at a near tie
             assert int(first[i]) == int(torch.argmax(logits[-1])), i
+
+
+@pytest.mark.parametrize("n,k", [(64, 64), (96, 72), (256, 512), (320, 200), (1536, 2048)])
+@pytest.mark.parametrize("epi", ["store", "swiglu"])
+def test_grouped_gemm_tiles(n, k, epi):
+    """Experts with rows at the edges of the work tiles (16 columns, 128-row segments, 256-row tiles), and the form without a
+    list of work tiles, against the fp32 product; rows that no work tile has are left alone."""
+    from pie_b200 import ops
+    dev = torch.device("cuda")
+    counts = [0, 1, 15, 16, 17, 127, 128, 129, 0, 255, 256, 257, 384, 385, 600]
+    e = len(counts)
+    g = torch.Generator(device=dev).manual_seed(n + k)
+    w = (torch.randn(e, n, k, device=dev, generator=g) * k ** -0.5).to(torch.bfloat16)
+    buf = ops.MoeBuffers(sum(counts), k, n, e, 1, dev)
+    buf.counts.copy_(torch.tensor(counts))
+    buf.xs.normal_(generator=g)
+    ops.moe_align(buf)
+    code, width = (ops.EPI_SWIGLU, n // 2) if epi == "swiglu" else (ops.EPI_STORE, n)
+    for listed in (True, False):
+        out = torch.full((buf.xs.shape[0], width), 7.0, dtype=torch.bfloat16, device=dev)
+        ops.grouped_gemm(buf.xs, w, buf.tile_expert, out, buf.max_mtiles, code, buf.tile_list if listed else None)
+        torch.cuda.synchronize()
+        ops.check_kernel_status(dev)
+        used = torch.zeros(out.shape[0], dtype=torch.bool, device=dev)
+        for ex, (c, at) in enumerate(zip(counts, buf.seg_start.tolist())):
+            rows = c if listed else -(-c // 128) * 128
+            used[at:at + rows] = True
+            y = buf.xs[at:at + rows].float() @ w[ex].float().t()
+            if epi == "swiglu":
+                y = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
+            # one rounding to bf16 (2^-9) of sums whose order differs
+            torch.testing.assert_close(out[at:at + rows].float(), y, rtol=2 ** -8, atol=1e-3)
+        assert bool((out[~used] == 7.0).all())
