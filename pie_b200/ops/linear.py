@@ -253,7 +253,8 @@ def scored_experts(x, router, correction, gate_up, down, spec, buf):
     ops.moe_permute(x, buf)
     ne, n2, k = gate_up.shape
     check(fn("pie_grouped_gemm_clamp_glu")(ptr(buf.xs), ptr(gate_up), ptr(buf.act), ptr(buf.tile_expert), ptr(buf.tile_list), mt, ne, n2, k,
-                                           buf.xs.stride(0), buf.act.stride(0), spec.limit, ptr(ops.kernel_status(dev)), ops.num_sms(dev), stream_ptr()),
+                                           buf.xs.stride(0), buf.act.stride(0), spec.limit, ptr(ops.kernel_status(dev)), ops.num_sms(dev),
+                                           stream_ptr()),
           "grouped_gemm_clamp_glu")
     ops.grouped_gemm(buf.act, down, buf.tile_expert, buf.ys, mt, ops.EPI_STORE, buf.tile_list)
     out = torch.empty(n, buf.H, dtype=x.dtype, device=dev)
