@@ -230,8 +230,8 @@ qk_norm_rope_kvwrite_kernel(const bf16* __restrict__ qkv, const int* __restrict_
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const float s = s_sin[g * 8 + e], c = s_cos[g * 8 + e], a = lo[e], b = hi[e];
-                lo[e] = a * c - b * s;
-                hi[e] = b * c + a * s;
+                lo[e] = __fmaf_rn(a, c, -__fmul_rn(b, s));
+                hi[e] = __fmaf_rn(b, c, __fmul_rn(a, s));
             }
         }
         float scale = 0.f;
