@@ -413,12 +413,14 @@ __device__ __forceinline__ void skinny_store(const float (&v)[16], int feat, int
                                              const bf16* __restrict__ R, int ldr, const EpiArgs& ex, const XieluCoef& act) {
     const bool live = feat < F;
     if constexpr (EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_CLAMP_GLU) {
-        const bool even = !(threadIdx.x & 1);
+        // the even lane of a pair holds gates, the odd one ups: the even lane takes the first eight tokens, the odd one the others
+        const bool odd = threadIdx.x & 1;
 #pragma unroll
-        for (int t = 0; t < 16; ++t) {
-            const float other = __shfl_xor_sync(0xffffffffu, v[t], 1);
-            if (live && even && tok0 + t < tok_end)
-                C[(size_t)(tok0 + t) * ldc + (feat >> 1)] = __float2bfloat16(glu_value<EPI>(v[t], other, ex.limit));
+        for (int t = 0; t < 8; ++t) {
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? v[t] : v[t + 8], 1);
+            const int tok = tok0 + t + (odd ? 8 : 0);
+            if (live && tok < tok_end)
+                C[(size_t)tok * ldc + (feat >> 1)] = __float2bfloat16(glu_value<EPI>(odd ? got : v[t], odd ? v[t + 8] : got, ex.limit));
         }
         return;
     }
@@ -447,6 +449,10 @@ __device__ __forceinline__ void skinny_store(const float (&v)[16], int feat, int
         }
         C[(size_t)tok * ldc + feat] = __float2bfloat16(o);
     }
+}
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
 }  // namespace pie

@@ -7,7 +7,8 @@
 // reads of A. Bound by the weights' bytes where experts have few rows, else by the reads of tiles from L2 and the MMAs.
 //
 // Qwen3-30B-A3B's experts (128 of 2048 x 768), 200 tokens, 8 experts each: gate / up 240 us and down 149 us with 128 x 128 tiles
-// on single CTAs, 141 and 89 us like this (the weights alone: 123 and 62 us); 2900 tokens: 387 and 213, 277 and 190 us.
+// on single CTAs, 141 and 89 us like this, the launches before included (the weights alone: 123 and 62 us). 188 rows per expert:
+// 178 and 113 us.
 //
 // Roles per CTA: warp 0 TMA producer; warp 1 MMA issuer (leader CTA); warps 2-5 epilogue (thread = one output feature). Every
 // mbarrier wait is bounded; the cluster-wide barriers (start, end) are reached by every thread on every path.
@@ -41,12 +42,26 @@ __device__ __forceinline__ bool grouped_tile(const GroupedWork& w, int i, Groupe
     return t.expert >= 0;
 }
 
-// tma_w: boxes of 128 weight rows; tma_x8 / 32 / 128: boxes of that many rows of A.
+// Boxes of 128 weight rows, and of 8, 16, 32, 64 and 128 rows of A.
+struct GroupedMaps {
+    CUtensorMap w, x[5];
+};
+// `rows` (a multiple of 8, up to 128) as one or two boxes (log2 of their rows / 8, -1 for none). A box of its own for every 8 rows
+// cost more than the rows themselves: tiles of 48 tokens took longer than tiles of 64 (166 against 148 us for the
+// gate / up products above). Rows past `rows` land in the slot and are not read.
+__device__ __forceinline__ void grouped_boxes(int rows, int& first, int& second) {
+    first = 31 - __clz(rows >> 3);
+    const int rest = (rows >> 3) - (1 << first);
+    second = rest == 0 ? -1 : 32 - __clz(rest - 1);
+    if (second == first) {
+        ++first;
+        second = -1;
+    }
+}
+
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_grouped_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x8,
-                    const __grid_constant__ CUtensorMap tma_x32, const __grid_constant__ CUtensorMap tma_x128, bf16* __restrict__ C,
-                    int N, int K, int ldc, int* status, const GroupedWork work, const __grid_constant__ EpiArgs ex) {
+gemm_grouped_kernel(const __grid_constant__ GroupedMaps maps, bf16* __restrict__ C, int N, int K, int ldc, int* status, const GroupedWork work, const __grid_constant__ EpiArgs ex) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t ring = (raw + 1023u) & ~1023u;
@@ -91,7 +106,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_cons
 
     if (warp == 0) {
         if (lane == 0) {
-            tma_prefetch_desc(&tma_w);
+            tma_prefetch_desc(&maps.w);
             const uint32_t leader_full0 = map_to_cta(full_bar(0), 0);
             uint32_t it = 0;
             bool ok = true;
@@ -99,23 +114,20 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_cons
                 GroupedTile t;
                 if (!grouped_tile(work, item / tiles_n, t)) continue;
                 const int half = (t.rows + 15) / 16 * 8;                     // rows of A in this CTA
+                int b0, b1;
+                grouped_boxes(half, b0, b1);
+                const uint32_t bytes = GG_W_BYTES + (uint32_t)((8 << b0) + (b1 >= 0 ? 8 << b1 : 0)) * (GEMM_BK * 2);
                 const int x_row = t.row0 + (int)crank * half, w_row = t.expert * N + item % tiles_n * 2 * GEMM_BM + (int)crank * GEMM_BM;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % GG_STAGES;
                     if (!mbar_wait_cluster(empty_bar(s), ((it / GG_STAGES) & 1u) ^ 1u, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
                     // both CTAs' loads complete on the leader's barrier, armed for the pair's bytes
-                    if (leader) mbar_arrive_expect_tx(full_bar(s), 2 * (GG_W_BYTES + (uint32_t)half * (GEMM_BK * 2)));
+                    if (leader) mbar_arrive_expect_tx(full_bar(s), 2 * bytes);
                     const uint32_t lbar = leader_full0 + 8u * s, dst = ring + s * GG_STAGE_BYTES;
-                    tma_load_2d_pair(dst, &tma_w, lbar, kb * GEMM_BK, w_row);
-                    int at = 0;
-                    if (half == 128) {
-                        tma_load_2d_pair(dst + GG_W_BYTES, &tma_x128, lbar, kb * GEMM_BK, x_row);
-                        at = 128;
-                    }
-                    for (; at + 32 <= half; at += 32)
-                        tma_load_2d_pair(dst + GG_W_BYTES + at * (GEMM_BK * 2), &tma_x32, lbar, kb * GEMM_BK, x_row + at);
-                    for (; at < half; at += 8)
-                        tma_load_2d_pair(dst + GG_W_BYTES + at * (GEMM_BK * 2), &tma_x8, lbar, kb * GEMM_BK, x_row + at);
+                    tma_load_2d_pair(dst, &maps.w, lbar, kb * GEMM_BK, w_row);
+                    tma_load_2d_pair(dst + GG_W_BYTES, &maps.x[b0], lbar, kb * GEMM_BK, x_row);
+                    if (b1 >= 0)
+                        tma_load_2d_pair(dst + GG_W_BYTES + (8 << b0) * (GEMM_BK * 2), &maps.x[b1], lbar, kb * GEMM_BK, x_row + (8 << b0));
                 }
             }
             // no copy may be in flight when the pair exits: the leader's barriers cover both CTAs
@@ -200,12 +212,12 @@ using namespace pie;
 extern "C" int pie_make_tma_2d_bf16(CUtensorMap* map, const void* ptr, long rows, long cols, long ld, int box_rows);
 
 template <int EPI>
-static int launch_grouped(const CUtensorMap& tw, const CUtensorMap (&tx)[3], void* C, int N, int K, int ldc, int* status, int pairs,
+static int launch_grouped(const GroupedMaps& maps, void* C, int N, int K, int ldc, int* status, int pairs,
                           const GroupedWork& work, const EpiArgs& ex, cudaStream_t st) {
     auto kern = gemm_grouped_kernel<EPI>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM);
     if (e != cudaSuccess) return (int)e;
-    e = launch_pdl(kern, dim3(2 * pairs), dim3(GEMM_THREADS), GG_SMEM, st, tw, tx[0], tx[1], tx[2], (bf16*)C, N, K, ldc, status, work, ex);
+    e = launch_pdl(kern, dim3(2 * pairs), dim3(GEMM_THREADS), GG_SMEM, st, maps, (bf16*)C, N, K, ldc, status, work, ex);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
@@ -220,17 +232,17 @@ static int grouped_gemm(const void* A, const void* W, void* C, const int* tile_e
     if (K <= 0 || K % 8 || N % 8 || ldc % 8) return (int)cudaErrorInvalidValue;
     if ((epilogue == EPI_SWIGLU || epilogue == EPI_CLAMP_GLU) && N % 32) return (int)cudaErrorInvalidValue;
     const long rows = (long)max_mtiles * GEMM_BM;
-    CUtensorMap tw, tx[3];
-    if (pie_make_tma_2d_bf16(&tw, W, (long)num_experts * N, K, K, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
-    for (int i = 0; i < 3; ++i)
-        if (pie_make_tma_2d_bf16(&tx[i], A, rows, K, lda, i == 0 ? 8 : i == 1 ? 32 : 128) != 0) return (int)cudaErrorInvalidValue;
+    GroupedMaps maps;
+    if (pie_make_tma_2d_bf16(&maps.w, W, (long)num_experts * N, K, K, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
+    for (int i = 0; i < 5; ++i)
+        if (pie_make_tma_2d_bf16(&maps.x[i], A, rows, K, lda, 8 << i) != 0) return (int)cudaErrorInvalidValue;
     const long items = (long)max_mtiles * ((N + 2 * GEMM_BM - 1) / (2 * GEMM_BM));
     const int pairs = (int)(items < num_sms / 2 ? items : num_sms / 2);
     const GroupedWork work{tile_expert, tile_list, max_mtiles};
     switch (epilogue) {
-        case EPI_STORE: return launch_grouped<EPI_STORE>(tw, tx, C, N, K, ldc, status, pairs, work, ex, st);
-        case EPI_SWIGLU: return launch_grouped<EPI_SWIGLU>(tw, tx, C, N, K, ldc, status, pairs, work, ex, st);
-        case EPI_CLAMP_GLU: return launch_grouped<EPI_CLAMP_GLU>(tw, tx, C, N, K, ldc, status, pairs, work, ex, st);
+        case EPI_STORE: return launch_grouped<EPI_STORE>(maps, C, N, K, ldc, status, pairs, work, ex, st);
+        case EPI_SWIGLU: return launch_grouped<EPI_SWIGLU>(maps, C, N, K, ldc, status, pairs, work, ex, st);
+        case EPI_CLAMP_GLU: return launch_grouped<EPI_CLAMP_GLU>(maps, C, N, K, ldc, status, pairs, work, ex, st);
         default: return (int)cudaErrorInvalidValue;
     }
 }

@@ -25,10 +25,6 @@ constexpr int SKINNY_MAX_STAGES = 8;
 constexpr uint32_t SKINNY_RING = 108 * 1024;                   // two CTAs per SM
 constexpr uint32_t SKINNY_SMEM = SKINNY_RING + 1024 /*align*/ + 256 /*barriers*/;
 
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // tma_w walks the weights in boxes of 128 rows, tma_x the batch in boxes of all its rows.
 // splits = CTAs of a cluster, each with its share of K; with splits > 1 the grid is one cluster per tile.
 template <int EPI>
