@@ -17,6 +17,21 @@ using namespace pie_host;
 PYBIND11_MODULE(pie_host, m) {
     m.doc() = "native host runtime of pie_b200";
 
+    // `count` byte strings of `size` bytes with writable views of them, to be filled before anyone else sees the strings.
+    // Their pages are touched here: while the GPU works, and not when its results are there to be copied.
+    m.def("fresh_bytes", [](size_t count, size_t size) {
+        py::list strings, views;
+        for (size_t i = 0; i < count; ++i) {
+            PyObject* b = PyBytes_FromStringAndSize(nullptr, (Py_ssize_t)size);
+            if (!b) throw py::error_already_set();
+            strings.append(py::reinterpret_steal<py::bytes>(b));
+            char* at = PyBytes_AS_STRING(b);
+            for (size_t j = 0; j < size; j += 4096) at[j] = 0;
+            views.append(py::memoryview::from_memory(at, (Py_ssize_t)size));
+        }
+        return py::make_tuple(strings, views);
+    }, py::arg("count"), py::arg("size"));
+
     // ------------------------------------------------------------------ BRLE
     m.def("brle_encode", [](py::array_t<bool, py::array::c_style | py::array::forcecast> bits) {
         return brle_encode(reinterpret_cast<const uint8_t*>(bits.data()), (size_t)bits.size());

@@ -132,6 +132,18 @@ class _Graph:
     launches: int = 0
 
 
+def _rows_as_bytes(t: torch.Tensor) -> List[bytes]:
+    """Each row of a float32 matrix as its bytes. From a device they are copied straight into the strings, whose memory is made
+    while the device still works."""
+    if not t.is_cuda or t.numel() == 0:
+        return [row.tobytes() for row in t.cpu().numpy()]
+    from .._C import pie_host
+    strings, views = pie_host.fresh_bytes(t.shape[0], t.shape[1] * 4)
+    for row, view in zip(t, views):
+        torch.from_numpy(np.frombuffer(view, np.float32)).copy_(row)
+    return strings
+
+
 class TorchDriver:
     """PyTorch + sm_100a-kernel model driver for one tensor-parallel rank."""
 
@@ -834,30 +846,32 @@ class TorchDriver:
     def _probes(self, req, logits, slot_logit_row, probe_slots, out_slots):
         """Probe slots (distribution, raw logits, log-probabilities of labels, entropy) of one fire, batched per kind:
         one pass of device work and one device-to-host copy per kind, whatever the number of slots."""
-        rows = torch.from_numpy(slot_logit_row[probe_slots].astype(np.int64)).to(logits.device)
-        lg = logits[rows]
+        rows = slot_logit_row[probe_slots].astype(np.int64)
+        whole = len(rows) == logits.shape[0] and bool((rows == np.arange(len(rows))).all())
+        lg = logits if whole else logits[torch.from_numpy(rows).to(logits.device)]      # an index copied to the device waits for it
         if self.model.sharded_logits:       # probes read whole rows: gather the few rows they name
             lg = self.par.comm.all_gather_logits(lg)
         lg = lg.contiguous()
-        stats = ops.row_stats(lg).float().cpu().numpy()            # max, log-sum-exp, entropy per row
         by_kind: Dict[int, list] = {}
         for j, i in enumerate(probe_slots):
             by_kind.setdefault(int(req.slot_samplers[i].kind), []).append((j, i))
         dev = lg.device
+        stats = None                                               # max, log-sum-exp, entropy per row
+        if any(kind in (SamplerKind.LOGPROB, SamplerKind.LOGPROBS, SamplerKind.ENTROPY) for kind in by_kind):
+            stats = ops.row_stats(lg).float().cpu().numpy()
         for kind, members in by_kind.items():
-            js = torch.tensor([j for j, _ in members], dtype=torch.long, device=dev)
+            mine = lambda: lg if len(by_kind) == 1 else lg[torch.tensor([j for j, _ in members], dtype=torch.long, device=dev)]
             sps = [req.slot_samplers[i] for _, i in members]
             if kind == SamplerKind.DIST:
                 temp = torch.tensor([sp.temperature if sp.temperature > 0 else 1.0 for sp in sps], dtype=torch.float32, device=dev)
                 ks = [min(sp.top_k if sp.top_k > 0 else 32, lg.shape[1]) for sp in sps]
-                pv, pi = torch.topk(torch.softmax(lg[js].float() / temp[:, None], -1), max(ks))
+                pv, pi = torch.topk(torch.softmax(mine().float() / temp[:, None], -1), max(ks))
                 pv, pi = pv.cpu().numpy(), pi.cpu().numpy()
                 for n, (_, i) in enumerate(members):
                     out_slots[i] = SlotOutput("distribution", ids=pi[n, :ks[n]].tolist(), probs=pv[n, :ks[n]].tolist())
             elif kind == SamplerKind.RAW_LOGITS:
-                raw = lg[js].float().cpu().numpy()
-                for n, (_, i) in enumerate(members):
-                    out_slots[i] = SlotOutput("logits", logits=raw[n].tobytes())
+                for (_, i), data in zip(members, _rows_as_bytes(mine().float())):
+                    out_slots[i] = SlotOutput("logits", logits=data)
             elif kind in (SamplerKind.LOGPROB, SamplerKind.LOGPROBS):
                 counts = [len(sp.labels) for sp in sps]
                 row_of = torch.tensor([j for (j, _), c in zip(members, counts) for _ in range(c)], dtype=torch.long, device=dev)

@@ -268,6 +268,7 @@ def _to_i32(packed_i64):
 
 # --------------------------------------------------------------------------- GEMM
 _GEMM_WS = {}
+_GEMM_DEV = {}      # device index -> (status word's address, multiprocessors)
 
 
 def ensure_gemm_workspace(device) -> None:
@@ -323,10 +324,13 @@ def gemm(x, w, residual=None, epilogue: int = EPI_STORE, out=None, force_bn: int
         out = torch.empty(m, n_out, dtype=x.dtype, device=x.device)
     if m == 0:
         return out
-    ensure_gemm_workspace(x.device)
+    at = _GEMM_DEV.get(x.get_device())
+    if at is None:
+        ensure_gemm_workspace(x.device)
+        at = _GEMM_DEV[x.get_device()] = (ptr(kernel_status(x.device)), num_sms(x.device))
     check(fn("pie_gemm_bf16")(ptr(x), ptr(w), ptr(out), ptr(residual), m, n, k, x.stride(0), w.stride(0),
                               out.stride(0), residual.stride(0) if residual is not None else 0, epilogue,
-                              force_bn, ptr(kernel_status(x.device)), num_sms(x.device), stream_ptr()),
+                              force_bn, *at, stream_ptr()),
           "gemm_bf16")
     return out
 

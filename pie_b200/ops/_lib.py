@@ -172,11 +172,16 @@ def load(required: bool = True):
         return _LIB
 
 
+_FNS = {}
+
+
 def fn(name: str):
-    lib = load(required=True)
-    f = getattr(lib, name, None)
+    f = _FNS.get(name)
     if f is None:
-        raise KernelLibraryError(f"symbol {name} not found in {_LIB_PATH}; rebuild the kernel library")
+        f = getattr(load(required=True), name, None)
+        if f is None:
+            raise KernelLibraryError(f"symbol {name} not found in {_LIB_PATH}; rebuild the kernel library")
+        _FNS[name] = f
     return f
 
 
@@ -189,6 +194,9 @@ def declare(name: str, argtypes, restype=i32):
 
 
 def stream_ptr() -> int:
+    """The current stream's handle, without the stream object: that costs more than a launch (3 us), once per kernel."""
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     return torch.cuda.current_stream().cuda_stream
 
 
