@@ -20,6 +20,8 @@
 // fp8 weights (driver/cuda/src/ops/gemm.cpp:1166-1211, driver/cuda/src/kernels/dequant_fp8.cu:41).
 #include <cuda_fp8.h>
 
+#include <algorithm>
+
 #include "gemm_common.cuh"
 
 namespace pie {
@@ -238,12 +240,243 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     }
 }
 
+// ------------------------------------------------------------------------------------------ batches of up to 64 rows
+// Laid out for streaming the weights, as the bf16 kernel for such batches (gemm_skinny.cu): operands swapped (weight rows are
+// the MMA's rows, the batch its 16..64 columns), half an SM per CTA, the ring filled with weights before the producing kernel is
+// done. K is not split: the sum over its blocks keeps the order of the kernel above, because the next layer's quantiser turns a
+// last bit into a step of 8-bit numbers. (Split over clusters, 48 rows against 5120 x 25600 took 47 us instead of 96; results of
+// one layer then agree to 3e-5, logits of four layers only to 4 %.) Instead a tile has as few weight rows as fill the machine
+// (`height`): the MMA's other rows are whatever shared memory holds, each reaches its own accumulator row alone, and these are
+// not read.
+//
+// What block scaling adds: every 128 of K has a partial product of its own in tensor memory (four of them in flight), which the
+// epilogue warps scale and add up in registers - warp w the 32 features of quarter w % 4 and every other group of 16 tokens.
+// The scales of features and tokens come through shared memory, four K blocks at a time and three such chunks ahead.
+//
+// 48 rows against 51200 x 5120 (gate / up): 120 us with 128-row boxes of activations that are zero-filled row by row, weight scales
+// gathered per K block and 400 tiles on 148 SMs; 71 us (3.8 TB/s) like this.
+constexpr int F8S_THREADS = 64 + 256, F8S_CHUNK = 4;
+constexpr uint32_t F8S_MMA_BYTES = GEMM_BM * F8_BK;          // what an MMA reads from a slot's start on
+constexpr int F8S_DEPTH = 4;                                   // chunks of scales: one in use, three on their way
+constexpr uint32_t F8S_RING = 96 * 1024;
+constexpr uint32_t F8S_SCALES = F8S_DEPTH * F8S_CHUNK * (64 + GEMM_BM) * 4;
+constexpr uint32_t F8S_SMEM = F8S_RING + F8S_SCALES + 1024 /*align*/ + 512 /*barriers*/;
+constexpr int F8S_MAX_STAGES = 12;
+
+// height: weight rows of a tile and of its box, a multiple of 8.
+template <int EPI>
+__global__ void __launch_bounds__(F8S_THREADS, 2)
+gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x,
+                       const float* __restrict__ sa, const float* __restrict__ sw, bf16* __restrict__ C, const bf16* __restrict__ R,
+                       int M, int N, int K, int ldc, int ldr, int* status, int stages, int height) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_addr(smem_raw);
+    const uint32_t ring = (raw + 1023u) & ~1023u;
+    uint8_t* ring_ptr = smem_raw + (ring - raw);
+    float* sx = reinterpret_cast<float*>(ring_ptr + F8S_RING);           // [F8S_DEPTH][F8S_CHUNK][64]
+    float* swt = sx + F8S_DEPTH * F8S_CHUNK * 64;                        // [F8S_DEPTH][128 features][F8S_CHUNK]
+    const uint32_t bar0 = ring + F8S_RING + F8S_SCALES;
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (F8S_MAX_STAGES + s); };
+    auto tfull_bar = [&](int a) { return bar0 + 8u * (2 * F8S_MAX_STAGES + a); };
+    auto tempty_bar = [&](int a) { return bar0 + 8u * (2 * F8S_MAX_STAGES + 4 + a); };
+    volatile uint32_t* tmem_slot =
+        reinterpret_cast<volatile uint32_t*>(ring_ptr + F8S_RING + F8S_SCALES + 8 * (2 * F8S_MAX_STAGES + 8));
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cols = (M + 15) / 16 * 16, groups = cols / 16;
+    const uint32_t w_bytes = (uint32_t)height * F8_BK, slot_bytes = w_bytes + (uint32_t)cols * F8_BK, slot_tx = (uint32_t)(height + M) * F8_BK;
+    constexpr uint32_t bufs = 4, buf_cols = 64;
+    const int tiles = (N + height - 1) / height, num_kb = (K + F8_BK - 1) / F8_BK;
+    const int tile0 = blockIdx.x, tile_step = gridDim.x;
+    const int quarters = (height + 31) / 32;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (uint32_t a = 0; a < bufs; ++a) {
+            mbar_init(tfull_bar(a), 1);
+            mbar_init(tempty_bar(a), 2 * quarters);
+        }
+        fence_barrier_init();
+        fence_proxy_async();
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_addr(const_cast<uint32_t*>(tmem_slot)), 256);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            tma_prefetch_desc(&tma_w);
+            tma_prefetch_desc(&tma_x);
+            // the weights depend on nothing and fill the ring at once; the batch's tiles follow when the producing kernel is done
+            int s = 0, parked = 0, parked_kb = 0;
+            uint32_t ph = 0, issued = 0;
+            bool ok = true, ready = false;
+            auto resolve = [&]() {
+                pdl_wait();
+                for (int j = 0; j < parked; ++j) {
+                    tma_load_2d(ring + j * slot_bytes + w_bytes, &tma_x, full_bar(j), parked_kb * F8_BK, 0);
+                    if (++parked_kb == num_kb) parked_kb = 0;
+                }
+                ready = true;
+            };
+            for (int tile = tile0; tile < tiles && ok; tile += tile_step) {
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    if (!ready && issued == (uint32_t)stages) resolve();
+                    if (!mbar_wait(empty_bar(s), ph ^ 1u, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
+                    const uint32_t dst = ring + s * slot_bytes;
+                    mbar_arrive_expect_tx(full_bar(s), slot_tx);
+                    tma_load_2d(dst, &tma_w, full_bar(s), kb * F8_BK, tile * height);
+                    if (ready) tma_load_2d(dst + w_bytes, &tma_x, full_bar(s), kb * F8_BK, 0);
+                    else ++parked;
+                    ++issued;
+                    if (++s == stages) { s = 0; ph ^= 1u; }
+                }
+            }
+            if (!ready) resolve();
+            // no copy may be in flight when the CTA exits
+            const uint32_t first = issued > (uint32_t)stages ? issued - stages : 0u;
+            for (uint32_t j = first; j < issued; ++j)
+                mbar_wait(full_bar(j % stages), (j / stages) & 1u, status, PIE_ERR_WAIT_TMA, 200000000ll);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc_e4m3(GEMM_BM, cols);
+            int s = 0;
+            uint32_t ph = 0, buf = 0, bph = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < tiles && ok; tile += tile_step) {
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    if (!mbar_wait(tempty_bar(buf), bph ^ 1u, status, PIE_ERR_WAIT_EPILOGUE) ||
+                        !mbar_wait(full_bar(s), ph, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t wd = make_smem_desc_sw128(ring + s * slot_bytes);
+                    const uint64_t xd = make_smem_desc_sw128(ring + s * slot_bytes + w_bytes);
+#pragma unroll
+                    for (int k = 0; k < F8_BK / 32; ++k) umma_f8(tmem_base + buf * buf_cols, wd + 2u * k, xd + 2u * k, idesc, k != 0);
+                    umma_commit(empty_bar(s));
+                    umma_commit(tfull_bar(buf));
+                    if (++s == stages) { s = 0; ph ^= 1u; }
+                    if (++buf == bufs) { buf = 0; bph ^= 1u; }
+                }
+            }
+        }
+    } else {
+        const int q = warp & 3, half = (warp - 2) >> 2, et = threadIdx.x - 64;
+        const bool vec = num_kb % F8S_CHUNK == 0 && ((uintptr_t)sw & 15) == 0, active = q < quarters;
+        const int chunks = (num_kb + F8S_CHUNK - 1) / F8S_CHUNK, total = (tiles - tile0 + tile_step - 1) / tile_step * chunks;
+        uint32_t buf = 0, bph = 0;
+        bool ok = true;
+        float acc[2][16];                                                // group 2 i + half, token
+        pdl_wait();          // outputs, residual and the tokens' scales may still be in use by the previous kernel
+        auto request = [&](int c) {                                      // one group of copies per chunk, empty past the last one
+            if (c < total) {
+                const int kb = c % chunks * F8S_CHUNK, feat0 = (tile0 + c / chunks * tile_step) * height, b = c % F8S_DEPTH;
+                for (int i = et; i < F8S_CHUNK * cols; i += 256) {
+                    const int tok = i / F8S_CHUNK, j = i % F8S_CHUNK;
+                    const bool live = tok < M && kb + j < num_kb;
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_addr(sx + (b * F8S_CHUNK + j) * 64 + tok)),
+                                 "l"(live ? sa + (size_t)tok * num_kb + kb + j : sa), "r"(live ? 4 : 0) : "memory");
+                }
+                if (vec) {
+                    if (et < height)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(swt + (b * GEMM_BM + et) * F8S_CHUNK)),
+                                     "l"(sw + (size_t)min(feat0 + et, N - 1) * num_kb + kb) : "memory");
+                } else {
+                    for (int i = et; i < height * F8S_CHUNK; i += 256) {
+                        const int f = i / F8S_CHUNK, j = i % F8S_CHUNK;
+                        const bool live = kb + j < num_kb;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_addr(swt + (b * GEMM_BM + f) * F8S_CHUNK + j)),
+                                     "l"(live ? sw + (size_t)min(feat0 + f, N - 1) * num_kb + kb + j : sw), "r"(live ? 4 : 0) : "memory");
+                    }
+                }
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+        for (int c = 0; c < F8S_DEPTH - 1; ++c) request(c);
+        for (int c = 0; c < total; ++c) {
+            const int tile = tile0 + c / chunks * tile_step, kb = c % chunks * F8S_CHUNK, b = c % F8S_DEPTH;
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(F8S_DEPTH - 2) : "memory");
+            asm volatile("bar.sync 1, 256;\n" ::: "memory");             // a warp whose wait ran out still comes here
+            request(c + F8S_DEPTH - 1);
+            if (!active) continue;
+            if (kb == 0) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) acc[i][t] = 0.f;
+            }
+            const float4 of = *reinterpret_cast<const float4*>(swt + (b * GEMM_BM + q * 32 + lane) * F8S_CHUNK);
+            const float mine[F8S_CHUNK] = {of.x, of.y, of.z, of.w};
+#pragma unroll
+            for (int j = 0; j < F8S_CHUNK; ++j) {
+                if (kb + j >= num_kb) break;
+                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(buf), bph, status, PIE_ERR_WAIT_MMA));
+                if (ok) {
+                    tc_fence_after();
+                    const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * buf_cols;
+                    const float* scales = sx + (b * F8S_CHUNK + j) * 64;
+                    uint32_t v[2][16];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        if (2 * i + half < groups) tmem_ld_32x16(t_row + (2 * i + half) * 16, v[i]);
+                    tmem_ld_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty_bar(buf));
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int g = 2 * i + half;
+                        if (g >= groups) break;
+#pragma unroll
+                        for (int t = 0; t < 16; t += 4) {
+                            const float4 f = *reinterpret_cast<const float4*>(scales + g * 16 + t);
+                            acc[i][t] = fmaf(__uint_as_float(v[i][t]), f.x * mine[j], acc[i][t]);
+                            acc[i][t + 1] = fmaf(__uint_as_float(v[i][t + 1]), f.y * mine[j], acc[i][t + 1]);
+                            acc[i][t + 2] = fmaf(__uint_as_float(v[i][t + 2]), f.z * mine[j], acc[i][t + 2]);
+                            acc[i][t + 3] = fmaf(__uint_as_float(v[i][t + 3]), f.w * mine[j], acc[i][t + 3]);
+                        }
+                    }
+                }
+                if (++buf == bufs) { buf = 0; bph ^= 1u; }
+            }
+            if (kb + F8S_CHUNK >= num_kb && ok) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int g = 2 * i + half;
+                    if (g >= groups) break;
+                    skinny_store<EPI>(acc[i], tile * height + q * 32 + lane, g * 16, min(N, (tile + 1) * height), M, C, ldc, R, ldr, EpiArgs(),
+                                      XieluCoef(nullptr));
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 256);
+    }
+}
+
 // 1 x 128 activation quantisation: one warp per (row, 128-column block).
 __global__ void quant_act_fp8_kernel(const bf16* __restrict__ x, int ldx, uint8_t* __restrict__ x8, float* __restrict__ sx,
                                      int M, int K) {
     const int kbs = (K + 127) / 128;
     const long gw = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    pdl_trigger();
+    pdl_wait();
     if (gw >= (long)M * kbs) return;
     const int row = (int)(gw / kbs), kb = (int)(gw - (long)row * kbs);
     const int c = kb * 128 + lane * 4;
@@ -303,8 +536,8 @@ PIE_API int pie_quant_act_fp8(const void* x, int ldx, void* x8, float* sx, int M
     if (K % 16 || ldx % 4) return (int)cudaErrorInvalidValue;
     const long warps = (long)M * ((K + 127) / 128);
     const int blocks = (int)((warps * 32 + 255) / 256);
-    quant_act_fp8_kernel<<<blocks, 256, 0, st>>>((const bf16*)x, ldx, (uint8_t*)x8, sx, M, K);
-    return (int)cudaGetLastError();
+    const cudaError_t e = launch_pdl(quant_act_fp8_kernel, dim3(blocks), dim3(256), 0, st, (const bf16*)x, ldx, (uint8_t*)x8, sx, M, K);
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 // C[M,N] (or [M,N/2] with SwiGLU) from fp8 operands and their scales (see the header comment).
@@ -331,6 +564,39 @@ PIE_API int pie_gemm_fp8_blockscaled_tp(const void* A8, const float* sa, const v
     return gemm_fp8_launch(A8, sa, W8, sw, C, nullptr, M, N, K, ldc, 0, epilogue, status, num_sms, st, tp);
 }
 
+// Weight rows of a tile: whole rounds of the machine (two CTAs per SM) of as little as possible, a CTA's work being its weight
+// rows, the batch's rows (from L2: at 0.4) and what a tile costs beside them. 48 rows: 5120 features in 214 tiles of 24 rows,
+// 10240 in 256 of 40, 51200 in two rounds of 88 (and not 400 tiles of 128 on 296 places).
+static int fp8_skinny_height(int M, int N, int num_sms) {
+    int height = GEMM_BM;
+    double best = 0.;
+    for (int h = GEMM_BM; h >= 16; h -= 8) {
+        const long rounds = ((N + h - 1) / h + 2 * num_sms - 1) / (2 * num_sms);
+        const double cost = (double)rounds * (h + 0.4 * M + 6.);
+        if (h == GEMM_BM || cost < best) { best = cost; height = h; }
+    }
+    return height;
+}
+
+template <int EPI>
+static int launch_fp8_skinny(const void* A8, const float* sa, const void* W8, const float* sw, void* C, const void* R, int M, int N, int K,
+                             int ldc, int ldr, int* status, int num_sms, cudaStream_t st) {
+    const int height = fp8_skinny_height(M, N, num_sms);
+    CUtensorMap tw, tx;
+    if (make_tma_2d_u8(&tw, W8, N, K, K, height) != 0) return (int)cudaErrorInvalidValue;
+    if (make_tma_2d_u8(&tx, A8, M, K, K, M) != 0) return (int)cudaErrorInvalidValue;      // the box ends with the batch
+    auto kern = gemm_fp8_skinny_kernel<EPI>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F8S_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    const int tiles = (N + height - 1) / height;
+    // an MMA reads 128 rows from the last slot's start, too: they have to lie in the ring
+    const uint32_t slot = (uint32_t)(height + (M + 15) / 16 * 16) * F8_BK;
+    const int stages = (int)std::min({(uint32_t)F8S_MAX_STAGES, F8S_RING / slot, (F8S_RING - F8S_MMA_BYTES) / slot + 1});
+    e = launch_pdl(kern, dim3(std::min(tiles, 2 * num_sms)), dim3(F8S_THREADS), F8S_SMEM, st, tw, tx, sa, sw, (bf16*)C, (const bf16*)R, M, N, K,
+                   ldc, ldr, status, stages, height);
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
 static int gemm_fp8_launch(const void* A8, const float* sa, const void* W8, const float* sw, void* C,
                            const void* R, int M, int N, int K, int ldc, int ldr, int epilogue, int* status,
                            int num_sms, cudaStream_t st, const TpArgs& tp) {
@@ -338,6 +604,14 @@ static int gemm_fp8_launch(const void* A8, const float* sa, const void* W8, cons
     if (K <= 0 || K % 16 || N % 16 || (epilogue != EPI_RS && ldc % 8) || (epilogue == EPI_RESIDUAL && ldr % 8))
         return (int)cudaErrorInvalidValue;
     if (epilogue == EPI_SWIGLU && N % 32) return (int)cudaErrorInvalidValue;
+    // The form for small batches where its tiles are tall or the batch is very small: 48 rows against 51200 features 120 -> 71 us,
+    // 8 rows 135 -> 66 us and against 10240 / 5120 features 36 -> 29 / 95 -> 90 us; but 48 rows against 5120 x 25600 would take
+    // 139 us instead of 96, for 214 tiles of 24 rows then wait for the same rows of the batch in L2.
+    if (M <= 64 && N >= 128 && K >= 512 && (M <= 16 || fp8_skinny_height(M, N, num_sms) >= 64)) {
+        if (epilogue == EPI_STORE) return launch_fp8_skinny<EPI_STORE>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
+        if (epilogue == EPI_RESIDUAL) return launch_fp8_skinny<EPI_RESIDUAL>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
+        if (epilogue == EPI_SWIGLU) return launch_fp8_skinny<EPI_SWIGLU>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
+    }
     const int tm = (M + GEMM_BM - 1) / GEMM_BM;
     // tile width: the widest of {128, 112, ..., 16} whose tile count fills its waves best
     int bn = 128;

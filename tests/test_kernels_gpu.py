@@ -842,3 +842,24 @@ def test_fp8_dequant_row_lengths(n, k):
     w8 = (torch.randn(n, k, device=DEV) * 100).clamp(-448, 448).to(torch.float8_e4m3fn)
     q = ops.Fp8Linear(w8, torch.rand(n, (k + 127) // 128, device=DEV) + 0.1)
     assert torch.equal(ops.dequant_fp8(q), (w8.float() * q.scale.repeat_interleave(128, 1)[:, :k]).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 128, 512), (15, 160, 528), (16, 5120, 1024), (17, 40000, 640), (48, 22016, 1168), (64, 51200, 512),
+                                   (9, 640, 25600), (65, 40000, 640)])
+@pytest.mark.parametrize("epi", ["store", "residual", "swiglu"])
+def test_fp8_gemm_of_small_batches(m, n, k, epi):
+    """Up to 64 rows: column counts, tile heights, several tiles per CTA, K blocks that are not whole, against the fp32 evaluation
+    of the same operands: one rounding to bf16 (2^-9) of 32-bit sums in another order."""
+    g = torch.Generator(device=DEV).manual_seed(m * 7 + n)
+    w8 = (torch.randn(n, k, device=DEV, generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    q = ops.Fp8Linear(w8, (torch.rand(n, (k + 127) // 128, device=DEV, generator=g) + 0.5) / 50 * k ** -0.5)
+    x = torch.randn(m, k, device=DEV, generator=g).to(torch.bfloat16)
+    r = torch.randn(m, n, device=DEV, generator=g).to(torch.bfloat16) if epi == "residual" else None
+    x8, sx = ops.quant_act_fp8(x)
+    want = ops.gemm_fp8_reference(x8, sx, q)
+    want = want + r.float() if epi == "residual" else ref.swiglu_interleaved(want) if epi == "swiglu" else want
+    code = {"store": ops.EPI_STORE, "residual": ops.EPI_RESIDUAL, "swiglu": ops.EPI_SWIGLU}[epi]
+    y = ops.gemm_fp8w(x, q, residual=r, epilogue=code, mode="fused")
+    torch.cuda.synchronize()
+    ops.check_kernel_status()
+    torch.testing.assert_close(y.float(), want, rtol=2 ** -8, atol=1e-3)
