@@ -68,6 +68,7 @@ struct SampleShared {
     float mass[SAMPLE_BINS];
     uint32_t wcnt[SAMPLE_WARPS];
     float wmass[SAMPLE_WARPS];
+    uint32_t best[4];                              // best score key of a Gumbel pass so far
     int hit;
     uint32_t base_cnt;
     float base_mass;
@@ -168,6 +169,7 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
     rv.rank = blockIdx.x - row * cl;
     const int mr = mask_row ? mask_row[row] : -1;
     rv.mask = (mask_bits && mr >= 0) ? mask_bits + (size_t)mr * mask_words : nullptr;
+    if (tid < 4) sh.best[tid] = 0;                   // seen by all after the first barrier
     rv.count = (rv.nvec + cl * SAMPLE_THREADS - 1) / (cl * SAMPLE_THREADS);
 
     // ---- exchanges within the row's CTAs. A slot is written again two exchanges later: by then every CTA has read it.
@@ -298,13 +300,19 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
             pick = cand > pick ? cand : pick;
         };
         consider(arg, (uint16_t)((kmax & 0x8000u) ? kmax & 0x7fffu : ~kmax));
-        auto bound = [&]() { return pick ? ex2(f32_of_key((uint32_t)(pick >> 32)) * -LOG2E) * 1.0001f : INFINITY; };
-        float B = bound();
+        uint32_t seen = (uint32_t)(pick >> 32);      // the largest score this thread knows of
+        float B = seen ? ex2(f32_of_key(seen) * -LOG2E) * 1.0001f : INFINITY;
+        volatile uint32_t* shared_best = &sh.best[salt & 3];
         const float xlow = fmaxf(sortable_value((int)lo - 0x8000), x_floor);    // necessary for key >= lo, not sufficient
         float z = 0.f;
         const bool all = Z || xlow == -INFINITY;
         rv.scan([&](int idx0, const uint4& p) {
             if (!all && !__any_sync(0xffffffffu, !(sortable_value(rv.top(p)) < xlow))) return;
+            const uint32_t others = *shared_best;    // one score found anywhere in the CTA spares the other warps theirs
+            if (others > seen) {
+                seen = others;
+                B = ex2(f32_of_key(seen) * -LOG2E) * 1.0001f;
+            }
             const uint32_t hb = ((uint32_t)idx0 + from) * 0x9E3779B1u;
             auto passes = [&](int k, float w) {
                 uint32_t hsh = (hb + (uint32_t)k * 0x9E3779B1u) ^ s1;
@@ -329,7 +337,11 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
                 }
                 __syncwarp();
                 const uint32_t high = __reduce_max_sync(0xffffffffu, (uint32_t)(pick >> 32));
-                if (high) B = ex2(f32_of_key(high) * -LOG2E) * 1.0001f;
+                if (high > seen) {
+                    seen = high;
+                    B = ex2(f32_of_key(seen) * -LOG2E) * 1.0001f;
+                    if (lane == 0) atomicMax(&sh.best[salt & 3], seen);
+                }
             }
         });
         if (Z) *Z = z;
