@@ -61,7 +61,8 @@ __device__ __forceinline__ void grouped_boxes(int rows, int& first, int& second)
 
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_grouped_kernel(const __grid_constant__ GroupedMaps maps, bf16* __restrict__ C, int N, int K, int ldc, int* status, const GroupedWork work, const __grid_constant__ EpiArgs ex) {
+gemm_grouped_kernel(const __grid_constant__ GroupedMaps maps, bf16* __restrict__ C, int N, int K, int ldc, int* status,
+                    const GroupedWork work, const __grid_constant__ EpiArgs ex) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t ring = (raw + 1023u) & ~1023u;
