@@ -434,6 +434,10 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
             });
             Z = row_sums().x;
         }
+        if (need_p && 0.f >= P * Z) {                 // top-p of nothing: the arg-max, also where others equal it
+            if (writer) out_tokens[row] = arg;
+            return;
+        }
         const uint32_t cnt0 = (uint32_t)__cvta_generic_to_shared(&sh.cnt[0]), mass0 = (uint32_t)__cvta_generic_to_shared(&sh.mass[0]);
         uint32_t base_cnt = 0;
         float base_mass = 0.f;

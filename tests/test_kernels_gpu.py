@@ -887,3 +887,14 @@ def test_sample_does_not_depend_on_the_batch_or_the_run(vocab, k, base):
     for step in (1, 40, 148):
         got = torch.cat([one(slice(a, min(a + step, rows))) for a in range(0, rows, step)])
         assert torch.equal(got, want), (step, int((got != want).sum()))
+
+
+def test_sample_top_p_of_nothing_is_the_arg_max():
+    """top_p = 0 keeps no mass: the lowest index of the largest entries, however many are equal and whatever else is asked for."""
+    rows, vocab = 40, 32000
+    lg = bf(rows, vocab, scale=2.0, seed=77)
+    for r in range(rows):
+        lg[r, torch.randperm(vocab, device=DEV)[: 1 + r * 7]] = 30.0
+    want = torch.stack([(lg[r] == 30.0).nonzero()[0, 0] for r in range(rows)])
+    for t, k, mp in ((1.0, 0, 0.0), (0.7, 50, 0.0), (5.0, 0, 0.1)):
+        assert torch.equal(ops.sample(lg, *_params(rows, t, k, 0.0, mp)).long(), want)

@@ -128,6 +128,25 @@ def test_sharded_sampler_honours_vocabulary_masks():
         assert all(tok[i] == vocab - 7 for i in range(rows) if mr[i] == 2)
 
 
+def test_sharded_sampler_with_equal_largest_entries():
+    """top_p = 0 and top-k among entries that equal the largest, spread over the shards: the single-GPU sampler's tokens."""
+    world, vl, rows = 4, 2048, 21
+    emu = Emu(world, vl, grid_max=8, rows_max=32)
+    lg = make_logits(rows, world * vl, 9, False)
+    g = torch.Generator().manual_seed(2)
+    for r in range(rows):
+        lg[r, torch.randperm(world * vl, generator=g)[: 1 + 5 * r].to(DEV)] = 6.0
+    first = torch.stack([(lg[r] == 6.0).nonzero()[0, 0] for r in range(rows)])
+    for top_k, top_p in ((0, 0.0), (30, 0.0), (1, 1.0), (0, 0.01)):
+        pr = params(rows, "top_p", 21)
+        pr[1][:], pr[2][:] = top_k, top_p
+        want = ops.sample(lg, *pr)
+        got = emu.sample(lg, *pr)
+        assert torch.equal(got[0], want) and torch.equal(got[-1], want)
+        if top_p == 0.0:
+            assert torch.equal(want.long(), first)
+
+
 def test_sharded_sampler_distribution():
     """Temperature sampling draws from softmax(logits): chi-square-free sanity check on a tiny vocabulary."""
     world, vl = 2, 8
