@@ -293,7 +293,7 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
     // per-row stream keys from the 64-bit seed; per-element noise is one 32-bit mix of the index
     const unsigned long long seed = splitmix64(seeds[row]);
     const uint32_t s0 = (uint32_t)seed, s1 = (uint32_t)(seed >> 32);
-    const float c1 = inv_t * LOG2E;
+    const float c1 = inv_t == 0.f ? 0x1p-126f : inv_t * LOG2E;         // at an infinite temperature -inf still weighs nothing
     auto weight = [&](float x) { return ex2((x - xmax) * c1); };       // relative to the largest entry's
     auto mix = [&](uint32_t hsh) {
         hsh ^= s1;

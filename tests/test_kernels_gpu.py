@@ -898,3 +898,20 @@ def test_sample_top_p_of_nothing_is_the_arg_max():
     want = torch.stack([(lg[r] == 30.0).nonzero()[0, 0] for r in range(rows)])
     for t, k, mp in ((1.0, 0, 0.0), (0.7, 50, 0.0), (5.0, 0, 0.1)):
         assert torch.equal(ops.sample(lg, *_params(rows, t, k, 0.0, mp)).long(), want)
+
+
+def test_sample_at_an_infinite_temperature():
+    """All allowed entries weigh the same, entries outside the mask and past the row's end nothing: top-p keeps that share of the keys."""
+    rows, vocab = 64, 1000
+    lg = torch.randperm(vocab, device=DEV).float().mul(0.25).to(torch.bfloat16).repeat(rows, 1)
+    allowed = torch.zeros(vocab, dtype=torch.bool, device=DEV)
+    allowed[::2] = True
+    words = torch.zeros(32 * 32, dtype=torch.int64, device=DEV)
+    words[:vocab] = allowed
+    words = (words.view(32, 32) << torch.arange(32, device=DEV)).sum(1)
+    mask = torch.where(words >= 2 ** 31, words - 2 ** 32, words).int()[None]
+    for p in (0.2, 0.6):
+        got = ops.sample(lg, *_params(rows, math.inf, 0, p, 0.0), mask_bits=mask, mask_row=torch.zeros(rows, dtype=torch.int32, device=DEV)).long()
+        x = lg[0].float()
+        higher = torch.stack([(allowed & (x > x[g])).sum() for g in got])
+        assert bool(allowed[got].all()) and bool((higher < p * allowed.sum()).all()) and len(got.unique()) > 20
