@@ -20,7 +20,8 @@ enum GemmEpilogue : int {
     EPI_GEGLU = 7,     // as EPI_SWIGLU with the tanh form of GELU on the gate
 };
 
-// Operands of the epilogues with a bias. xIELU(z) = a z^2 + z / 2 for z > 0, b (e^z - 1 - z) + z / 2 below, with
+// What a launch needs beside its matrices: operands of the epilogues with a bias, and whether the weights are the output of an
+// earlier launch. xIELU(z) = a z^2 + z / 2 for z > 0, b (e^z - 1 - z) + z / 2 below, with
 // a = softplus(act[0]) and b = 1/2 + softplus(act[1]).
 struct EpiArgs {
     const bf16* bias = nullptr;    // [N], or null
@@ -29,6 +30,7 @@ struct EpiArgs {
     float* out32 = nullptr;
     int ld32 = 0;
     float limit = 0.f;             // EPI_CLAMP_GLU
+    int fresh_w = 0;               // the weights were written by an earlier launch: no load of them ahead of the grid dependency
 };
 
 template <int EPI>

@@ -80,8 +80,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         if (lane == 0) {
             tma_prefetch_desc(&tma_w);
             tma_prefetch_desc(&tma_x);
-            // The weights depend on nothing and fill the ring at once; the batch's tiles follow when the producing
-            // kernel is done.
+            // Weights that depend on nothing fill the ring at once; the batch's tiles follow when the producing kernel is
+            // done. Weights that an earlier launch wrote (fp8 just expanded) wait like the batch.
             int s = 0, parked = 0, parked_kb = kb0;
             uint32_t ph = 0, issued = 0;
             bool ok = true, ready = false;
@@ -93,6 +93,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 }
                 ready = true;
             };
+            if (ex.fresh_w) resolve();
             for (int tile = tile0; tile < tiles && ok; tile += tile_step) {
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!ready && issued == (uint32_t)stages) resolve();

@@ -107,8 +107,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             tma_prefetch_desc(&tma_b);
             uint32_t it = 0;
             bool ok = true;
-            // The weight tiles depend on nothing: they stream into the ring at once. The activation
-            // tiles wait for the producing kernel (grid dependency) and, under tensor parallelism,
+            // The weight tiles depend on nothing (unless an earlier launch wrote them, ex.fresh_w): they
+            // stream into the ring at once. The activation tiles wait for the producing kernel (grid dependency) and, under tensor parallelism,
             // for every rank's push of the gathered activation; their loads are parked meanwhile.
             bool dep_ready = false;
             int pending = 0;
@@ -127,6 +127,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 pending = 0;
                 dep_ready = true;
             };
+            if (ex.fresh_w) resolve();
             SegmentWalk walk(sk.enabled != 0, num_tiles, num_kb, blockIdx.x, gridDim.x);
             Segment seg;
             while (ok && walk.next(seg)) {
@@ -558,6 +559,8 @@ static int current_workspace(GemmWorkspace* out) {
 
 // C[M,N] (or [M,N/2] for the SwiGLU epilogue) = A[M,K] * W[N,K]^T.
 // `status` is a device int that stays 0 unless a bounded wait ran out.
+// `ex.fresh_w`: W is the output of an earlier launch of the stream. The single-CTA kernels request weights ahead of the grid
+// dependency, and an earlier launch's stores are only sure to be seen behind it. The pair kernel is launched without overlap.
 static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda, int ldw, int ldc, int ldr,
                      int epilogue, int force_bn, int* status, int num_sms, cudaStream_t st, const EpiArgs& ex) {
     if (M <= 0 || N <= 0) return 0;
@@ -584,10 +587,10 @@ static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M
     if (pie_make_tma_2d_bf16(&tb, W, N, K, ldw, plan.bn) != 0) return (int)cudaErrorInvalidValue;
 #define GO(BN_)                                                                                   \
     switch (epilogue) {                                                                           \
-        case EPI_STORE: return launch_gemm<BN_, EPI_STORE>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
-        case EPI_RESIDUAL: return launch_gemm<BN_, EPI_RESIDUAL>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
-        case EPI_SWIGLU: return launch_gemm<BN_, EPI_SWIGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
-        case EPI_GEGLU: return launch_gemm<BN_, EPI_GEGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st); \
+        case EPI_STORE: return launch_gemm<BN_, EPI_STORE>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
+        case EPI_RESIDUAL: return launch_gemm<BN_, EPI_RESIDUAL>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
+        case EPI_SWIGLU: return launch_gemm<BN_, EPI_SWIGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
+        case EPI_GEGLU: return launch_gemm<BN_, EPI_GEGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
         case EPI_XIELU: return launch_gemm<BN_, EPI_XIELU>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
         case EPI_STREAM: return launch_gemm<BN_, EPI_STREAM>(ta, tb, C, R, M, N, K, ldc, ldr, status, plan, bm, w, st, TpArgs{}, ex); \
         default: return (int)cudaErrorInvalidValue;                                               \
@@ -600,10 +603,12 @@ static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M
 }
 
 PIE_API int pie_gemm_bf16(const void* A, const void* W, void* C, const void* R, int M, int N, int K,
-                          int lda, int ldw, int ldc, int ldr, int epilogue, int force_bn,
+                          int lda, int ldw, int ldc, int ldr, int epilogue, int force_bn, int fresh_w,
                           int* status, int num_sms, cudaStream_t st) {
     if ((epilogue < EPI_STORE || epilogue > EPI_SWIGLU) && epilogue != EPI_GEGLU) return (int)cudaErrorInvalidValue;
-    return gemm_bf16(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, force_bn, status, num_sms, st, EpiArgs());
+    EpiArgs ex;
+    ex.fresh_w = fresh_w;
+    return gemm_bf16(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, force_bn, status, num_sms, st, ex);
 }
 
 // C = xIELU(A * W^T + bias): `act` holds the activation's two learned numbers.

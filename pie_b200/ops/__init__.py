@@ -310,8 +310,9 @@ def set_gemm_pairs(enabled: bool) -> None:
     check(fn("pie_gemm_set_pairs")(1 if enabled else 0), "gemm_set_pairs")
 
 
-def gemm(x, w, residual=None, epilogue: int = EPI_STORE, out=None, force_bn: int = 0):
-    """y = x @ w.T (+ residual | SwiGLU or GeGLU over interleaved gate/up columns). x [M,K], w [N,K]."""
+def gemm(x, w, residual=None, epilogue: int = EPI_STORE, out=None, force_bn: int = 0, fresh_w: bool = False):
+    """y = x @ w.T (+ residual | SwiGLU or GeGLU over interleaved gate/up columns). x [M,K], w [N,K]. `fresh_w`: w was written by
+    work that this stream has not waited for (an expanded weight); the kernel then requests none of it ahead of its predecessor's end."""
     if not x.is_cuda:
         y = reference.gemm(x, w, residual if epilogue == EPI_RESIDUAL else None)
         if epilogue == EPI_GEGLU:
@@ -330,7 +331,7 @@ def gemm(x, w, residual=None, epilogue: int = EPI_STORE, out=None, force_bn: int
         at = _GEMM_DEV[x.get_device()] = (ptr(kernel_status(x.device)), num_sms(x.device))
     check(fn("pie_gemm_bf16")(ptr(x), ptr(w), ptr(out), ptr(residual), m, n, k, x.stride(0), w.stride(0),
                               out.stride(0), residual.stride(0) if residual is not None else 0, epilogue,
-                              force_bn, *at, stream_ptr()),
+                              force_bn, int(fresh_w), *at, stream_ptr()),
           "gemm_bf16")
     return out
 
@@ -456,7 +457,7 @@ def gemm_fp8w(x, q: "Fp8Linear", residual=None, epilogue: int = EPI_STORE, mode:
     if buf is None:
         buf = _FP8_SCRATCH[key] = torch.empty(*q.shape, dtype=torch.bfloat16, device=q.device)
     dequant_fp8(q, out=buf)
-    return gemm(x, buf, residual=residual, epilogue=epilogue)
+    return gemm(x, buf, residual=residual, epilogue=epilogue, fresh_w=True)
 
 
 # --------------------------------------------------------------------------- mixture of experts

@@ -156,3 +156,15 @@ def test_gemm_tiles_of_no_more_rows_than_the_batch_has(m, n, k, epi):
             ops.set_gemm_swap(128)
             ops.set_gemm_pairs(True)
         check(y, want, k)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 2048), (100, 1024, 512), (40, 96, 256), (200, 256, 512), (300, 4096, 8192)])
+def test_products_over_expanded_weights_of_one_shape(m, n, k):
+    """Layers of one shape share the memory that their fp8 weights are expanded into: every product reads its own expansion."""
+    x = bf(m, k, seed=51)
+    layers = [ops.quantize_fp8_block(bf(n, k, scale=0.05, seed=52 + i).float()) for i in range(6)]
+    want = [ops.gemm(x, q.dequant()) for q in layers]
+    got = [ops.gemm_fp8w(x, q, mode="dequant") for _ in range(4) for q in layers]
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % len(layers)])
+    ops.check_kernel_status()
