@@ -445,7 +445,7 @@ __device__ __forceinline__ void skinny_store(const float (&v)[16], int feat, int
         if constexpr (EPI == EPI_RESIDUAL) o += add[t];
         if constexpr (EPI == EPI_XIELU) o = act(o + bias);
         if constexpr (EPI == EPI_STREAM) {
-            o = add[t] + o + bias;
+            o = o + bias + add[t];                       // in the order of epilogue_store_64
             ex.out32[(size_t)tok * ex.ld32 + feat] = o;
             if (!C) continue;
         }

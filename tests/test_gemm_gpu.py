@@ -168,3 +168,34 @@ def test_products_over_expanded_weights_of_one_shape(m, n, k):
     for i, y in enumerate(got):
         assert torch.equal(y, want[i % len(layers)])
     ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("n,k", [(256, 512), (1024, 1536), (1536, 1000), (4096, 768)])
+def test_rows_are_the_same_in_the_kernel_for_small_batches(n, k):
+    """Where K is not split (below 2048) a row's result is the same in a small batch's kernel and in the general one, in all epilogues:
+    one order of sums, bias and residual included."""
+    from pie_b200.ops import latent as lops
+    x, w, r, b = bf(129, k, seed=61), bf(n, k, scale=0.03, seed=62), bf(129, n, seed=63), bf(n, seed=64)
+    act = torch.tensor([0.3, -0.2], dtype=torch.bfloat16, device=DEV)
+    stream = torch.randn(129, n, device=DEV, generator=torch.Generator(device=DEV).manual_seed(65)) * 3
+    runs = {
+        "store": lambda m: ops.gemm(x[:m], w),
+        "residual": lambda m: ops.gemm(x[:m], w, residual=r[:m], epilogue=ops.EPI_RESIDUAL),
+        "swiglu": lambda m: ops.gemm(x[:m], w, epilogue=ops.EPI_SWIGLU),
+        "geglu": lambda m: ops.gemm(x[:m], w, epilogue=ops.EPI_GEGLU),
+        "xielu": lambda m: lops.gemm_xielu(x[:m], w, b, act, torch.empty(m, n, dtype=torch.bfloat16, device=DEV)),
+        "stream": lambda m: lops.gemm_stream(x[:m], w, b, stream[:m].clone())[0],
+        "stream without bias": lambda m: lops.gemm_stream(x[:m], w, None, stream[:m].clone())[0],
+    }
+    for name, run in runs.items():
+        if n % 32 and "glu" in name:
+            continue
+        large = run(129)
+        for m, swap in ((1, 128), (40, 128), (128, 128), (128, 1000)):
+            ops.set_gemm_swap(swap)
+            try:
+                small = run(m)
+            finally:
+                ops.set_gemm_swap(128)
+            assert torch.equal(small, large[:m]), (name, m, int((small != large[:m]).sum()))
+    ops.check_kernel_status()
