@@ -25,7 +25,8 @@ constexpr uint32_t GG_SMEM = GG_STAGES * GG_STAGE_BYTES + 1024 /*align*/ + 256 /
 constexpr uint32_t GG_TMEM_COLS = 512;                              // two accumulators of 256 columns
 
 // Work tiles: tile_list[0] of them, entry 1 + i = (first 128-row tile << 9 | rows). Without a list each used 128-row tile is
-// one, with all of its rows.
+// one, with all of its rows. Rows from tile max_mtiles on are left out: the list may be of a call with more, or of more routes than
+// max_mtiles tiles hold, and A, C and tile_expert end there.
 struct GroupedWork {
     const int *tile_expert, *tile_list;
     int max_mtiles;
@@ -36,9 +37,10 @@ struct GroupedTile {
 __device__ __forceinline__ int grouped_count(const GroupedWork& w) { return w.tile_list ? min(w.tile_list[0], w.max_mtiles) : w.max_mtiles; }
 __device__ __forceinline__ bool grouped_tile(const GroupedWork& w, int i, GroupedTile& t) {
     const int entry = w.tile_list ? w.tile_list[1 + i] : (i << 9 | GEMM_BM);
-    t.row0 = (entry >> 9) * GEMM_BM;
-    t.rows = entry & 511;
-    t.expert = w.tile_expert[entry >> 9];
+    const int tile = entry >> 9;
+    t.row0 = tile * GEMM_BM;
+    t.rows = min(entry & 511, (w.max_mtiles - tile) * GEMM_BM);
+    t.expert = (unsigned)tile < (unsigned)w.max_mtiles ? w.tile_expert[tile] : -1;
     return t.expert >= 0;
 }
 

@@ -117,3 +117,32 @@ def test_grouped_gemm_tiles(n, k, epi):
             # one rounding to bf16 (2^-9) of sums whose order differs
             torch.testing.assert_close(out[at:at + rows].float(), y, rtol=2 ** -8, atol=1e-3)
         assert bool((out[~used] == 7.0).all())
+
+
+@pytest.mark.parametrize("aligned", [3, 5, 7])
+def test_grouped_gemm_ends_with_its_tiles(aligned):
+    """More routes than the call's tiles hold, and a work list of a call with more tiles: rows of the tiles are as ever, none past them is
+    read or written."""
+    from pie_b200 import ops
+    dev = torch.device("cuda")
+    counts, k, n, mt = [100, 300, 257], 64, 64, 4
+    g = torch.Generator(device=dev).manual_seed(3)
+    w = (torch.randn(3, n, k, device=dev, generator=g) * k ** -0.5).to(torch.bfloat16)
+    buf = ops.MoeBuffers(sum(counts), k, n, 3, 1, dev)
+    buf.counts.copy_(torch.tensor(counts))
+    buf.xs.normal_(generator=g)
+    ops.moe_align(buf, aligned)
+    used = min(mt, aligned)
+    a = buf.xs[:mt * 128].clone()
+    out = torch.full((buf.xs.shape[0], n), 7.0, dtype=torch.bfloat16, device=dev)
+    ops.grouped_gemm(a, w, buf.tile_expert[:used].clone(), out, used, ops.EPI_STORE, buf.tile_list)
+    torch.cuda.synchronize()
+    ops.check_kernel_status(dev)
+    want = torch.full_like(out, 7.0)
+    for e, (c, at) in enumerate(zip(counts, (0, 128, 512))):
+        end = min(at + c, used * 128)
+        if end > at:
+            y = a[at:end].float() @ w[e].float().t()
+            torch.testing.assert_close(out[at:end].float(), y, rtol=2 ** -8, atol=1e-3)
+            want[at:end] = out[at:end]
+    assert torch.equal(out, want)
