@@ -9,7 +9,8 @@
 //   * at most half of an SM's shared memory and tensor memory per CTA. Two CTAs of one launch share an SM, so uneven tile
 //     counts even out (what bounds the launch is memory, and every resident CTA has the same bytes in flight), and under
 //     programmatic dependent launch the next product's weights stream in while this one's last tiles are stored.
-// The split depends on N and K only: a request's numbers do not change with the batch it runs in.
+// The split depends on N and K only: a request's numbers do not change with the batch it runs in, as long as that batch runs here
+// (see pie_gemm_skinny_rows); where K is not split they are the general kernels' too.
 //
 // Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue (thread = one output feature). Every mbarrier wait is
 // bounded; on a time-out the kernel records a status word and leaves through its normal teardown.
@@ -234,6 +235,24 @@ static int skinny_splits(int N, int K, int num_sms) {
     int s = 1;
     while (K >= 2048 && s < 8 && tiles * 2 * s <= 2 * num_sms && num_kb >= 8 * s) s *= 2;
     return s;
+}
+
+// Most rows of a batch that runs here. Every CTA takes 128 weight rows and the whole batch through one SM, where the general kernel
+// takes narrower tiles on more SMs; from 96 rows on three ring slots are left, and the epilogue has eight groups of tokens. So
+// few tiles or a short K want few rows. Measured with cold caches, this kernel against the general one (us):
+//   K >= 4096:        4096 x 4096 18.5 / 22.5 at 64 rows, 4096 x 14336 41 / 58 at 128; 28672 x 4096 59 / 61 at 64, 61 / 61 at 128
+//   K < 4096, tiles for all SMs or more (weights bound both; uneven rounds count from K = 1536 on):
+//                     51200 x 1536 43 / 47 at 64, 46 / 48 at 128; 28672 x 2040 41 / 39 at 112; 57344 x 768 29 / 31 at 96
+//   K split in 8:     1024 x 2880 14.3 / 20.5 at 112 rows, 4096 x 2048 20.5 / 18.4 at 128 (but 2048 x 2048 16.4 / 18.5)
+//   K split in 4:     6144 x 2880 20.7 / 22.6 at 112, 6144 x 2048 20.4 / 19.3 at 128
+//   K split in 2:     10240 x 2880 and 14336 x 2048 gain up to 12 % at 32 rows, even out at 80, lose 8 % at 112
+//   K not split:      2048 x 1024 14.3 / 14.3 at 48 rows, 16.4 / 14.3 at 96; 4096 x 1536 16.4 / 16.4 at 32, 20.5 / 16.4 at 128
+int pie_gemm_skinny_rows(int N, int K, int num_sms) {
+    if (K >= 4096) return 128;
+    if ((N + GEMM_BM - 1) / GEMM_BM >= num_sms) return K >= 1536 ? 96 : 128;
+    if (K < 2048) return K >= 1536 ? 48 : 64;
+    const int splits = skinny_splits(N, K, num_sms);
+    return splits >= 8 ? 128 : splits == 4 ? 112 : 80;
 }
 
 template <int EPI>

@@ -421,10 +421,9 @@ PIE_API int pie_set_pdl(int enabled) { g_pie_pdl = enabled; return 0; }
 static int g_gemm_pairs = 1;
 PIE_API int pie_gemm_set_pairs(int enabled) { g_gemm_pairs = enabled; return 0; }
 
-// Batches of up to this many rows take the kernel for small batches (0: never; 1000: whatever the shape), where N >= 128 and
-// K >= 512: below, a weight tile's worth of set-up outweighs the streaming. Measured, 1 / 64 / 128 rows: 6144 x 4096 12 / 14 /
-// 17 us against 21 / 22 / 22 us on whole tiles here, 4096 x 14336 22 / 28 / 33 us against 46 / 49 / 53 us, 28672 x 4096
-// 37 / 47 / 55 us against 48 / 50 / 51 us; the last column is the price of one summation order for all batches of a tile.
+// Batches of up to this many rows, and of no more than pie_gemm_skinny_rows says for the shape, take the kernel for small batches
+// (0: never; 1000: whatever the shape), where N >= 128 and K >= 512: below, a weight tile's worth of set-up outweighs the
+// streaming.
 static int g_gemm_swap_max_m = 128;
 PIE_API int pie_gemm_set_swap(int max_m) { g_gemm_swap_max_m = max_m; return 0; }
 
@@ -433,6 +432,7 @@ int pie_gemm2_dispatch(const void* A, const void* W, void* C, const void* R, int
                        const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, int* handled,
                        const EpiArgs& ex = EpiArgs());
 
+int pie_gemm_skinny_rows(int N, int K, int num_sms);
 int pie_gemm_skinny(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda, int ldw, int ldc, int ldr,
                     int epilogue, int* status, int num_sms, cudaStream_t st, const EpiArgs& ex);
 
@@ -575,7 +575,8 @@ static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M
                                           nullptr, w.ws, w.ws_floats, w.cnt, w.cnt_ints, &handled, ex);
         if (handled || rc) return rc;
     }
-    if (force_bn == 0 && M <= GEMM_BM && (g_gemm_swap_max_m >= 1000 || (M <= g_gemm_swap_max_m && N >= 128 && K >= 512)))
+    if (force_bn == 0 && M <= GEMM_BM &&
+        (g_gemm_swap_max_m >= 1000 || (M <= g_gemm_swap_max_m && N >= 128 && K >= 512 && M <= pie_gemm_skinny_rows(N, K, num_sms))))
         return pie_gemm_skinny(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, status, num_sms, st, ex);
     bool allow_sk = true;
     if (force_bn < 0) { allow_sk = false; force_bn = -force_bn == 1 ? 0 : -force_bn; }  // negative: whole-tile only

@@ -300,8 +300,8 @@ def set_pdl(enabled: bool) -> None:
 
 def set_gemm_swap(max_m: int) -> None:
     """Batches of up to max_m rows (default and at most 128) run the kernel for small batches (weights on the 128-row side of
-    the MMA, K split over a cluster) where N >= 128 and K >= 512; 0 turns that off, 1000 takes every shape of up to 128 rows
-    (tests)."""
+    the MMA, K split over a cluster) where N >= 128 and K >= 512 and it is the faster one for their rows; 0 turns that off, 1000
+    takes every shape of up to 128 rows (tests)."""
     fn("pie_gemm_set_swap")(int(max_m))
 
 
