@@ -39,6 +39,8 @@ constexpr int PIE_STATUS_WORDS = 8;
 // pdl_trigger() lets the successor's blocks start as soon as resources free up.
 extern int g_pie_pdl;
 
+constexpr int PIE_SMS = 148;       // of a B200, for launch rules that are not given the device's number
+
 namespace pie {
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

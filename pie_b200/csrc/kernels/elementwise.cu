@@ -138,7 +138,8 @@ __global__ void glu_interleaved_kernel(const bf16* __restrict__ gu, bf16* __rest
 }
 
 // -------------------------------------------- q/k norm + rope + paged KV write
-// One block per token of the packed qkv rows [Hq*d | Hkv*d | Hkv*d], D / 16 lanes per head, each with 8 elements of both halves.
+// Blocks of 256 threads over the packed qkv rows [Hq*d | Hkv*d | Hkv*d], D / 16 lanes per head, each with 8 elements of both halves:
+// 2^per_log tokens per block where a token's heads leave lanes idle, else one, its heads by grid.y blocks in turn.
 // q heads: optional RMSNorm over the head (weight qn[d]) then rotate-half RoPE,
 // written to q_out[t, h, :]. k heads: same with kn, written to the K half of
 // the token's KV slot. v heads: copied to the V half.
@@ -149,19 +150,22 @@ __global__ void glu_interleaved_kernel(const bf16* __restrict__ gu, bf16* __rest
 // VEC: everything lies on 16-byte boundaries; else elements are read and written one by one.
 // Bound by memory. The token's sines and cosines are worked out once and not by every head's warp again, and rows move in
 // 16-byte pieces. 8300 tokens of 32 + 2 x 8 heads of 128, inputs cold: 91 us with a warp per head, 51 us like this (4.0 TB/s);
-// 512 tokens 12.3 and 10.2 us.
+// 512 tokens 12.3 and 10.2 us. 8300 tokens of 4 + 2 heads: 18 us with a warp per head, 29 with a block per token, 16 with four tokens
+// per block; 1 token of 64 + 2 x 8 heads: 8.0 us, 10.4 with its heads in turn, 8.1 with three blocks.
+constexpr int ROPE_ANGLES = 512;          // of a block's tokens
 template <int D, bool KV8, bool VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)
 qk_norm_rope_kvwrite_kernel(const bf16* __restrict__ qkv, const int* __restrict__ positions,
                             const int* __restrict__ slots, const float* __restrict__ inv_freq,
                             const bf16* __restrict__ qn, const bf16* __restrict__ kn,
                             bf16* __restrict__ q_out, bf16* __restrict__ kv_layer,
                             int hq, int hkv, int page_size, float eps, int qkv_stride,
-                            float* __restrict__ kv_scale, const bf16* __restrict__ bias) {
+                            float* __restrict__ kv_scale, const bf16* __restrict__ bias, int n_tokens, int per_log) {
     constexpr int LPH = D / 16, HEADS = 256 / LPH;      // lanes of a head, heads at a time
-    __shared__ __align__(16) float s_cos[D / 2], s_sin[D / 2];
+    __shared__ __align__(16) float s_cos[ROPE_ANGLES], s_sin[ROPE_ANGLES];
     pdl_trigger();
-    const int t = blockIdx.x, g = threadIdx.x % LPH, heads = hq + 2 * hkv;
+    const int at_once = HEADS >> per_log, at = threadIdx.x / LPH, sub = (at << per_log) / HEADS, head0 = blockIdx.y * at_once;
+    const int t0 = blockIdx.x << per_log, t = min(t0 + sub, n_tokens - 1), g = threadIdx.x % LPH, heads = hq + 2 * hkv;
     pdl_wait();
     auto load8 = [](const bf16* p, float (&f)[8]) {
         if (VEC) {
@@ -177,13 +181,14 @@ qk_norm_rope_kvwrite_kernel(const bf16* __restrict__ qkv, const int* __restrict_
         load8(src, lo);
         load8(src + D / 2, hi);
     };
-    load(threadIdx.x / LPH);
-    if (threadIdx.x < D / 2) sincosf((float)positions[t] * inv_freq[threadIdx.x], &s_sin[threadIdx.x], &s_cos[threadIdx.x]);
+    load(head0 + (at & (at_once - 1)));
+    for (int i = threadIdx.x; i < (D / 2) << per_log; i += 256)
+        sincosf((float)positions[min(t0 + i / (D / 2), n_tokens - 1)] * inv_freq[i % (D / 2)], &s_sin[i], &s_cos[i]);
     const int slot = slots[t], page = slot / page_size, off = slot - page * page_size;
     __syncthreads();
-    for (int h0 = 0; h0 < heads; h0 += HEADS) {
-        const int h = h0 + threadIdx.x / LPH;
-        if (h0) load(h);
+    for (int h0 = head0; h0 < heads; h0 += at_once * gridDim.y) {
+        const int h = h0 + (at & (at_once - 1));
+        if (h0 != head0) load(h);
         if (bias) {     // projection bias (Qwen2): added here instead of by a pass of its own over the packed rows, rounded as that pass would
             float b[8];
             const bf16* bp = bias + (size_t)min(h, heads - 1) * D + g * 8;
@@ -229,7 +234,7 @@ qk_norm_rope_kvwrite_kernel(const bf16* __restrict__ qkv, const int* __restrict_
         if (is_q || is_k) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const float s = s_sin[g * 8 + e], c = s_cos[g * 8 + e], a = lo[e], b = hi[e];
+                const float s = s_sin[sub * (D / 2) + g * 8 + e], c = s_cos[sub * (D / 2) + g * 8 + e], a = lo[e], b = hi[e];
                 lo[e] = __fmaf_rn(a, c, -__fmul_rn(b, s));
                 hi[e] = __fmaf_rn(b, c, __fmul_rn(a, s));
             }
@@ -243,7 +248,7 @@ qk_norm_rope_kvwrite_kernel(const bf16* __restrict__ qkv, const int* __restrict_
             for (int o = LPH / 2; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
             scale = fmaxf(amax, 1e-12f) * (1.0f / 448.0f);
         }
-        if (h >= heads || (!is_q && slot < 0)) continue;
+        if (h >= heads || t0 + sub >= n_tokens || (!is_q && slot < 0)) continue;
         const int kvh = is_k ? h - hq : h - hq - hkv;
         const size_t row = (((size_t)page * 2 + (is_k ? 0 : 1)) * hkv + kvh) * page_size + off;
         if (KV8 && !is_q) {
@@ -493,7 +498,7 @@ PIE_API int pie_dequant_fp8_rowblock(const void* w8, const float* scale, void* o
     if (K % 16) return (int)cudaErrorInvalidValue;
     const int per_row = (K + DEQ_CHUNK - 1) / DEQ_CHUNK;
     const long chunks = rows * per_row;
-    const int blocks = (int)min((chunks + 7) / 8, (long)148 * 8);
+    const int blocks = (int)min((chunks + 7) / 8, (long)PIE_SMS * 8);
     dequant_fp8_rowblock_kernel<<<blocks, 256, 0, st>>>((const uint8_t*)w8, scale, (bf16*)out, K, chunks, per_row);
     return (int)cudaGetLastError();
 }
@@ -502,7 +507,7 @@ PIE_API int pie_swiglu(const void* gate_up, void* out, long rows, int inter, cud
     if (rows <= 0) return 0;
     if (inter % 8) return (int)cudaErrorInvalidValue;
     const long total = rows * (inter / 8);
-    const int blocks = (int)min((total + 255) / 256, (long)148 * 16);
+    const int blocks = (int)min((total + 255) / 256, (long)PIE_SMS * 16);
     swiglu_kernel<<<blocks, 256, 0, st>>>((const bf16*)gate_up, (bf16*)out, inter, total);
     return (int)cudaGetLastError();
 }
@@ -511,7 +516,7 @@ PIE_API int pie_glu_interleaved(const void* gate_up, void* out, long rows, int i
     if (rows <= 0) return 0;
     if (inter % 8 || act < 0 || act > 1) return (int)cudaErrorInvalidValue;
     const long total = rows * (inter / 8);
-    const int blocks = (int)min((total + 255) / 256, (long)148 * 16);
+    const int blocks = (int)min((total + 255) / 256, (long)PIE_SMS * 16);
     if (act == 0)
         glu_interleaved_kernel<0><<<blocks, 256, 0, st>>>((const bf16*)gate_up, (bf16*)out, total);
     else
@@ -555,12 +560,18 @@ PIE_API int pie_qk_bias_norm_rope_kvwrite(const void* qkv, const void* qkv_bias,
     if (n_tokens <= 0) return 0;
     const uintptr_t all = (uintptr_t)qkv | (uintptr_t)qkv_bias | (uintptr_t)q_norm_w | (uintptr_t)k_norm_w | (uintptr_t)q_out | (uintptr_t)kv_layer;
     const bool vec = qkv_stride % 8 == 0 && all % 16 == 0;
+    if (head_dim != 64 && head_dim != 128 && head_dim != 256) return (int)cudaErrorInvalidValue;
+    // Narrow rows (a tensor-parallel shard's) share a block between tokens; a few wide rows are spread over blocks.
+    const int heads = hq + 2 * hkv, at_once = 256 / (head_dim / 16);
+    int per_log = 0, split = 1;
+    while (heads << (per_log + 1) <= at_once && head_dim << per_log <= ROPE_ANGLES) ++per_log;
+    if (n_tokens <= PIE_SMS) split = (heads + at_once - 1) / at_once;
 #define LAUNCH(D, KV8)                                                                           \
     launch_pdl(vec ? qk_norm_rope_kvwrite_kernel<D, KV8, true> : qk_norm_rope_kvwrite_kernel<D, KV8, false>, \
-        dim3(n_tokens), dim3(256), 0, st,                                                       \
+        dim3((n_tokens + (1 << per_log) - 1) >> per_log, split), dim3(256), 0, st,              \
         (const bf16*)qkv, positions, slots, inv_freq, (const bf16*)q_norm_w,                    \
         (const bf16*)k_norm_w, (bf16*)q_out, (bf16*)kv_layer, hq, hkv, page_size, eps,          \
-        qkv_stride, kv_scale, (const bf16*)qkv_bias)
+        qkv_stride, kv_scale, (const bf16*)qkv_bias, n_tokens, per_log)
     if (kv_scale) {
         if (head_dim == 64) LAUNCH(64, true);
         else if (head_dim == 128) LAUNCH(128, true);

@@ -915,3 +915,26 @@ def test_sample_at_an_infinite_temperature():
         x = lg[0].float()
         higher = torch.stack([(allowed & (x > x[g])).sum() for g in got])
         assert bool(allowed[got].all()) and bool((higher < p * allowed.sum()).all()) and len(got.unique()) > 20
+
+
+@pytest.mark.parametrize("d,hq,hkv", [(64, 1, 1), (64, 3, 1), (64, 32, 8), (128, 1, 1), (128, 4, 1), (128, 6, 2), (128, 12, 2), (128, 64, 8),
+                                      (256, 2, 1), (256, 16, 2)])
+def test_rope_kvwrite_splits_of_blocks(d, hq, hkv):
+    """Several tokens per block, heads over several blocks and heads in turn: the reference's numbers, and those of every token alone."""
+    page = 16
+    freq = 500000.0 ** (-torch.arange(0, d, 2, device=DEV).float() / d)
+    for n in (1, 2, 7, 33, 148, 149, 300):
+        packed, qn, kn = bf(n, (hq + 2 * hkv) * d, seed=n), bf(d, seed=7) + 1, bf(d, seed=8) + 1
+        pos = torch.randint(0, 100000, (n,), device=DEV, generator=torch.Generator(device=DEV).manual_seed(n)).int()
+        slots = torch.randperm(n, device=DEV).int()
+        if n > 2:
+            slots[n // 2] = -1
+        pages = -(-max(n, 16) // page)
+        kv = [torch.zeros(pages, 2, hkv, page, d, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+        norm = lambda q, k, a: ops.qk_norm_rope_kvwrite(q[a], pos[a], slots[a], freq, qn, kn, k, hq, hkv, d, page, 1e-5)
+        got = norm(packed, kv[0], slice(None))
+        want = ref.qk_norm_rope_kvwrite(packed, pos, slots, freq, qn, kn, kv[1], hq, hkv, d, page, 1e-5)
+        close(got.view(n, -1), want.reshape(n, -1), 3e-2)
+        close(kv[0], kv[1], 3e-2)
+        one = torch.cat([norm(packed, kv[2], slice(t, t + 1)) for t in range(n)])
+        assert torch.equal(one, got) and torch.equal(kv[2], kv[0])
