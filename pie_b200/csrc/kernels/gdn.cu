@@ -83,6 +83,7 @@ __global__ void gdn_conv_state_kernel(const bf16* __restrict__ x, int x_stride, 
 constexpr int GDN_COEF = 40;               // numbers of a group of four tokens, see gdn_groups_kernel
 constexpr int GDN_STAGE = 16;              // tokens of a stage of gdn_walk
 constexpr int GDN_WARPS = 4;               // of gdn_walk
+constexpr int GDN_STEP_TOKENS = 4;         // of a request that gdn_step still takes
 
 // y = conv + SiLU over q | k | v; then q * rsqrt(q.q + 1e-6) * dk^-1/2 and k * rsqrt(k.k + 1e-6) per head. 128 channels (whole
 // heads) of 16 tokens per block: a channel's inputs are read once and slide through registers, and the heads' norms are taken
@@ -461,47 +462,49 @@ gdn_norm_kernel(const float* __restrict__ y, const bf16* __restrict__ x, int x_s
                 __float2bfloat16(v[i] * f * __bfloat162float(norm_w[lane + 32 * i]) * silu_f(zz[i]));
 }
 
-// Decode: a block per (request, value head) with 128 columns, an eighth of the rows per warp and four columns per lane: the
-// whole state is requested in 16-byte loads before anything waits for it. Both sums of a token run over the old state,
+// Decode: a block per (request, value head) with up to 4 LANES columns, four per lane, an eighth of the rows per group of LANES
+// threads: the whole state is requested in 16-byte loads before anything waits for it. Both sums of a token run over the old state,
 //   delta = beta (v - exp(g) S^T k),  o = exp(g) S^T q + (q . k) delta,  S <- exp(g) S + k delta^T.
 // Bound by memory (the state in and out). 40 requests x 32 heads of 128 x 128: 65.7 us token-serial with block-wide sums over
-// 64 rows per lane, 33 us like this (5.1 TB/s). Any number of tokens per request is right here; the walk is faster from three on.
-template <int DK>
-__global__ void __launch_bounds__(256)
+// 64 rows per lane, 33 us like this (5.1 TB/s). Any number of tokens per request is right here.
+template <int DK, int LANES>
+__global__ void __launch_bounds__(8 * LANES)
 gdn_step_kernel(const float* __restrict__ y, const bf16* __restrict__ x, int x_stride, const float* __restrict__ a_log,
                 const float* __restrict__ dt_bias, const bf16* __restrict__ norm_w, float* __restrict__ rec_state,
                 const int* __restrict__ qo_indptr, const int* __restrict__ slots, const int* __restrict__ reset,
-                bf16* __restrict__ out, int hk, int hv, float eps) {
-    constexpr int DV = 128, ROWS = DK / 8;
-    __shared__ __align__(16) float sq[DK], sk[DK], part_y[8][DV], part_z[8][DV];
+                bf16* __restrict__ out, int hk, int hv, int dv, float eps) {
+    constexpr int GROUPS = 8, ROWS = DK / GROUPS;
+    __shared__ __align__(16) float sq[DK], sk[DK], part_y[GROUPS][4 * LANES], part_z[GROUPS][4 * LANES];
     __shared__ float red[32];
-    const int r = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, rg = threadIdx.x >> 5, tid = threadIdx.x;
+    const int r = blockIdx.x, h = blockIdx.y, lane = threadIdx.x % LANES, rg = threadIdx.x / LANES, tid = threadIdx.x;
+    const bool own = lane * 4 < dv;        // columns past dv are zeros that nobody stores
     pdl_trigger();
     pdl_wait();
     const int first = qo_indptr[r], len = qo_indptr[r + 1] - first, slot = slots[r];
     if (len <= 0 || slot < 0) return;      // a padding request of a decode graph's bucket: no state, no output
-    const int kh = h / (hv / hk), c = 2 * hk * DK + hv * DV;
-    float* sp = rec_state + (((size_t)slot * hv + h) * DK + rg * ROWS) * DV + lane * 4;
+    const int kh = h / (hv / hk), c = 2 * hk * DK + hv * dv;
+    float* sp = rec_state + (((size_t)slot * hv + h) * DK + rg * ROWS) * dv + lane * 4;
     float4 S[ROWS];
-    if (reset[r]) {
+    if (reset[r] || !own) {
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) S[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
 #pragma unroll
-        for (int i = 0; i < ROWS; ++i) S[i] = *reinterpret_cast<const float4*>(sp + (size_t)i * DV);
+        for (int i = 0; i < ROWS; ++i) S[i] = *reinterpret_cast<const float4*>(sp + (size_t)i * dv);
     }
     const float decay_rate = -__expf(a_log[h]), bias = dt_bias[h];
     for (int t = first; t < first + len; ++t) {
         const float* row = y + (size_t)t * c;
         float qk = 0.f;
-        if (tid < DK) {
-            const float q = row[kh * DK + tid], k = row[hk * DK + kh * DK + tid];
-            sq[tid] = q;
-            sk[tid] = k;
-            qk = q * k;
+        for (int i = tid; i < DK; i += 8 * LANES) {
+            const float q = row[kh * DK + i], k = row[hk * DK + kh * DK + i];
+            sq[i] = q;
+            sk[i] = k;
+            qk += q * k;
         }
-        const float2 gates = gdn_gates(x + (size_t)t * x_stride + c + hv * DV, h, hv, decay_rate, bias);
-        const float4 v = *reinterpret_cast<const float4*>(row + 2 * hk * DK + h * DV + lane * 4);
+        const float2 gates = gdn_gates(x + (size_t)t * x_stride + c + hv * dv, h, hv, decay_rate, bias);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (own) v = *reinterpret_cast<const float4*>(row + 2 * hk * DK + h * dv + lane * 4);
         qk = block_sum(qk, red);
         float4 ys = make_float4(0.f, 0.f, 0.f, 0.f), zs = ys;
 #pragma unroll
@@ -515,7 +518,7 @@ gdn_step_kernel(const float* __restrict__ y, const bf16* __restrict__ x, int x_s
         __syncthreads();
         ys = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < GROUPS; ++j) {
             const float4 p = *reinterpret_cast<const float4*>(&part_y[j][lane * 4]);
             ys.x += p.x; ys.y += p.y; ys.z += p.z; ys.w += p.w;
         }
@@ -527,25 +530,40 @@ gdn_step_kernel(const float* __restrict__ y, const bf16* __restrict__ x, int x_s
             S[i].x = gates.y * S[i].x + k * d.x; S[i].y = gates.y * S[i].y + k * d.y;
             S[i].z = gates.y * S[i].z + k * d.z; S[i].w = gates.y * S[i].w + k * d.w;
         }
-        if (rg == 0) {                     // this warp has all columns: output, its norm and gate
+        constexpr int OUT = LANES < 32 ? 32 : LANES;       // threads that have all columns: output, its norm and gate
+        float o[4], ms = 0.f;
+        if (tid < OUT) {
             zs = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < GROUPS; ++j) {
                 const float4 p = *reinterpret_cast<const float4*>(&part_z[j][lane * 4]);
                 zs.x += p.x; zs.y += p.y; zs.z += p.z; zs.w += p.w;
             }
-            const float o[4] = {gates.y * zs.x + qk * d.x, gates.y * zs.y + qk * d.y, gates.y * zs.z + qk * d.z, gates.y * zs.w + qk * d.w};
-            const float f = rsqrtf(warp_sum(o[0] * o[0] + o[1] * o[1] + o[2] * o[2] + o[3] * o[3]) / (float)DV + eps);
-            const bf16* z = x + (size_t)t * x_stride + c + h * DV + lane * 4;
-            bf16* dst = out + ((size_t)t * hv + h) * DV + lane * 4;
+            o[0] = gates.y * zs.x + qk * d.x; o[1] = gates.y * zs.y + qk * d.y;
+            o[2] = gates.y * zs.z + qk * d.z; o[3] = gates.y * zs.w + qk * d.w;
+            ms = o[0] * o[0] + o[1] * o[1] + o[2] * o[2] + o[3] * o[3];
+#pragma unroll
+            for (int s = (LANES < 32 ? LANES : 32) / 2; s; s >>= 1) ms += __shfl_xor_sync(0xffffffffu, ms, s);
+        }
+        if constexpr (LANES > 32) {
+            __syncthreads();               // `red` has been read
+            if (lane % 32 == 0 && tid < OUT) red[tid / 32] = ms;
+            __syncthreads();
+            ms = red[0] + red[1];
+        }
+        if (tid < OUT) {
+            const float f = rsqrtf(ms / (float)dv + eps);
+            const bf16* z = x + (size_t)t * x_stride + c + h * dv + lane * 4;
+            bf16* dst = out + ((size_t)t * hv + h) * dv + lane * 4;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                dst[i] = __float2bfloat16(o[i] * f * __bfloat162float(norm_w[lane * 4 + i]) * silu_f(__bfloat162float(z[i])));
+                if (own && tid < LANES) dst[i] = __float2bfloat16(o[i] * f * __bfloat162float(norm_w[lane * 4 + i]) * silu_f(__bfloat162float(z[i])));
         }
         __syncthreads();                   // the partial sums and q, k are rewritten by the next token
     }
 #pragma unroll
-    for (int i = 0; i < ROWS; ++i) *reinterpret_cast<float4*>(sp + (size_t)i * DV) = S[i];
+    for (int i = 0; i < ROWS; ++i)
+        if (own) *reinterpret_cast<float4*>(sp + (size_t)i * dv) = S[i];
 }
 
 // Mamba-2 state update: grid (requests, heads), block = head_dim threads; thread p holds S[p, :] (NS values)
@@ -610,24 +628,27 @@ __global__ void gdn_copy_slot_kernel(float* __restrict__ buf, size_t layer_strid
 
 }  // namespace pie
 
-// The block-per-head step takes fires of at most two tokens per request on average; more are walked through in fours.
-static bool gdn_steps(int n, int r, int dv) { return dv == 128 && n <= 2 * r; }
+// The block-per-head step takes fires of short requests (`longest`: most tokens of one), others are walked through in fours: the
+// step's chain grows with every token, the walk's with every four. Measured, step against walk: 64 requests of 32 heads of
+// 128 x 128 with 3 tokens 108 / 126 us, 4 tokens 125 / 128, 6 tokens 168 / 159; one request with 4 tokens 16.0 / 15.9, 6 tokens 19.6 / 16.9. Of
+// 64 x 64 heads, 64 requests with one token: 14 / 30 us.
+static bool gdn_steps(int longest) { return longest <= pie::GDN_STEP_TOKENS; }
 
 // 32-bit numbers of workspace (`coef`) that a fire needs.
-PIE_API long pie_gdn_coef_elems(int n, int r, int hv, int dv) {
-    return gdn_steps(n, r, dv) ? 0 : ((long)n / 4 + r + 1) * hv * pie::GDN_COEF;
+PIE_API long pie_gdn_coef_elems(int n, int r, int longest, int hv) {
+    return gdn_steps(longest) ? 0 : ((long)n / 4 + r + 1) * hv * pie::GDN_COEF;
 }
 
 template <int DK>
 static int launch_gdn(const void* x, int x_stride, const void* conv_w, const float* a_log, const float* dt_bias, const void* norm_w,
                       float* conv_state, float* rec_state, const int* qo_indptr, const int* tok_req, const int* slots,
-                      const int* reset, float* y, float* coef, void* out, int n, int r, int hk, int hv, int dv, float eps,
+                      const int* reset, float* y, float* coef, void* out, int n, int r, int longest, int hk, int hv, int dv, float eps,
                       cudaStream_t st) {
     using namespace pie;
     const int qk = 2 * hk * DK, c = qk + hv * dv;
     const bf16* xb = static_cast<const bf16*>(x);
     const bf16* nw = static_cast<const bf16*>(norm_w);
-    const int tile = (long)n * ((c + 127) / 128) <= 16 * 148 * 4 ? 4 : 16;
+    const int tile = (long)n * ((c + 127) / 128) <= 16L * PIE_SMS * 4 ? 4 : 16;
     cudaError_t e = launch_pdl(tile == 4 ? gdn_prep_kernel<DK, 4> : gdn_prep_kernel<DK, 16>, dim3((c + 127) / 128, (n + tile - 1) / tile),
                                dim3(128), 0, st, xb, x_stride, static_cast<const bf16*>(conv_w), conv_state, qo_indptr, tok_req, slots,
                                reset, y, n, c, qk);
@@ -635,9 +656,12 @@ static int launch_gdn(const void* x, int x_stride, const void* conv_w, const flo
         e = launch_pdl(gdn_conv_state_kernel<4>, dim3((c + 127) / 128, r), dim3(128), 0, st, xb, x_stride, conv_state, qo_indptr, slots,
                        reset, c);
     if (e != cudaSuccess) return (int)e;
-    if (gdn_steps(n, r, dv)) {
-        e = launch_pdl(gdn_step_kernel<DK>, dim3(r, hv), dim3(256), 0, st, y, xb, x_stride, a_log, dt_bias, nw, rec_state, qo_indptr,
-                       slots, reset, static_cast<bf16*>(out), hk, hv, eps);
+    if (gdn_steps(longest)) {
+        auto kern = dv <= 32 ? gdn_step_kernel<DK, 8> : dv <= 64 ? gdn_step_kernel<DK, 16> : gdn_step_kernel<DK, 32>;
+        if constexpr (DK < 128)
+            if (dv > 128) kern = gdn_step_kernel<DK, 64>;
+        e = launch_pdl(kern, dim3(r, hv), dim3(dv <= 32 ? 64 : dv <= 64 ? 128 : dv <= 128 ? 256 : 512), 0, st, y, xb, x_stride, a_log, dt_bias, nw, rec_state,
+                       qo_indptr, slots, reset, static_cast<bf16*>(out), hk, hv, dv, eps);
         return (int)(e != cudaSuccess ? e : cudaGetLastError());
     }
     if (!coef) return (int)cudaErrorInvalidValue;
@@ -654,7 +678,7 @@ static int launch_gdn(const void* x, int x_stride, const void* conv_w, const flo
     // Four columns per lane read shared memory half as often as two, but leave half the warps: they win where there are plenty
     // (26 prompts of 100 tokens: 406 against 482 us for the mixer) and lose where a few long prompts run (1300 + 700 + 500 tokens:
     // 679 against 581 us).
-    const bool wide = DK == 128 && dv % 64 == 0 && (long)r * hv * (dv / 64) >= 4 * 148;
+    const bool wide = DK == 128 && dv % 64 == 0 && (long)r * hv * (dv / 64) >= 4 * PIE_SMS;
     if (wide) walk(std::integral_constant<int, 8>{}, std::integral_constant<int, DK == 128 ? 4 : 2>{});
     else walk(std::integral_constant<int, 8>{}, std::integral_constant<int, 2>{});
     if (e == cudaSuccess)
@@ -666,7 +690,7 @@ static int launch_gdn(const void* x, int x_stride, const void* conv_w, const flo
 PIE_API int pie_gdn_mixer(const void* x, int x_stride, const void* conv_w, const float* a_log, const float* dt_bias,
                           const void* norm_w, float* conv_state, float* rec_state, const int* qo_indptr,
                           const int* tok_req, const int* slots, const int* reset, float* conv_scratch, float* coef,
-                          void* out, int n, int r, int hk, int hv, int dk, int dv, int kernel, float eps, cudaStream_t st) {
+                          void* out, int n, int r, int longest, int hk, int hv, int dk, int dv, int kernel, float eps, cudaStream_t st) {
     using namespace pie;
     if (n <= 0 || r <= 0) return 0;
     if (kernel != 4) return (int)cudaErrorInvalidValue;
@@ -674,7 +698,7 @@ PIE_API int pie_gdn_mixer(const void* x, int x_stride, const void* conv_w, const
     auto launch = dk == 32 ? launch_gdn<32> : dk == 64 ? launch_gdn<64> : dk == 128 ? launch_gdn<128> : nullptr;
     if (!launch) return (int)cudaErrorInvalidValue;
     return launch(x, x_stride, conv_w, a_log, dt_bias, norm_w, conv_state, rec_state, qo_indptr, tok_req, slots, reset, conv_scratch, coef,
-                  out, n, r, hk, hv, dv, eps, st);
+                  out, n, r, longest, hk, hv, dv, eps, st);
 }
 
 PIE_API int pie_mamba2_mixer(const void* x, int x_stride, const void* conv_w, const void* conv_b, const float* a_log,

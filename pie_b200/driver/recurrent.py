@@ -65,6 +65,11 @@ class RecurrentInputs:
         return self.linear_state[:, self.token_at].view(torch.int32)
 
     @cached_property
+    def longest(self) -> int:
+        """Tokens of the request that brings most of them."""
+        return int(max((b - a for a, b in zip(self.qo_host, self.qo_host[1:])), default=0))
+
+    @cached_property
     def has_portions(self) -> bool:
         """Whether some request of the fire brings more than one token."""
         return any(b - a > 1 for a, b in zip(self.qo_host, self.qo_host[1:]))

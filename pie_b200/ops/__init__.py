@@ -1076,11 +1076,11 @@ def gdn_mixer(mix, lw: dict, cfg, rs, layer: int):
                                    rs.slots_host, rs.reset_host)
     n, r = mix.shape[0], len(rs.slots_host)
     out = torch.empty(n, hv * dv, dtype=torch.bfloat16, device=mix.device)
-    elems = fn("pie_gdn_coef_elems")(n, r, hv, dv)
+    elems = fn("pie_gdn_coef_elems")(n, r, rs.longest, hv)
     coef = torch.empty(elems, dtype=torch.float32, device=mix.device) if elems else None
     check(fn("pie_gdn_mixer")(ptr(mix), mix.stride(0), ptr(lw["gdn_conv"]), ptr(lw["gdn_A_log"]), ptr(lw["gdn_dt_bias"]),
                               ptr(lw["gdn_norm"]), ptr(conv_state), ptr(rec_state), ptr(rs.qo_indptr), ptr(rs.tok_req),
-                              ptr(rs.slots), ptr(rs.reset), ptr(rs.scratch), ptr(coef), ptr(out), n, r, hk, hv, dk, dv,
+                              ptr(rs.slots), ptr(rs.reset), ptr(rs.scratch), ptr(coef), ptr(out), n, r, rs.longest, hk, hv, dk, dv,
                               cfg.linear_conv_kernel_dim, cfg.rms_norm_eps, stream_ptr()), "gdn_mixer")
     return out
 

@@ -59,7 +59,7 @@ _SIGNATURES = {
     "pie_feed_tokens": [p, p, p, i32, p],
     "pie_validate_indices": [p, i32, i32, i32, i32, p, p],
     "pie_gdn_coef_elems": [i32, i32, i32, i32],
-    "pie_gdn_mixer": [p, i32, p, p, p, p, p, p, p, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, i32, f32, p],
+    "pie_gdn_mixer": [p, i32, p, p, p, p, p, p, p, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, i32, i32, f32, p],
     "pie_gdn_copy_slot": [p, i64, i64, i32, i32, i32, p],
     "pie_mamba2_mixer": [p, i32, p, p, p, p, p, p, p, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, p],
     "pie_stream_embed": [p, p, p, i32, i32, i32, i32, f32, i32, p],

@@ -785,7 +785,7 @@ def test_sample_over_cluster_sizes(vocab):
 
 @pytest.mark.parametrize("dk,dv,hk,hv,lens", [
     (128, 128, 2, 4, [1, 2, 3, 4, 5, 15, 16, 17, 33]),       # walk: groups of four, stages of sixteen
-    (128, 128, 2, 4, [1, 2, 1, 3, 1, 0]),                    # step: up to two tokens per request on average
+    (128, 128, 2, 4, [1, 2, 1, 3, 1, 0]),                    # step: up to four tokens per request
     (128, 128, 1, 32, [7] * 10),                             # walk with four columns per lane
     (128, 32, 1, 3, [1, 1]), (64, 96, 3, 3, [1, 6, 1]), (32, 256, 1, 2, [19]), (64, 128, 2, 2, [1, 1, 2])])
 def test_gdn_mixer_routes_match_reference(dk, dv, hk, hv, lens):
@@ -915,6 +915,14 @@ def test_sample_at_an_infinite_temperature():
         x = lg[0].float()
         higher = torch.stack([(allowed & (x > x[g])).sum() for g in got])
         assert bool(allowed[got].all()) and bool((higher < p * allowed.sum()).all()) and len(got.unique()) > 20
+
+
+@pytest.mark.parametrize("dk,dv,hk,hv", [(32, 32, 2, 2), (32, 64, 1, 2), (64, 64, 2, 4), (64, 96, 1, 3), (128, 64, 2, 2), (128, 96, 1, 2),
+                                         (32, 160, 1, 2), (64, 256, 2, 2)])
+def test_gdn_short_requests_of_all_head_sizes(dk, dv, hk, hv):
+    """The step up to its last token and the walk from there on: columns that fill a group of lanes and columns that do not."""
+    for lens in ([1, 2, 1, 3, 1, 0, 1], [4, 1, 4], [5, 1, 0]):
+        test_gdn_mixer_routes_match_reference(dk, dv, hk, hv, lens)
 
 
 @pytest.mark.parametrize("d,hq,hkv", [(64, 1, 1), (64, 3, 1), (64, 32, 8), (128, 1, 1), (128, 4, 1), (128, 6, 2), (128, 12, 2), (128, 64, 8),
