@@ -21,8 +21,7 @@ namespace pie {
 
 constexpr int SAMPLE_THREADS = 512;
 constexpr int SAMPLE_WARPS = SAMPLE_THREADS / 32;
-constexpr int SAMPLE_CLUSTER = 8;                  // most CTAs of a row; 1, 2, 4 or 8 of them
-constexpr int SAMPLE_PARTS = SAMPLE_CLUSTER;       // of a row, see SampleRow
+constexpr int SAMPLE_CLUSTER = 8;                  // most CTAs of a row
 constexpr int SAMPLE_BINS = SAMPLE_THREADS;        // one per thread
 constexpr uint32_t NEG_INF2 = 0xFF80FF80u;         // two bf16 of -inf
 constexpr float LOG2E = 1.4426950408889634f;
@@ -51,11 +50,6 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 __device__ __forceinline__ void st_cluster_u64(uint32_t addr, unsigned long long v) {
     asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
 }
-__device__ __forceinline__ unsigned long long ld_cluster_u64(uint32_t addr) {
-    unsigned long long v;
-    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
-    return v;
-}
 __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
     uint32_t v;
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -67,12 +61,21 @@ struct SampleShift {
     uint32_t by9, by13, by16;
 };
 
+// Masses as whole numbers of 2^-40, NaN as bit 63.
+constexpr unsigned long long NAN_UNITS = 1ull << 63;
+__device__ __forceinline__ unsigned long long add_units(unsigned long long a, unsigned long long b) {
+    return ((a & ~NAN_UNITS) + (b & ~NAN_UNITS)) | ((a | b) & NAN_UNITS);
+}
+__device__ __forceinline__ unsigned long long warp_add_u64(unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v = add_units(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
 struct SampleShared {
     unsigned long long red[SAMPLE_WARPS];
-    unsigned long long slot[2][SAMPLE_PARTS];      // one word of each CTA or part of the row, two exchanges deep
-    unsigned long long mass[SAMPLE_BINS];          // in units of 2^-42
-    float2 part[SAMPLE_PARTS][SAMPLE_WARPS];       // sums of this CTA's parts, by warp
-    uint32_t cnt[SAMPLE_BINS];
+    unsigned long long slot[2][SAMPLE_CLUSTER];    // one word of each CTA of the row, two exchanges deep
+    uint32_t cnt[SAMPLE_BINS], mass[3][SAMPLE_BINS];       // masses: whole numbers in three words
     uint32_t wcnt[SAMPLE_WARPS];
     float wmass[SAMPLE_WARPS];
     uint32_t best[4];                              // best score key of a Gumbel pass so far
@@ -83,9 +86,7 @@ struct SampleShared {
 
 // One row, or a CTA's share of it: vectors of 8 bf16 at (i * cluster + rank) * SAMPLE_THREADS + thread. RESIDENT: they are
 // kept in shared memory from the first pass on, each read by the thread that wrote it; else they are read again (L2) in every
-// pass. For sums a row has SAMPLE_PARTS parts, blocks of SAMPLE_THREADS vectors dealt out in turn, whatever the cluster has of
-// CTAs: CTA `rank` holds the parts rank + cl j. A part's entries meet in one order and so do the parts, so that no sum depends
-// on how many CTAs the other rows of a batch leave to a row. Entries that the mask or the row's end excludes are -inf here, and `allowed` tells them from an -inf of the row where
+// pass. Entries that the mask or the row's end excludes are -inf here, and `allowed` tells them from an -inf of the row where
 // it matters.
 template <bool RESIDENT>
 struct SampleRow {
@@ -135,18 +136,7 @@ struct SampleRow {
                 }
         }
     }
-    // f(first index, vector), the CTA's parts one after the other, end(j) behind each; every thread of a warp makes the same
-    // number of calls
-    template <typename F, typename G>
-    __device__ __forceinline__ void scan(F&& f, G&& end) const {
-        const int parts = SAMPLE_PARTS / cl;
-#pragma unroll 1
-        for (int j = 0; j < parts; ++j) {
-#pragma unroll 1
-            for (int i = j; i < count; i += parts) f(index(i) * 8, RESIDENT ? kept[i * SAMPLE_THREADS + threadIdx.x] : load(index(i)));
-            end(j);
-        }
-    }
+    // f(first index, vector); every thread of a warp makes the same number of calls
     template <typename F>
     __device__ __forceinline__ void scan(F&& f) const {
 #pragma unroll 1
@@ -196,17 +186,14 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
     int turn = 0;
     bool started = cl == 1;
     const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(&sh.slot[0][0]);
-    auto post = [&](int at, unsigned long long v) {  // by a warp: a word into slot `at` of every CTA
+    auto exchange = [&](unsigned long long v) {      // v: this CTA's word, the same in all of its threads
         if (cl == 1) {
-            if (lane == 0) sh.slot[turn][at] = v;
-        } else if (lane < cl) {
-            st_cluster_u64(sm100::map_to_cta(slot0 + (turn * SAMPLE_PARTS + at) * 8, lane), v);
-        }
-    };
-    auto meet = [&]() {                              // the words posted before it are there
-        if (cl == 1) {
+            if (tid == 0) sh.slot[turn][0] = v;
             __syncthreads();
         } else {
+            if (!started) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");   // every CTA has started
+            started = true;
+            if (tid < cl) st_cluster_u64(sm100::map_to_cta(slot0 + (turn * SAMPLE_CLUSTER + rv.rank) * 8, tid), v);
             __syncwarp();
             sm100::cluster_sync_all();
         }
@@ -215,29 +202,34 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
         v = warp_max_u64(v);
         if (lane == 0) sh.red[wid] = v;
         __syncthreads();
-        if (!started) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");       // every CTA has started
-        started = true;
-        if (wid == 0) post(rv.rank, warp_max_u64(lane < SAMPLE_WARPS ? sh.red[lane] : 0ull));
-        meet();
+        exchange(warp_max_u64(lane < SAMPLE_WARPS ? sh.red[lane] : 0ull));
         v = warp_max_u64(lane < cl ? sh.slot[turn][lane] : 0ull);
         turn ^= 1;
         return v;
     };
-    auto row_sums = [&]() {                          // of `part`, over the row; not the first exchange
+    auto row_sum2 = [&](float& a, float& b) {
+        a = warp_sum(a);
+        b = warp_sum(b);
+        if (lane == 0) sh.red[wid] = ((unsigned long long)__float_as_uint(b) << 32) | __float_as_uint(a);
         __syncthreads();
-        if (wid < SAMPLE_PARTS / cl) {
-            const float2 t = lane < SAMPLE_WARPS ? sh.part[wid][lane] : make_float2(0.f, 0.f);
-            const float a = warp_sum(t.x), b = warp_sum(t.y);
-            post(rv.rank + cl * wid, ((unsigned long long)__float_as_uint(b) << 32) | __float_as_uint(a));
-        }
-        meet();
-        float2 sum = make_float2(0.f, 0.f);
-        for (int j = 0; j < SAMPLE_PARTS; ++j) {
-            sum.x += __uint_as_float((uint32_t)sh.slot[turn][j]);
-            sum.y += __uint_as_float((uint32_t)(sh.slot[turn][j] >> 32));
+        const unsigned long long t = lane < SAMPLE_WARPS ? sh.red[lane] : 0ull;
+        const float ta = warp_sum(__uint_as_float((uint32_t)t)), tb = warp_sum(__uint_as_float((uint32_t)(t >> 32)));
+        exchange(((unsigned long long)__float_as_uint(tb) << 32) | __float_as_uint(ta));
+        a = b = 0.f;
+        for (int j = 0; j < cl; ++j) {
+            a += __uint_as_float((uint32_t)sh.slot[turn][j]);
+            b += __uint_as_float((uint32_t)(sh.slot[turn][j] >> 32));
         }
         turn ^= 1;
-        return sum;
+    };
+    auto row_sum_units = [&](unsigned long long v) {
+        v = warp_add_u64(v);
+        if (lane == 0) sh.red[wid] = v;
+        __syncthreads();
+        exchange(warp_add_u64(lane < SAMPLE_WARPS ? sh.red[lane] : 0ull));
+        v = warp_add_u64(lane < cl ? sh.slot[turn][lane] : 0ull);
+        turn ^= 1;
+        return v & NAN_UNITS ? __uint_as_float(0x7fffffffu) : __ull2float_rn(v) * 0x1p-40f;
     };
 
     // ---- arg-max over the allowed entries, the lowest index of equals
@@ -302,7 +294,7 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
     };
 
     // Gumbel-max over the entries with key >= lo (and the min-p floor, and the mask); `salt` separates the noise streams of
-    // different rounds. Returns (score key << 32 | ~index) or 0. With `sum`, the weights of all entries are added up in `part`, too.
+    // different rounds. Returns (score key << 32 | ~index) or 0. With Z, adds up the weights of all entries too.
     //
     // The score of an entry of weight w (exp of its scaled distance from the largest) and uniform u is log w - log(-log u). As
     // -log u >= 1 - u, it cannot reach a score b seen before where 1 - u > w exp(-b): that test costs one exponential that the
@@ -312,7 +304,7 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
     // near 1 (2^-22) and the bits of u beyond 23; 1e-4 of B for the weights' relative error.
     // Shifts are products' high halves: shifts, logic and comparisons share one pipe of half rate, and it is what the pass is
     // bound by (62 million instructions for 300 rows of 128256, that pipe 65 % busy, before the test was thinned out).
-    auto gumbel_pass = [&](uint32_t lo, uint32_t salt, bool sum) -> unsigned long long {
+    auto gumbel_pass = [&](uint32_t lo, uint32_t salt, float* Z) -> unsigned long long {
         if (lo > kmax) return 0ull;
         const uint32_t from = s0 + salt * 0x632BE5ABu;
         unsigned long long pick = 0ull;
@@ -332,7 +324,7 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
         volatile uint32_t* shared_best = &sh.best[salt & 3];
         const float xlow = fmaxf(sortable_value((int)lo - 0x8000), x_floor);    // necessary for key >= lo, not sufficient
         float z = 0.f;
-        const bool all = sum || xlow == -INFINITY;
+        const bool all = Z || xlow == -INFINITY;
         rv.scan([&](int idx0, const uint4& p) {
             if (!all && !__any_sync(0xffffffffu, !(sortable_value(rv.top(p)) < xlow))) return;
             const uint32_t others = *shared_best;    // one score found anywhere in the CTA spares the other warps theirs
@@ -354,7 +346,7 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
             for (int k = 0; k < 8; ++k) {
                 const float w = weight(bf16_at(p, k));
                 maybe |= passes(k, w);
-                if (sum) z += w;
+                if (Z) z += w;
             }
             if (__any_sync(0xffffffffu, maybe)) {
                 if (maybe) {
@@ -370,15 +362,28 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
                     if (lane == 0) atomicMax(&sh.best[salt & 3], seen);
                 }
             }
-        }, [&](int j) {
-            if (!sum) return;
-            z = warp_sum(z);
-            if (lane == 0) sh.part[j][wid].x = z;
-            z = 0.f;
         });
+        if (Z) *Z = z;
         return row_max(pick);
     };
 
+    // Mass of the entries with key >= lo, to the last bit whatever the order of the entries: in whole numbers of 2^-40 for eight
+    // entries at a time.
+    auto exact_mass = [&](uint32_t lo) {
+        unsigned long long units = 0;
+        bool nan = false;
+        rv.scan([&](int, const uint4& p) {
+            float w = 0.f;
+#pragma unroll 1
+            for (int k = 0; k < 8; ++k) w += bf16_key(bits_at(p, k)) >= lo ? weight(bf16_at(p, k)) : 0.f;
+            units += __float2ull_rn(w * 0x1p40f);
+            nan |= w != w;
+        });
+        return row_sum_units(nan ? NAN_UNITS : units);
+    };
+    // What the order of the additions can change in a 32-bit sum of a row's weights, twice, relative to the sum. It follows the number of
+    // CTAs, and so the rows of a batch: a decision that such sums leave open is made on exact masses.
+    const float order_error = (float)(rv.count * 8 + 64) * 0x1p-22f;
     if (need_k || need_p) {
         // Rejection rounds (no histogram, no atomics): draw a candidate from the distribution restricted to keys >= lo, then
         // measure how much probability mass lies strictly above its key. It belongs to the kept set iff that is below
@@ -388,16 +393,16 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
         // search takes over.
         uint32_t lo = 0;
         const int rounds = (need_p && !need_k && P >= 0.5f) ? 3 : 0;
-        float Z = 0.f;
+        float z_thread = 0.f;
         for (int round = 0; round < rounds; ++round) {
-            const unsigned long long pick = gumbel_pass(lo, (uint32_t)round, round == 0);
+            const unsigned long long pick = gumbel_pass(lo, (uint32_t)round, round == 0 ? &z_thread : nullptr);
             if (pick == 0ull) {                       // nothing left above lo: fall back to the arg-max
                 if (writer) out_tokens[row] = arg;
                 return;
             }
             const int cand = (int)(0xffffffffu - (uint32_t)(pick & 0xffffffffu));
             const uint32_t ckey = bf16_key(reinterpret_cast<const uint16_t*>(rv.vec)[cand]);
-            float above = 0.f;
+            float z = z_thread, above = 0.f;
             rv.scan([&](int, const uint4& p) {
                 if (rv.top(p) <= (int)ckey - 0x8000) return;
 #pragma unroll
@@ -405,14 +410,13 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
                     const uint32_t sv = sortable2(word_at(p, k >> 1)) << ((k & 1) ? 0 : 16);
                     if ((int)sv > (((int)ckey - 0x8000) * 0x10000 | 0xFFFF)) above += weight(bf16_at(p, k));
                 }
-            }, [&](int j) {
-                above = warp_sum(above);
-                if (lane == 0) sh.part[j][wid].y = above;
-                above = 0.f;
             });
-            const float2 sum = row_sums();
-            Z = sum.x;
-            if (sum.y < P * Z) {
+            row_sum2(z, above);
+            if (fabsf(above - P * z) <= z * order_error) {
+                above = exact_mass(ckey + 1u);
+                z = exact_mass(0u);
+            }
+            if (above < P * z) {
                 if (writer) out_tokens[row] = cand;
                 return;
             }
@@ -422,30 +426,22 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
         // largest entry's first (entries that can matter are almost always among them), else 128 at a time over all keys and
         // then one by one. A key's mass is its entries' number times their weight; that of 128 keys is added up in whole numbers: neither
         // depends on the order in which the entries come.
-        if (need_p && rounds == 0) {
-            float z = 0.f;
-            rv.scan([&](int, const uint4& p) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) z += weight(bf16_at(p, k));
-            }, [&](int j) {
-                z = warp_sum(z);
-                if (lane == 0) sh.part[j][wid] = make_float2(z, 0.f);
-                z = 0.f;
-            });
-            Z = row_sums().x;
-        }
+        const float Z = need_p ? exact_mass(0u) : 0.f;
         if (need_p && 0.f >= P * Z) {                 // top-p of nothing: the arg-max, also where others equal it
             if (writer) out_tokens[row] = arg;
             return;
         }
-        const uint32_t cnt0 = (uint32_t)__cvta_generic_to_shared(&sh.cnt[0]), mass0 = (uint32_t)__cvta_generic_to_shared(&sh.mass[0]);
+        const uint32_t cnt0 = (uint32_t)__cvta_generic_to_shared(&sh.cnt[0]), mass0 = (uint32_t)__cvta_generic_to_shared(&sh.mass[0][0]);
+        // a mass of 1 in units, and bits of a word: as many as the entries of a CTA cannot overflow (14 for up to 2^18 of them)
+        const int bits = min(14, __clz(rv.count * SAMPLE_THREADS * 8 - 1));
+        const float one = (float)(1ull << (3 * bits - 1));
         uint32_t base_cnt = 0;
         float base_mass = 0.f;
         // first bin of `bins` bins of 2^shift keys, downwards from `ktop`, at which a limit is reached, or -1
         auto search = [&](uint32_t ktop, int shift, int bins) -> int {
             __syncthreads();
             sh.cnt[tid] = 0;
-            sh.mass[tid] = 0ull;
+            sh.mass[0][tid] = sh.mass[1][tid] = sh.mass[2][tid] = 0;
             if (tid == 0) sh.hit = SAMPLE_BINS;
             __syncthreads();
             const int low = (int)ktop - (bins << shift) + 1 - 0x8000;
@@ -457,24 +453,31 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
                     const uint32_t bin = (ktop - key) >> shift;       // huge for keys above ktop
                     if (bin >= (uint32_t)bins) continue;
                     atomicAdd(&sh.cnt[bin], 1u);
-                    if (need_p && shift) atomicAdd(&sh.mass[bin], __float2ull_rn(weight(bf16_at(p, k)) * 4398046511104.f));
+                    if (need_p && shift) {
+                        const unsigned long long units = __float2ull_rn(weight(bf16_at(p, k)) * one);
+                        atomicAdd(&sh.mass[0][bin], (uint32_t)units & ((1u << bits) - 1u));
+                        atomicAdd(&sh.mass[1][bin], (uint32_t)(units >> bits) & ((1u << bits) - 1u));
+                        atomicAdd(&sh.mass[2][bin], (uint32_t)(units >> (2 * bits)));
+                    }
                 }
             });
             __syncthreads();
             uint32_t c = 0;
             unsigned long long units = 0;
+            auto word = [&](int w, uint32_t v) { units += (unsigned long long)v << (w * bits); };
             if (cl > 1) {
                 sm100::cluster_sync_all();
                 for (int j = 0; j < cl; ++j) {
                     c += ld_cluster_u32(sm100::map_to_cta(cnt0 + tid * 4, j));
-                    if (need_p && shift) units += ld_cluster_u64(sm100::map_to_cta(mass0 + tid * 8, j));
+                    if (need_p && shift)
+                        for (int w = 0; w < 3; ++w) word(w, ld_cluster_u32(sm100::map_to_cta(mass0 + (w * SAMPLE_BINS + tid) * 4, j)));
                 }
                 sm100::cluster_sync_all();                            // read by all before it changes or its CTA ends
             } else {
                 c = sh.cnt[tid];
-                units = sh.mass[tid];
+                for (int w = 0; w < 3; ++w) word(w, sh.mass[w][tid]);
             }
-            float m = __ull2float_rn(units) * 0x1p-42f;
+            float m = __ull2float_rn(units) / one;
             if (need_p && !shift && c) m = (float)c * weight(sortable_value((int)ktop - tid - 0x8000));
             const uint32_t c_own = c;
             const float m_own = m;
@@ -513,7 +516,7 @@ sample_kernel(const bf16* __restrict__ logits, long row_stride, int vocab,
         }
     }
     // ---- Gumbel-max over the kept set
-    const unsigned long long pick = gumbel_pass(thr_key, 7u, false);
+    const unsigned long long pick = gumbel_pass(thr_key, 7u, nullptr);
     if (writer) out_tokens[row] = pick ? (int)(0xffffffffu - (uint32_t)(pick & 0xffffffffu)) : arg;
 }
 
@@ -574,9 +577,8 @@ PIE_API int pie_sample(const void* logits, long row_stride, int rows, int vocab,
     // CTAs of a row: as few as hold it in 64 KB each (three per SM), for a row's reductions cost every CTA the same, but up to 8
     // while the machine has room, for latency. Rows beyond 8 x 192 KB are read again in every pass.
     const int nvec = vocab / 8, each = SAMPLE_THREADS * 16;
-    int cl = 1;
-    while (cl < SAMPLE_CLUSTER && nvec > cl * 4096) cl *= 2;
-    while (cl < SAMPLE_CLUSTER && nvec > cl * SAMPLE_THREADS && (long)rows * 2 * cl <= 2 * 148) cl *= 2;
+    int cl = std::min(SAMPLE_CLUSTER, (nvec + 4095) / 4096);
+    while (cl < SAMPLE_CLUSTER && nvec > cl * SAMPLE_THREADS && (long)rows * (cl + 1) <= 2 * PIE_SMS) ++cl;
     const int count = (nvec + cl * SAMPLE_THREADS - 1) / (cl * SAMPLE_THREADS);
     const bool resident = count * each <= 192 * 1024;
     auto kern = resident ? sample_kernel<true> : sample_kernel<false>;
