@@ -660,8 +660,9 @@ static int launch_gdn(const void* x, int x_stride, const void* conv_w, const flo
         auto kern = dv <= 32 ? gdn_step_kernel<DK, 8> : dv <= 64 ? gdn_step_kernel<DK, 16> : gdn_step_kernel<DK, 32>;
         if constexpr (DK < 128)
             if (dv > 128) kern = gdn_step_kernel<DK, 64>;
-        e = launch_pdl(kern, dim3(r, hv), dim3(dv <= 32 ? 64 : dv <= 64 ? 128 : dv <= 128 ? 256 : 512), 0, st, y, xb, x_stride, a_log, dt_bias, nw, rec_state,
-                       qo_indptr, slots, reset, static_cast<bf16*>(out), hk, hv, dv, eps);
+        const int threads = dv <= 32 ? 64 : dv <= 64 ? 128 : dv <= 128 ? 256 : 512;
+        e = launch_pdl(kern, dim3(r, hv), dim3(threads), 0, st, y, xb, x_stride, a_log, dt_bias, nw, rec_state, qo_indptr, slots, reset,
+                       static_cast<bf16*>(out), hk, hv, dv, eps);
         return (int)(e != cudaSuccess ? e : cudaGetLastError());
     }
     if (!coef) return (int)cudaErrorInvalidValue;
