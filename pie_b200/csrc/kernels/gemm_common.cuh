@@ -156,57 +156,6 @@ __device__ __forceinline__ int streamk_cta_of(long long unit, long long total, i
     return (int)(((unit + 1) * grid + total - 1) / total - 1);
 }
 
-
-// Final epilogue of 32 accumulator columns [col0, col0+32) of one output row held by a thread.
-template <int EPI>
-__device__ __forceinline__ void epilogue_store_chunk(const uint32_t (&v)[32], int row, int col0, int M, int N,
-                                                     bf16* __restrict__ C, int ldc, const bf16* __restrict__ R,
-                                                     int ldr, const TpArgs& tp, float limit = 0.f) {
-    if (row >= M || col0 >= N) return;
-    if (EPI == EPI_RS) {
-        const int owner = row / tp.rows_per_rank;
-        const int local = row - owner * tp.rows_per_rank;
-        bf16* dst = tp.peer_recv[owner] + ((size_t)tp.rank * tp.rows_per_rank + local) * (size_t)N + col0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (col0 + 8 * j >= N) break;
-            float o[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(v[8 * j + e]);
-            *reinterpret_cast<bf16x8*>(dst + 8 * j) = pack8(o);
-        }
-    } else if (EPI == EPI_SWIGLU || EPI == EPI_CLAMP_GLU || EPI == EPI_GEGLU) {
-        bf16* dst = C + (size_t)row * ldc + (col0 >> 1);
-        float o[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float g = __uint_as_float(v[2 * j]);
-            const float u = __uint_as_float(v[2 * j + 1]);
-            o[j] = glu_value<EPI>(g, u, limit);
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-            if (col0 + 16 * j < N) *reinterpret_cast<bf16x8*>(dst + 8 * j) = pack8(o + 8 * j);
-    } else {
-        bf16* dst = C + (size_t)row * ldc + col0;
-        const bf16* res = (EPI == EPI_RESIDUAL) ? R + (size_t)row * ldr + col0 : nullptr;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (col0 + 8 * j >= N) break;
-            float o[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(v[8 * j + e]);
-            if (EPI == EPI_RESIDUAL) {
-                float rr[8];
-                unpack8(*reinterpret_cast<const bf16x8*>(res + 8 * j), rr);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] += rr[e];
-            }
-            *reinterpret_cast<bf16x8*>(dst + 8 * j) = pack8(o);
-        }
-    }
-}
-
 // Epilogue of 64 accumulator columns [col0, col0+64) for the 32 rows of one warp, with coalesced
 // global accesses. Thread `lane` holds row (row0 + lane): v0 = columns col0..+31, v1 = +32..+63.
 // The values go through a per-warp staging tile in shared memory (32 rows x 128 B, 16-byte
@@ -223,7 +172,7 @@ __device__ __forceinline__ void epilogue_store_64(const uint32_t (&v0)[32], cons
                                                   const XieluCoef* act = nullptr) {
     const int lane = threadIdx.x & 31;
     auto slot = [&](int r, int c) { return reinterpret_cast<bf16x8*>(stage + r * 128 + ((c ^ (r & 7)) << 4)); };
-    if (EPI == EPI_SWIGLU || EPI == EPI_CLAMP_GLU || EPI == EPI_GEGLU) {
+    if (EPI == EPI_SWIGLU || EPI == EPI_GEGLU) {
         // 64 accumulator columns -> 32 outputs (64 B) per row
         float o[32];
 #pragma unroll
@@ -376,25 +325,6 @@ __device__ __forceinline__ bool ag_gate_wait_rows(const TpArgs& tp, int* status,
     __threadfence_system();
     asm volatile("fence.proxy.async;\n" ::: "memory");
     return true;
-}
-
-// All-gather gate: spin (bounded) until every rank's push flag reached this rank's epoch.
-__device__ __forceinline__ bool ag_gate_wait(const TpArgs& tp, int* status) {
-    const int e = *reinterpret_cast<const volatile int*>(tp.ag_epoch);
-    const long long t0 = clock64();
-    bool ok = true;
-    for (int src = 0; src < tp.world && ok; ++src) {
-        while (*reinterpret_cast<const volatile int*>(tp.ag_flags + src) < e) {
-            if (*reinterpret_cast<volatile int*>(status) != 0 || clock64() - t0 > 1500000000ll) {
-                atomicCAS(status, 0, PIE_ERR_WAIT_PEER);
-                ok = false;
-                break;
-            }
-        }
-    }
-    __threadfence_system();
-    asm volatile("fence.proxy.async;\n" ::: "memory");
-    return ok;
 }
 
 // --------------------------------------------------- swapped operands: rows are features, columns tokens

@@ -134,7 +134,8 @@ class _Graph:
 
 def _rows_as_bytes(t: torch.Tensor) -> List[bytes]:
     """Each row of a float32 matrix as its bytes. From a device they are copied straight into the strings, whose memory is made
-    while the device still works."""
+    while the device still works. A copy per row costs less than one of all rows whose strings are then cut from it: 7 rows of
+    151936 numbers 0.5 against 3.2 ms, 64 rows 17 against 33 ms, 512 rows 119 against 272 ms."""
     if not t.is_cuda or t.numel() == 0:
         return [row.tobytes() for row in t.cpu().numpy()]
     from .._C import pie_host
@@ -845,7 +846,7 @@ class TorchDriver:
 
     def _probes(self, req, logits, slot_logit_row, probe_slots, out_slots):
         """Probe slots (distribution, raw logits, log-probabilities of labels, entropy) of one fire, batched per kind:
-        one pass of device work and one device-to-host copy per kind, whatever the number of slots."""
+        one pass of device work per kind, whatever the number of slots, and one copy to the host (raw logits: one per slot)."""
         rows = slot_logit_row[probe_slots].astype(np.int64)
         whole = len(rows) == logits.shape[0] and bool((rows == np.arange(len(rows))).all())
         lg = logits if whole else logits[torch.from_numpy(rows).to(logits.device)]      # an index copied to the device waits for it
