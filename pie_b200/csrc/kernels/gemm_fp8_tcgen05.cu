@@ -578,6 +578,19 @@ static int fp8_skinny_height(int M, int N, int num_sms) {
     return height;
 }
 
+// The form for small batches runs where its tiles are tall, or where the batch is very small and K long enough: many low tiles wait
+// for the same rows of the batch in L2, and a short K does not pay for the start. Both give the same bits. Measured, this form
+// against the other (us, quantiser included):
+//   tall:           20480 x 5120 at 16 / 32 / 64 rows 34 / 34 / 40 against 71 / 60 / 60, 24576 x 4096 at 40 rows 34 against 56
+//   24 to 63 rows:  10240 x 5120 at 8 rows 30 against 40, 5120 x 25600 at 8 rows 90 against 99, but at 48 rows 139 against 96;
+//                   5120 x 3200 at 16 rows 22 against 26, but 5120 x 1024 17.4 against 15.4
+//   16 rows:        4096 x 12288 at 8 rows 41 against 49, at 12 rows 52 against 48; 1280 x 5120 at 4 rows 24 against 27, at 16 rows 29.5 against 27.6
+static bool fp8_skinny_takes(int M, int N, int K, int num_sms) {
+    if (M > 64 || N < 128 || K < 512) return false;
+    const int height = fp8_skinny_height(M, N, num_sms);
+    return height >= 64 || (K >= 2048 && M <= (height >= 24 ? 16 : 8));
+}
+
 template <int EPI>
 static int launch_fp8_skinny(const void* A8, const float* sa, const void* W8, const float* sw, void* C, const void* R, int M, int N, int K,
                              int ldc, int ldr, int* status, int num_sms, cudaStream_t st) {
@@ -604,10 +617,7 @@ static int gemm_fp8_launch(const void* A8, const float* sa, const void* W8, cons
     if (K <= 0 || K % 16 || N % 16 || (epilogue != EPI_RS && ldc % 8) || (epilogue == EPI_RESIDUAL && ldr % 8))
         return (int)cudaErrorInvalidValue;
     if (epilogue == EPI_SWIGLU && N % 32) return (int)cudaErrorInvalidValue;
-    // The form for small batches where its tiles are tall or the batch is very small: 48 rows against 51200 features 120 -> 71 us,
-    // 8 rows 135 -> 66 us and against 10240 / 5120 features 36 -> 29 / 95 -> 90 us; but 48 rows against 5120 x 25600 would take
-    // 139 us instead of 96, for 214 tiles of 24 rows then wait for the same rows of the batch in L2.
-    if (M <= 64 && N >= 128 && K >= 512 && (M <= 16 || fp8_skinny_height(M, N, num_sms) >= 64)) {
+    if (fp8_skinny_takes(M, N, K, num_sms)) {
         if (epilogue == EPI_STORE) return launch_fp8_skinny<EPI_STORE>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
         if (epilogue == EPI_RESIDUAL) return launch_fp8_skinny<EPI_RESIDUAL>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
         if (epilogue == EPI_SWIGLU) return launch_fp8_skinny<EPI_SWIGLU>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
