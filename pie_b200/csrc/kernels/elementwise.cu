@@ -150,8 +150,8 @@ __global__ void glu_interleaved_kernel(const bf16* __restrict__ gu, bf16* __rest
 // VEC: everything lies on 16-byte boundaries; else elements are read and written one by one.
 // Bound by memory. The token's sines and cosines are worked out once and not by every head's warp again, and rows move in
 // 16-byte pieces. 8300 tokens of 32 + 2 x 8 heads of 128, inputs cold: 91 us with a warp per head, 51 us like this (4.0 TB/s);
-// 512 tokens 12.3 and 10.2 us. 8300 tokens of 4 + 2 heads: 18 us with a warp per head, 29 with a block per token, 16 with four tokens
-// per block; 1 token of 64 + 2 x 8 heads: 8.0 us, 10.4 with its heads in turn, 8.1 with three blocks.
+// 512 tokens 12.3 and 10.2 us. 8300 tokens of 4 + 2 heads: 18 us with a warp per head, 29 with a block per token, 14 with four tokens
+// per block; 1 token of 64 + 2 x 8 heads: 8.2 us, 10.3 with its heads in turn, 8.2 with three blocks.
 constexpr int ROPE_ANGLES = 512;          // of a block's tokens
 template <int D, bool KV8, bool VEC>
 __global__ void __launch_bounds__(256, 5)
@@ -181,10 +181,11 @@ qk_norm_rope_kvwrite_kernel(const bf16* __restrict__ qkv, const int* __restrict_
         load8(src, lo);
         load8(src + D / 2, hi);
     };
+    const int slot = slots[t];
     load(head0 + (at & (at_once - 1)));
     for (int i = threadIdx.x; i < (D / 2) << per_log; i += 256)
         sincosf((float)positions[min(t0 + i / (D / 2), n_tokens - 1)] * inv_freq[i % (D / 2)], &s_sin[i], &s_cos[i]);
-    const int slot = slots[t], page = slot / page_size, off = slot - page * page_size;
+    const int page = slot / page_size, off = slot - page * page_size;
     __syncthreads();
     for (int h0 = head0; h0 < heads; h0 += at_once * gridDim.y) {
         const int h = h0 + (at & (at_once - 1));
