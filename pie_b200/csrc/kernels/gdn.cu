@@ -648,6 +648,8 @@ static int launch_gdn(const void* x, int x_stride, const void* conv_w, const flo
     const int qk = 2 * hk * DK, c = qk + hv * dv;
     const bf16* xb = static_cast<const bf16*>(x);
     const bf16* nw = static_cast<const bf16*>(norm_w);
+    // tokens of a block of gdn_prep: fewer where blocks are few. The mixer over 8192 channels: 40 decode rows 43 us with 4 and 53
+    // with 16, a prompt of 61 tokens 28 and 31, of 150 tokens 48 and 49, from 300 on the same
     const int tile = (long)n * ((c + 127) / 128) <= 16L * PIE_SMS * 4 ? 4 : 16;
     cudaError_t e = launch_pdl(tile == 4 ? gdn_prep_kernel<DK, 4> : gdn_prep_kernel<DK, 16>, dim3((c + 127) / 128, (n + tile - 1) / tile),
                                dim3(128), 0, st, xb, x_stride, static_cast<const bf16*>(conv_w), conv_state, qo_indptr, tok_req, slots,

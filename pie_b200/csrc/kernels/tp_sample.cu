@@ -5,7 +5,8 @@
 // over the kept set) with every block-wide reduction followed by a cross-rank combine: a few
 // words per row travel through peer memory instead of rows * V logits (131 MB per 512-row step at
 // V = 128 256). Noise and tie-breaks are functions of the GLOBAL vocabulary index, so the result
-// equals the single-GPU sampler's on the concatenated logits.
+// equals the single-GPU sampler's on the concatenated logits, but where a key's mass meets top-p to the last
+// bits: masses are 32-bit sums here, in the order of threads and ranks, and that one decides such rows on exact masses.
 //
 // Exchange protocol (plain peer stores / loads over NVLink, no multimem): a CTA owns one row at a
 // time and a mailbox [cta][parity][src rank] of 64-bit words on every rank. To exchange, it stores
