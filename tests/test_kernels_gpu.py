@@ -866,27 +866,39 @@ def test_fp8_gemm_of_small_batches(m, n, k, epi):
 
 
 @pytest.mark.parametrize("vocab", [1024, 32000, 128256, 151936])
-@pytest.mark.parametrize("k,base", [(0, 0.9), (0, 0.6), (0, 0.3), (400, 0.4)])
+@pytest.mark.parametrize("k,base", [(0, None), (0, 0.3), (0, 0.03), (3000, 0.02)])
 def test_sample_does_not_depend_on_the_batch_or_the_run(vocab, k, base):
     """A seed's token stays the same from run to run and whatever shares the batch, also where top-p lies on the edge of a key's mass
-    to the last bits: a sum in another order would move some of these rows to the other side."""
-    rows = 300
+    to the last bits: a sum in another order would move some of these rows to the other side. Edges: of the first candidate's key
+    (base None: rejection rounds), else of the keys around a mass of `base` (exact search)."""
+    rows, near = 300, 75
     lg = bf(1, vocab, scale=2.5, seed=vocab).repeat(rows, 1)
     levels, inverse = torch.unique(lg[0].float(), return_inverse=True)
     mass = torch.zeros(len(levels), dtype=torch.float64, device=DEV).index_add_(0, inverse, torch.softmax(lg[0].double(), 0))
-    above = mass.flip(0).cumsum(0)                                                # of the keys from the top on
-    near = (above - base).abs().argsort()[:20]
-    ulp = torch.arange(-7, 8, device=DEV).double() * 2.0 ** -25
-    p = (above[near][:, None] * (1 + ulp)).flatten()[:rows].float().clamp(max=1 - 2.0 ** -24)
-    seeds = torch.arange(rows, dtype=torch.int64, device=DEV) // 15 + 11
-    one = lambda a: ops.sample(lg[a], torch.ones(len(lg[a]), device=DEV), torch.full((len(lg[a]),), k, dtype=torch.int32, device=DEV), p[a],
-                               torch.zeros(len(lg[a]), device=DEV), seeds[a])
-    want = one(slice(0, rows))
-    for _ in range(5):
-        assert torch.equal(one(slice(0, rows)), want)
-    for step in (1, 40, 148):
-        got = torch.cat([one(slice(a, min(a + step, rows))) for a in range(0, rows, step)])
-        assert torch.equal(got, want), (step, int((got != want).sum()))
+    above = mass.sum() - mass.cumsum(0)                                           # of the keys over each
+
+    def draw(a, p, seeds):
+        n = len(seeds[a])
+        return ops.sample(lg[:n], torch.ones(n, device=DEV), torch.full((n,), k, dtype=torch.int32, device=DEV), p[a],
+                          torch.zeros(n, device=DEV), seeds[a])
+
+    many = torch.arange(1, rows + 1, dtype=torch.int64, device=DEV)
+    for turn in range(4):
+        if base is None:
+            first = draw(slice(0, rows), torch.full((rows,), 1 - 2.0 ** -24, device=DEV), many + turn * rows).long()
+            edge = above[inverse[first]]
+            at = ((edge > 0.5) & (edge < 0.99)).nonzero().flatten()[:rows // near]
+            edge, seed = edge[at], (many + turn * rows)[at]
+        else:
+            edge = above[(above - base).abs().argsort()[turn * 4:turn * 4 + 4]]
+            seed = many[turn * 4:turn * 4 + 4]
+        ulp = (torch.arange(near, device=DEV) - near // 2).double() * 2.0 ** -24
+        p = (edge[:, None] * (1 + ulp)).flatten().float().clamp(max=1 - 2.0 ** -24)
+        seeds = seed[:, None].repeat(1, near).flatten()
+        want = draw(slice(0, len(p)), p, seeds)
+        for step in (len(p), len(p), 148, 40, 1):
+            got = torch.cat([draw(slice(a, min(a + step, len(p))), p, seeds) for a in range(0, len(p), step)])
+            assert torch.equal(got, want), (step, int((got != want).sum()))
 
 
 def test_sample_top_p_of_nothing_is_the_arg_max():
