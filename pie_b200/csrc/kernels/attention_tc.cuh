@@ -151,7 +151,7 @@ paged_prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __
     volatile uint32_t* tmem_slot =
         reinterpret_cast<volatile uint32_t*>(base_ptr + (bar0 - base) + 8u * (1 + 4 * STAGES + NT * AT_TILE_BARS));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tile = blockIdx.x, h = blockIdx.y;
     const int req = tile_req[tile], qstart = tile_qstart[tile];
     const int q_base = qo_indptr[req];
@@ -222,7 +222,7 @@ paged_prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0 && nkb > 0) {
+        if (nkb > 0 && elect_one()) {
             tma_prefetch_desc(&tma_q);
             tma_prefetch_desc(&tma_kv);
             mbar_arrive_expect_tx(q_full(), NT * AT_Q_BYTES);
@@ -287,7 +287,7 @@ paged_prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __
     } else if (warp <= NT) {
         // ------------------------------------------------ MMA warp of tile t: S two blocks ahead of PV
         const int t = warp - 1;
-        if (lane == 0 && nkb > 0) {
+        if (nkb > 0 && elect_one()) {
             constexpr uint32_t idesc_s = make_idesc_bf16(AT_ROWS, AT_BK);
             constexpr uint32_t idesc_o = make_idesc_bf16_bmn(AT_ROWS, D);
             const int my = NT == 1 ? nkb : (t == 0 ? nkb_t[0] : nkb_t[NT - 1]);

@@ -49,7 +49,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     auto tempty_bar = [&](int a) { return bar0 + 8u * (3 * STAGES + 2 + a); };  // leader's is the one in use
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 3 * STAGES + 4);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t crank = cluster_ctarank();
     const bool leader = crank == 0;
     const bool relay = PIE_DIAG(sk.dbg & 4) != 0;
@@ -84,7 +84,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer (each CTA)
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tma_a);
             tma_prefetch_desc(&tma_b);
             uint32_t it = 0;
@@ -130,7 +130,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && !leader && relay) {
+        if (!leader && relay && elect_one()) {
             // ---------------------------------------------------- follower: relay "stage landed"
             uint32_t it = 0;
             bool ok = true;
@@ -143,7 +143,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
                     mbar_arrive_cluster(map_to_cta(peer_bar(s), 0));
                 }
             }
-        } else if (lane == 0 && leader) {
+        } else if (leader && elect_one()) {
             // ---------------------------------------------------- leader: MMA issuer of the pair
             constexpr uint32_t idesc = make_idesc_bf16(PAIR_M, BN);
             uint32_t it = 0, tcount = 0;

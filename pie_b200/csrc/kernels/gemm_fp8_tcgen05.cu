@@ -79,7 +79,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     float* sw_s = reinterpret_cast<float*>(tiles_ptr + STAGES * Cfg::STAGE_BYTES + 256);          // [4 warps][2][BN]
     uint8_t* stage_base = tiles_ptr + STAGES * Cfg::STAGE_BYTES + 256 + Cfg::SCALE_BYTES;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tiles_m = (M + GEMM_BM - 1) / GEMM_BM;
     const int tiles_n = (N + bn - 1) / bn;
     const int num_tiles = tiles_m * tiles_n;
@@ -108,7 +108,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tma_a);
             tma_prefetch_desc(&tma_b);
             uint32_t it = 0;
@@ -130,7 +130,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 mbar_wait(full_bar(j % STAGES), (j / STAGES) & 1u, status, PIE_ERR_WAIT_TMA, 200000000ll);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc_e4m3(GEMM_BM, bn);
             uint32_t it = 0;      // counts K blocks = TMEM buffer uses
             bool ok = true;
@@ -283,7 +283,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
     volatile uint32_t* tmem_slot =
         reinterpret_cast<volatile uint32_t*>(ring_ptr + F8S_RING + F8S_SCALES + 8 * (2 * F8S_MAX_STAGES + 8));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int cols = (M + 15) / 16 * 16, groups = cols / 16;
     const uint32_t w_bytes = (uint32_t)height * F8_BK, slot_bytes = w_bytes + (uint32_t)cols * F8_BK, slot_tx = (uint32_t)(height + M) * F8_BK;
     constexpr uint32_t bufs = 4, buf_cols = 64;
@@ -314,7 +314,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
     pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tma_w);
             tma_prefetch_desc(&tma_x);
             // the weights depend on nothing and fill the ring at once; the batch's tiles follow when the producing kernel is done
@@ -349,7 +349,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
                 mbar_wait(full_bar(j % stages), (j / stages) & 1u, status, PIE_ERR_WAIT_TMA, 200000000ll);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc_e4m3(GEMM_BM, cols);
             int s = 0;
             uint32_t ph = 0, buf = 0, bph = 0;

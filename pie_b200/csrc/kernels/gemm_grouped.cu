@@ -76,7 +76,7 @@ gemm_grouped_kernel(const __grid_constant__ GroupedMaps maps, bf16* __restrict__
     auto tempty_bar = [&](int a) { return bar0 + 8u * (2 * GG_STAGES + 2 + a); };   // the leader's is the one in use
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(ring_ptr + GG_STAGES * GG_STAGE_BYTES + 8 * (2 * GG_STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t crank = cluster_ctarank();
     const bool leader = crank == 0;
     const int pid = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -108,7 +108,7 @@ gemm_grouped_kernel(const __grid_constant__ GroupedMaps maps, bf16* __restrict__
     const int items = grouped_count(work) * tiles_n;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&maps.w);
             const uint32_t leader_full0 = map_to_cta(full_bar(0), 0);
             uint32_t it = 0;
@@ -141,7 +141,7 @@ gemm_grouped_kernel(const __grid_constant__ GroupedMaps maps, bf16* __restrict__
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader && elect_one()) {
             uint32_t it = 0, tcount = 0;
             bool ok = true;
             for (int item = pid; item < items && ok; item += npairs) {

@@ -44,7 +44,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     auto tempty_bar = [&](int a) { return bar0 + 8u * (2 * SKINNY_MAX_STAGES + 2 + a); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(ring_ptr + SKINNY_RING + 8 * (2 * SKINNY_MAX_STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int cols = (M + 15) / 16 * 16;                       // columns of the MMA
     const uint32_t slot_bytes = SKINNY_W_BYTES + (uint32_t)cols * (GEMM_BK * 2);
     const uint32_t slot_tx = SKINNY_W_BYTES + (uint32_t)M * (GEMM_BK * 2);
@@ -78,7 +78,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     pdl_trigger();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tma_w);
             tma_prefetch_desc(&tma_x);
             // Weights that depend on nothing fill the ring at once; the batch's tiles follow when the producing kernel is
@@ -115,7 +115,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 mbar_wait(full_bar(j % stages), (j / stages) & 1u, status, PIE_ERR_WAIT_TMA, 200000000ll);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc_bf16(GEMM_BM, cols);
             int s = 0;
             uint32_t ph = 0, count = 0;

@@ -69,7 +69,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     auto tempty_bar = [&](int a) { return bar0 + 8u * (2 * STAGES + 2 + a); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * STAGES + 4);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int tiles_m = (M + bm - 1) / bm;
     const int tiles_n = (N + bn - 1) / bn;
     const int num_tiles = tiles_m * tiles_n;
@@ -102,7 +102,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tma_a);
             tma_prefetch_desc(&tma_b);
             uint32_t it = 0;
@@ -184,7 +184,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         }
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc_bf16(GEMM_BM, bn);
             uint32_t it = 0, tcount = 0;
             bool ok = true;

@@ -144,7 +144,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
     int* tiles_s = reinterpret_cast<int*>(l_s + 4 * LT_HEADS);                  // tiles of the MMA warp's next 32 items
     volatile int* failed = tiles_s + 32;                                        // [2 groups] a warp of the group gave up on a wait
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int h0 = blockIdx.y * LT_HEADS, hn = min(LT_HEADS, a.heads - h0);
     if (threadIdx.x == 0) {
         for (int s = 0; s < LT_STAGES; ++s) {
@@ -227,7 +227,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
             __syncwarp();
             tiles_s[lane] = lt_item(a, chunk + lane, item1).tiles;
             __syncwarp();
-            if (lane != 0) continue;
+            if (!elect_one()) continue;
             for (int i = 0; i < min(32, item1 - chunk) && ok; ++i) {
                 const int tiles = tiles_s[i];
                 if (tiles == 0) continue;
