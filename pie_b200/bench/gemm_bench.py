@@ -56,7 +56,7 @@ def main():
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
     import ctypes as C
     from ..ops import _lib
-    thresholds = _lib.declare("pie_gemm_set_pair_thresholds", [C.c_double, C.c_double])
+    width = _lib.declare("pie_gemm_set_pair_width", [C.c_int])
     print(f"{'M':>6} {'N':>7} {'K':>6} | {'cuBLAS us':>10} {'TF':>6} | {'default us':>9} {'TF':>6} | {'1-CTA us':>9} {'TF':>6} | "
           f"{'pairs us':>9} {'TF':>6} | max err")
     for m, n, k in shapes:
@@ -70,9 +70,9 @@ def main():
         ops.set_gemm_pairs(False)
         t_1 = timeit(lambda: ops.gemm(x, w), flush)
         ops.set_gemm_pairs(True)
-        thresholds(0.0, 0.0)              # the CTA-pair kernel whatever the problem size
+        width(-1)                         # the CTA-pair kernel whatever the problem size
         t_f = timeit(lambda: ops.gemm(x, w), flush)
-        thresholds(1.0e10, 2.0e10)
+        width(0)
         err = (y.float() - torch.matmul(x, w.t()).float()).abs().max().item()
         print(f"{m:6d} {n:7d} {k:6d} | {t_cb*1e3:10.1f} {fl/t_cb/1e9:6.0f} | {t_p*1e3:9.1f} {fl/t_p/1e9:6.0f} | "
               f"{t_1*1e3:9.1f} {fl/t_1/1e9:6.0f} | {t_f*1e3:9.1f} {fl/t_f/1e9:6.0f} | {err:.3f}")

@@ -93,7 +93,7 @@ struct StreamKArgs {
     int* cnt;
     int enabled;
     // Diagnostics, compiled in only with -DPIE_GEMM_DIAG (a production build ignores both fields):
-    int dbg;   // 1 skip the MMAs, 2 skip the loads, 4 relay instead of direct signalling (results are meaningless)
+    int dbg;   // 1 skip the MMAs, 2 the activation loads, 4 the weight loads (results are meaningless)
     unsigned long long* trace;   // [grid][8] globaltimer stamps of the kernel's phases
 };
 
@@ -120,7 +120,7 @@ struct SegmentWalk {
     long long u, u_end;
     int t, t_step, num_tiles, num_kb;
     bool sk;
-    // worker = CTA (or CTA pair) index, workers = how many share the problem
+    // worker = CTA index, workers = how many share the problem
     __device__ SegmentWalk(bool streamk, int num_tiles_, int num_kb_, int worker, int workers)
         : num_tiles(num_tiles_), num_kb(num_kb_), sk(streamk) {
         if (sk) {

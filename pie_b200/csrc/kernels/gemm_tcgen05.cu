@@ -429,8 +429,7 @@ PIE_API int pie_gemm_set_swap(int max_m) { g_gemm_swap_max_m = max_m; return 0; 
 
 int pie_gemm2_dispatch(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda,
                        int ldw, int ldc, int ldr, int epilogue, int* status, int num_sms, cudaStream_t st,
-                       const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, int* handled,
-                       const EpiArgs& ex = EpiArgs());
+                       const TpArgs* tp_in, int* handled, const EpiArgs& ex = EpiArgs());
 
 int pie_gemm_skinny_rows(int N, int K, int num_sms);
 int pie_gemm_skinny(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda, int ldw, int ldc, int ldr,
@@ -560,7 +559,7 @@ static int current_workspace(GemmWorkspace* out) {
 // C[M,N] (or [M,N/2] for the SwiGLU epilogue) = A[M,K] * W[N,K]^T.
 // `status` is a device int that stays 0 unless a bounded wait ran out.
 // `ex.fresh_w`: W is the output of an earlier launch of the stream. The single-CTA kernels request weights ahead of the grid
-// dependency, and an earlier launch's stores are only sure to be seen behind it. The pair kernel is launched without overlap.
+// dependency, and an earlier launch's stores are only sure to be seen behind it. The pair kernel requests nothing before it.
 static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda, int ldw, int ldc, int ldr,
                      int epilogue, int force_bn, int* status, int num_sms, cudaStream_t st, const EpiArgs& ex) {
     if (M <= 0 || N <= 0) return 0;
@@ -572,7 +571,7 @@ static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M
     if (g_gemm_pairs && force_bn == 0) {
         int handled = 0;
         const int rc = pie_gemm2_dispatch(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, status, num_sms, st,
-                                          nullptr, w.ws, w.ws_floats, w.cnt, w.cnt_ints, &handled, ex);
+                                          nullptr, &handled, ex);
         if (handled || rc) return rc;
     }
     if (force_bn == 0 && M <= GEMM_BM &&
@@ -669,7 +668,7 @@ PIE_API int pie_gemm_bf16_tp(const void* A, const void* W, void* C, int M, int N
     if (g_gemm_pairs && force_bn == 0) {
         int handled = 0;
         const int rc = pie_gemm2_dispatch(A, W, C, nullptr, M, N, K, lda, ldw, ldc, 0, epilogue, status, num_sms,
-                                          st, &tp, w.ws, w.ws_floats, w.cnt, w.cnt_ints, &handled);
+                                          st, &tp, &handled);
         if (handled || rc) return rc;
     }
     if (force_bn < 0 || force_bn > 256 || force_bn % 16) return (int)cudaErrorInvalidValue;

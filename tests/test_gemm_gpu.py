@@ -1,9 +1,11 @@
 """tcgen05 GEMM against an fp32 PyTorch reference (and its fused epilogues)."""
+import ctypes
+
 import pytest
 import torch
 
 from pie_b200 import ops
-from pie_b200.ops import reference as ref
+from pie_b200.ops import _lib, reference as ref
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -102,6 +104,33 @@ def test_gemm_odd_tile_widths(bn, epi):
     if epi == "swiglu":
         want = ref.swiglu_interleaved(want)
     check(y, want, k)
+
+
+@pytest.mark.parametrize("bn", [64, 80, 96, 112, 144, 160, 176, 208, 224, 256])
+@pytest.mark.parametrize("m,n,k", [(129, 128, 64), (256, 1000, 72), (257, 1032, 520), (700, 2080, 1096), (2305, 520, 136), (1025, 9216, 256)])
+@pytest.mark.parametrize("epi", ["store", "residual", "swiglu"])
+def test_gemm_pair_tile_widths(bn, m, n, k, epi):
+    """CTA-pair tiles of every kind of width (last chunk of the epilogue whole or not, fewer columns than a chunk), one or more tiles
+    per pair, ragged ends of all three sizes. 32-bit sums of one product differ by their order alone: one rounding to bf16 (2^-9), or
+    two with a GLU's own error, of values near 1."""
+    if epi == "swiglu":
+        n = n // 32 * 32
+    x, w = bf(m, k, seed=51), bf(n, k, scale=k ** -0.5, seed=52)
+    r = bf(m, n, seed=53) if epi == "residual" else None
+    e = {"store": ops.EPI_STORE, "residual": ops.EPI_RESIDUAL, "swiglu": ops.EPI_SWIGLU}[epi]
+    width = _lib.declare("pie_gemm_set_pair_width", [ctypes.c_int])
+    width(bn)
+    try:
+        y = ops.gemm(x, w, residual=r, epilogue=e)
+    finally:
+        width(0)
+    want = x.float() @ w.float().t()
+    if epi == "residual":
+        want = want + r.float()
+    if epi == "swiglu":
+        want = ref.swiglu_interleaved(want)
+    ops.check_kernel_status()
+    torch.testing.assert_close(y.float(), want, rtol=2 ** -8, atol=2e-3)
 
 
 @pytest.mark.parametrize("m", [1, 7, 64, 65, 100, 128])
