@@ -424,24 +424,28 @@ class TorchDriver:
         k = len(token_slots)
         if k > self.max_rows:
             raise ValueError("too many sampler rows")
-        t, tk = s.h("temperature", np.float32), s.h("top_k")
-        tp, mp = s.h("top_p", np.float32), s.h("min_p", np.float32)
-        seeds = s.h("seeds", np.int64)
-        for j, i in enumerate(token_slots):
-            sp = req.slot_samplers[i]
-            t[j] = sp.temperature
-            tk[j] = sp.top_k if sp.kind in (SamplerKind.TOP_K, SamplerKind.TOP_K_TOP_P) else 0
-            tp[j] = sp.top_p if sp.kind in (SamplerKind.TOP_P, SamplerKind.TOP_K_TOP_P) else 1.0
-            mp[j] = sp.min_p if sp.kind == SamplerKind.MIN_P else 0.0
-            if sp.seed and sp.seed_final:
-                seeds[j] = sp.seed
-            elif sp.seed:
-                # a user-fixed seed is mixed with the position of the sampled row, as the cohort does
-                row = int(req.slot_row[i]) if req.slot_row is not None else -1
-                pos = int(req.positions[row]) if 0 <= row < len(req.positions) else 0
-                seeds[j] = int(position_seed(sp.seed, pos))
-            else:
-                seeds[j] = int(self.rng.integers(1, 2**62))
+        if k == 0:
+            return token_slots
+        # filled an array at a time: mixing a fixed seed slot by slot, as numpy scalars, took 9 us of every slot
+        specs = [req.slot_samplers[i] for i in token_slots]
+        s.h("temperature", np.float32)[:k] = [sp.temperature for sp in specs]
+        s.h("top_k")[:k] = [sp.top_k if sp.kind in (SamplerKind.TOP_K, SamplerKind.TOP_K_TOP_P) else 0 for sp in specs]
+        s.h("top_p", np.float32)[:k] = [sp.top_p if sp.kind in (SamplerKind.TOP_P, SamplerKind.TOP_K_TOP_P) else 1.0 for sp in specs]
+        s.h("min_p", np.float32)[:k] = [sp.min_p if sp.kind == SamplerKind.MIN_P else 0.0 for sp in specs]
+        seeds = np.array([sp.seed for sp in specs], dtype=np.int64)
+        mixed = (seeds != 0) & ~np.array([bool(sp.seed_final) for sp in specs])
+        if mixed.any():
+            # a user-fixed seed is mixed with the position of the sampled row, as the cohort does
+            positions = np.asarray(req.positions)
+            at = np.full(k, -1, np.int64) if req.slot_row is None else np.asarray(req.slot_row, dtype=np.int64)[token_slots]
+            inside = (at >= 0) & (at < len(positions))
+            pos = np.zeros(k, np.int64)
+            pos[inside] = positions[at[inside]]
+            seeds = np.where(mixed, position_seed(seeds, pos), seeds)
+        fresh = np.array([not sp.seed for sp in specs])
+        if fresh.any():
+            seeds[fresh] = self.rng.integers(1, 2**62, size=int(fresh.sum()))
+        s.h("seeds", np.int64)[:k] = seeds
         return token_slots
 
     # ------------------------------------------------------------------ forward variants

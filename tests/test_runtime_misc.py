@@ -303,3 +303,36 @@ def test_ragged_brle_expansion_on_the_cpu_path():
         assert np.array_equal(got, brle.decode(r, n)), i
     empty, offs0 = ops.brle_expand_ragged([], [], "cpu")
     assert empty.numel() == 0 and offs0.tolist() == [0]
+
+
+def test_sampler_parameters_of_a_fire_equal_those_worked_out_slot_by_slot():
+    """Parameters and seeds of a fire's token slots, filled an array at a time: every kind, probes in between, seeds that are final, fixed
+    (mixed with the position of the row; rows outside the batch count as position 0) or drawn one after the other."""
+    from pie_b200.driver.executor import TorchDriver, _Slab
+    from pie_b200.driver.schema import ForwardRequest, SamplerKind, SamplerSpec, position_seed
+
+    rng = np.random.default_rng(3)
+    kinds = [k for k in SamplerKind]
+    specs = [SamplerSpec(kinds[i % len(kinds)], temperature=float(rng.random()), top_k=int(rng.integers(0, 99)), top_p=float(rng.random()),
+                         min_p=float(rng.random()), seed=int(rng.integers(1, 2 ** 62)) * (i % 3 > 0), seed_final=i % 6 > 3) for i in range(60)]
+    positions = rng.integers(0, 5000, 40).astype(np.int32)
+    for rows in (rng.integers(-2, 45, len(specs)).astype(np.int32), None):
+        for chosen in (specs, specs[:1], []):
+            drv = TorchDriver.__new__(TorchDriver)
+            drv.max_rows, drv.rng = 64, np.random.default_rng(7)
+            drv.slab = _Slab({"temperature": 64, "top_k": 64, "top_p": 64, "min_p": 64, "seeds": 128}, "cpu")
+            req = ForwardRequest(tokens=np.zeros(40, np.int32), positions=positions, qo_indptr=np.array([0, 40]), kv_page_indices=None,
+                                 kv_page_indptr=None, kv_last_page_lens=None, slot_row=rows, slot_samplers=chosen)
+            got = drv._sampler_params(req, None)
+            assert got == [i for i, sp in enumerate(chosen) if sp.is_token]
+            draw = np.random.default_rng(7)
+            for j, i in enumerate(got):
+                sp, row = chosen[i], -1 if rows is None else int(rows[i])
+                seed = sp.seed if sp.seed and sp.seed_final else int(position_seed(sp.seed, int(positions[row]) if 0 <= row < 40 else 0)) \
+                    if sp.seed else int(draw.integers(1, 2 ** 62))
+                want = (np.float32(sp.temperature), sp.top_k if sp.kind in (SamplerKind.TOP_K, SamplerKind.TOP_K_TOP_P) else 0,
+                        np.float32(sp.top_p if sp.kind in (SamplerKind.TOP_P, SamplerKind.TOP_K_TOP_P) else 1.0),
+                        np.float32(sp.min_p if sp.kind == SamplerKind.MIN_P else 0.0), seed)
+                s = drv.slab
+                assert (s.h("temperature", np.float32)[j], s.h("top_k")[j], s.h("top_p", np.float32)[j], s.h("min_p", np.float32)[j],
+                        s.h("seeds", np.int64)[j]) == want
