@@ -242,30 +242,35 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 
 // ------------------------------------------------------------------------------------------ batches of up to 64 rows
 // Laid out for streaming the weights, as the bf16 kernel for such batches (gemm_skinny.cu): operands swapped (weight rows are
-// the MMA's rows, the batch its 16..64 columns), half an SM per CTA, the ring filled with weights before the producing kernel is
-// done. K is not split: the sum over its blocks keeps the order of the kernel above, because the next layer's quantiser turns a
-// last bit into a step of 8-bit numbers. (Split over clusters, 48 rows against 5120 x 25600 took 47 us instead of 96; results of
-// one layer then agree to 3e-5, logits of four layers only to 4 %.) Instead a tile has as few weight rows as fill the machine
-// (`height`): the MMA's other rows are whatever shared memory holds, each reaches its own accumulator row alone, and these are
-// not read.
+// the MMA's rows, the batch its 16..64 columns), the ring filled with weights before the producing kernel is done. K is not
+// split: the sum over its blocks keeps the order of the kernel above, because the next layer's quantiser turns a last bit into
+// a step of 8-bit numbers. (Split over clusters, results of one layer agree to 3e-5, logits of four layers only to 4 %.) A tile has
+// `height` weight rows: the MMA's other rows are whatever shared memory holds, each reaches its own accumulator row alone, and
+// these are not read.
 //
-// What block scaling adds: every 128 of K has a partial product of its own in tensor memory (four of them in flight), which the
-// epilogue warps scale and add up in registers - warp w the 32 features of quarter w % 4 and every other group of 16 tokens.
-// The scales of features and tokens come through shared memory, four K blocks at a time and three such chunks ahead.
+// What block scaling adds: every 128 of K has a partial product of its own in tensor memory, which the epilogue warps scale and
+// add up in registers - warp w the 32 features of quarter w % 4 and every other group of 16 tokens. With a hand-over per block that
+// chain was what a launch took (0.3 us a block whatever the tile), so blocks are handed over in groups of four, two groups in
+// flight: one barrier, and the loads of two blocks under way at once. That takes all of tensor memory and the registers of one CTA
+// per SM, which also halves the CTAs that ask L2 for the same rows of the batch. The scales of features and tokens come through
+// shared memory, four K blocks at a time and seven such chunks ahead.
 //
-// 48 rows against 51200 x 5120 (gate / up): 120 us with 128-row boxes of activations that are zero-filled row by row, weight scales
-// gathered per K block and 400 tiles on 148 SMs; 71 us (3.8 TB/s) like this.
+// Weights cold, at 8 / 24 / 48 / 64 rows (us): 5120 x 25600 (20.6 at the memory's rate) with two CTAs per SM, block by block,
+// 65 / 74 / 89 / 98, by the kernel above 74 / 74 / 75 / 75, like this 48 / 51 / 56 / 66; 10240 x 5120 17 / 19 / 21 / 23 and 13 / 14 / 15 / 16;
+// 51200 x 5120 42 / 43 / 51 / 57 and 41 / 42 / 45 / 48 (6.4 to 5.5 TB/s); 24576 x 4096 18.1 / 18.8 / 21.8 / 24.2 and 19.0 / 20.1 / 22.2 / 24.4.
 constexpr int F8S_THREADS = 64 + 256, F8S_CHUNK = 4;
 constexpr uint32_t F8S_MMA_BYTES = GEMM_BM * F8_BK;          // what an MMA reads from a slot's start on
-constexpr int F8S_DEPTH = 4;                                   // chunks of scales: one in use, three on their way
-constexpr uint32_t F8S_RING = 96 * 1024;
+constexpr uint32_t F8S_BUFS = 2;                               // groups of F8S_CHUNK blocks in tensor memory
+constexpr uint32_t F8S_BLOCK_COLS = 64, F8S_TMEM_COLS = F8S_BUFS * F8S_CHUNK * F8S_BLOCK_COLS;
+constexpr int F8S_DEPTH = 8;                                   // chunks of scales: one in use, the others on their way
+constexpr uint32_t F8S_RING = 176 * 1024;
 constexpr uint32_t F8S_SCALES = F8S_DEPTH * F8S_CHUNK * (64 + GEMM_BM) * 4;
 constexpr uint32_t F8S_SMEM = F8S_RING + F8S_SCALES + 1024 /*align*/ + 512 /*barriers*/;
-constexpr int F8S_MAX_STAGES = 12;
+constexpr int F8S_MAX_STAGES = 20;
 
-// height: weight rows of a tile and of its box, a multiple of 8.
+// height: weight rows of a tile and of its box, a multiple of 16.
 template <int EPI>
-__global__ void __launch_bounds__(F8S_THREADS, 2)
+__global__ void __launch_bounds__(F8S_THREADS, 1)
 gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x,
                        const float* __restrict__ sa, const float* __restrict__ sw, bf16* __restrict__ C, const bf16* __restrict__ R,
                        int M, int N, int K, int ldc, int ldr, int* status, int stages, int height) {
@@ -286,7 +291,6 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int cols = (M + 15) / 16 * 16, groups = cols / 16;
     const uint32_t w_bytes = (uint32_t)height * F8_BK, slot_bytes = w_bytes + (uint32_t)cols * F8_BK, slot_tx = (uint32_t)(height + M) * F8_BK;
-    constexpr uint32_t bufs = 4, buf_cols = 64;
     const int tiles = (N + height - 1) / height, num_kb = (K + F8_BK - 1) / F8_BK;
     const int tile0 = blockIdx.x, tile_step = gridDim.x;
     const int quarters = (height + 31) / 32;
@@ -296,7 +300,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
-        for (uint32_t a = 0; a < bufs; ++a) {
+        for (uint32_t a = 0; a < F8S_BUFS; ++a) {
             mbar_init(tfull_bar(a), 1);
             mbar_init(tempty_bar(a), 2 * quarters);
         }
@@ -304,7 +308,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
         fence_proxy_async();
     }
     if (warp == 1) {
-        tmem_alloc(smem_addr(const_cast<uint32_t*>(tmem_slot)), 256);
+        tmem_alloc(smem_addr(const_cast<uint32_t*>(tmem_slot)), F8S_TMEM_COLS);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -355,18 +359,24 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
             uint32_t ph = 0, buf = 0, bph = 0;
             bool ok = true;
             for (int tile = tile0; tile < tiles && ok; tile += tile_step) {
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(tempty_bar(buf), bph ^ 1u, status, PIE_ERR_WAIT_EPILOGUE) ||
-                        !mbar_wait(full_bar(s), ph, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t wd = make_smem_desc_sw128(ring + s * slot_bytes);
-                    const uint64_t xd = make_smem_desc_sw128(ring + s * slot_bytes + w_bytes);
+                for (int kb = 0; kb < num_kb; kb += F8S_CHUNK) {
+                    if (!mbar_wait(tempty_bar(buf), bph ^ 1u, status, PIE_ERR_WAIT_EPILOGUE)) { ok = false; break; }
 #pragma unroll
-                    for (int k = 0; k < F8_BK / 32; ++k) umma_f8(tmem_base + buf * buf_cols, wd + 2u * k, xd + 2u * k, idesc, k != 0);
-                    umma_commit(empty_bar(s));
+                    for (int j = 0; j < F8S_CHUNK; ++j) {
+                        if (kb + j >= num_kb) break;
+                        if (!mbar_wait(full_bar(s), ph, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint64_t wd = make_smem_desc_sw128(ring + s * slot_bytes);
+                        const uint64_t xd = make_smem_desc_sw128(ring + s * slot_bytes + w_bytes);
+#pragma unroll
+                        for (int k = 0; k < F8_BK / 32; ++k)
+                            umma_f8(tmem_base + (buf * F8S_CHUNK + j) * F8S_BLOCK_COLS, wd + 2u * k, xd + 2u * k, idesc, k != 0);
+                        umma_commit(empty_bar(s));
+                        if (++s == stages) { s = 0; ph ^= 1u; }
+                    }
+                    if (!ok) break;
                     umma_commit(tfull_bar(buf));
-                    if (++s == stages) { s = 0; ph ^= 1u; }
-                    if (++buf == bufs) { buf = 0; bph ^= 1u; }
+                    if (++buf == F8S_BUFS) { buf = 0; bph ^= 1u; }
                 }
             }
         }
@@ -417,38 +427,45 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
             }
             const float4 of = *reinterpret_cast<const float4*>(swt + (b * GEMM_BM + q * 32 + lane) * F8S_CHUNK);
             const float mine[F8S_CHUNK] = {of.x, of.y, of.z, of.w};
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(buf), bph, status, PIE_ERR_WAIT_MMA));
+            if (ok) {
+                tc_fence_after();
+                const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * F8S_CHUNK * F8S_BLOCK_COLS;
 #pragma unroll
-            for (int j = 0; j < F8S_CHUNK; ++j) {
-                if (kb + j >= num_kb) break;
-                if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(buf), bph, status, PIE_ERR_WAIT_MMA));
-                if (ok) {
-                    tc_fence_after();
-                    const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * buf_cols;
-                    const float* scales = sx + (b * F8S_CHUNK + j) * 64;
-                    uint32_t v[2][16];
+                for (int j1 = 0; j1 < F8S_CHUNK; j1 += 2) {              // two blocks' products in registers at once
+                    uint32_t v[2][2][16];
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        if (2 * i + half < groups) tmem_ld_32x16(t_row + (2 * i + half) * 16, v[i]);
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            if (2 * i + half < groups) tmem_ld_32x16(t_row + (j1 + j) * F8S_BLOCK_COLS + (2 * i + half) * 16, v[j][i]);
                     tmem_ld_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(tempty_bar(buf));
+                    if (j1 + 2 == F8S_CHUNK) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(tempty_bar(buf));
+                    }
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int g = 2 * i + half;
-                        if (g >= groups) break;
+                    for (int j = 0; j < 2; ++j) {
+                        if (kb + j1 + j >= num_kb) break;
+                        const float* scales = sx + (b * F8S_CHUNK + j1 + j) * 64;
 #pragma unroll
-                        for (int t = 0; t < 16; t += 4) {
-                            const float4 f = *reinterpret_cast<const float4*>(scales + g * 16 + t);
-                            acc[i][t] = fmaf(__uint_as_float(v[i][t]), f.x * mine[j], acc[i][t]);
-                            acc[i][t + 1] = fmaf(__uint_as_float(v[i][t + 1]), f.y * mine[j], acc[i][t + 1]);
-                            acc[i][t + 2] = fmaf(__uint_as_float(v[i][t + 2]), f.z * mine[j], acc[i][t + 2]);
-                            acc[i][t + 3] = fmaf(__uint_as_float(v[i][t + 3]), f.w * mine[j], acc[i][t + 3]);
+                        for (int i = 0; i < 2; ++i) {
+                            const int g = 2 * i + half;
+                            if (g >= groups) break;
+#pragma unroll
+                            for (int t = 0; t < 16; t += 4) {
+                                const float4 f = *reinterpret_cast<const float4*>(scales + g * 16 + t);
+                                acc[i][t] = fmaf(__uint_as_float(v[j][i][t]), f.x * mine[j1 + j], acc[i][t]);
+                                acc[i][t + 1] = fmaf(__uint_as_float(v[j][i][t + 1]), f.y * mine[j1 + j], acc[i][t + 1]);
+                                acc[i][t + 2] = fmaf(__uint_as_float(v[j][i][t + 2]), f.z * mine[j1 + j], acc[i][t + 2]);
+                                acc[i][t + 3] = fmaf(__uint_as_float(v[j][i][t + 3]), f.w * mine[j1 + j], acc[i][t + 3]);
+                            }
                         }
                     }
                 }
-                if (++buf == bufs) { buf = 0; bph ^= 1u; }
             }
+            if (++buf == F8S_BUFS) { buf = 0; bph ^= 1u; }
             if (kb + F8S_CHUNK >= num_kb && ok) {
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
@@ -465,7 +482,7 @@ gemm_fp8_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_c
     if (warp == 1) {
         __syncwarp();
         tc_fence_after();
-        tmem_dealloc(tmem_base, 256);
+        tmem_dealloc(tmem_base, F8S_TMEM_COLS);
     }
 }
 
@@ -564,37 +581,27 @@ PIE_API int pie_gemm_fp8_blockscaled_tp(const void* A8, const float* sa, const v
     return gemm_fp8_launch(A8, sa, W8, sw, C, nullptr, M, N, K, ldc, 0, epilogue, status, num_sms, st, tp);
 }
 
-// Weight rows of a tile: whole rounds of the machine (two CTAs per SM) of as little as possible, a CTA's work being its weight
-// rows, the batch's rows (from L2: at 0.4) and what a tile costs beside them. 48 rows: 5120 features in 214 tiles of 24 rows,
-// 10240 in 256 of 40, 51200 in two rounds of 88 (and not 400 tiles of 128 on 296 places).
-static int fp8_skinny_height(int M, int N, int num_sms) {
-    int height = GEMM_BM;
-    double best = 0.;
-    for (int h = GEMM_BM; h >= 16; h -= 8) {
-        const long rounds = ((N + h - 1) / h + 2 * num_sms - 1) / (2 * num_sms);
-        const double cost = (double)rounds * (h + 0.4 * M + 6.);
-        if (h == GEMM_BM || cost < best) { best = cost; height = h; }
-    }
-    return height;
+// Weight rows of a tile: where one round of the machine will do, as many as leave 64 tiles or so - what a round takes hardly depends on
+// its tiles' rows, and more CTAs ask L2 for the same rows of the batch - else as few as leave the rounds as few. Whole quarters of 32 (two
+// warps each), or halves of them where that would end at 128. Measured at 4 / 48 rows (us): 5120 x 25600 in tiles of 24 rows (two rounds)
+// 91 / 110, of 40 49 / 57, of 64 48 / 56; 6144 x 4096 of 48 12.6 / 13.0, of 64 11.4 / 12.3, of 96 10.1 / 11.6; 8192 x 8192 of 64 19.3 / 21.0, of
+// 128 17.2 / 20.8; 28672 x 4096 of 112 20.5 / 23.1, of 128 21.5 / 23.9; 51200 x 5120 of 88 (four rounds) 42.0 / 50.5, of 128 41.5 / 44.2.
+static int fp8_skinny_height(int N, int num_sms) {
+    const int rounds = ((N + GEMM_BM - 1) / GEMM_BM + num_sms - 1) / num_sms;
+    int least = (N + rounds * num_sms - 1) / (rounds * num_sms);
+    if (rounds == 1) least = std::min(GEMM_BM, std::max(least, (N + 63) / 64));
+    const int height = (least + 31) / 32 * 32;
+    return height < GEMM_BM ? height : (least + 15) / 16 * 16;
 }
 
-// The form for small batches runs where its tiles are tall, or where the batch is very small and K long enough: many low tiles wait
-// for the same rows of the batch in L2, and a short K does not pay for the start. Both give the same bits. Measured, this form
-// against the other (us, quantiser included):
-//   tall:           20480 x 5120 at 16 / 32 / 64 rows 34 / 34 / 40 against 71 / 60 / 60, 24576 x 4096 at 40 rows 34 against 56
-//   24 to 63 rows:  10240 x 5120 at 8 rows 30 against 40, 5120 x 25600 at 8 rows 90 against 99, but at 48 rows 139 against 96;
-//                   5120 x 3200 at 16 rows 22 against 26, but 5120 x 1024 17.4 against 15.4
-//   16 rows:        4096 x 12288 at 8 rows 41 against 49, at 12 rows 52 against 48; 1280 x 5120 at 4 rows 24 against 27, at 16 rows 29.5 against 27.6
-static bool fp8_skinny_takes(int M, int N, int K, int num_sms) {
-    if (M > 64 || N < 128 || K < 512) return false;
-    const int height = fp8_skinny_height(M, N, num_sms);
-    return height >= 64 || (K >= 2048 && M <= (height >= 24 ? 16 : 8));
-}
+// Up to 64 rows run here: the bits of the kernel above in less time wherever measured (1 to 64 rows, 1280 to 51200 features, K from 1024
+// on: 5120 x 1024 4.6 to 6.0 us against 7.2). Fewer features or a shorter K are not worth the set-up.
+static bool fp8_skinny_takes(int M, int N, int K) { return M <= 64 && N >= 128 && K >= 512; }
 
 template <int EPI>
 static int launch_fp8_skinny(const void* A8, const float* sa, const void* W8, const float* sw, void* C, const void* R, int M, int N, int K,
                              int ldc, int ldr, int* status, int num_sms, cudaStream_t st) {
-    const int height = fp8_skinny_height(M, N, num_sms);
+    const int height = fp8_skinny_height(N, num_sms);
     CUtensorMap tw, tx;
     if (make_tma_2d_u8(&tw, W8, N, K, K, height) != 0) return (int)cudaErrorInvalidValue;
     if (make_tma_2d_u8(&tx, A8, M, K, K, M) != 0) return (int)cudaErrorInvalidValue;      // the box ends with the batch
@@ -605,7 +612,7 @@ static int launch_fp8_skinny(const void* A8, const float* sa, const void* W8, co
     // an MMA reads 128 rows from the last slot's start, too: they have to lie in the ring
     const uint32_t slot = (uint32_t)(height + (M + 15) / 16 * 16) * F8_BK;
     const int stages = (int)std::min({(uint32_t)F8S_MAX_STAGES, F8S_RING / slot, (F8S_RING - F8S_MMA_BYTES) / slot + 1});
-    e = launch_pdl(kern, dim3(std::min(tiles, 2 * num_sms)), dim3(F8S_THREADS), F8S_SMEM, st, tw, tx, sa, sw, (bf16*)C, (const bf16*)R, M, N, K,
+    e = launch_pdl(kern, dim3(std::min(tiles, num_sms)), dim3(F8S_THREADS), F8S_SMEM, st, tw, tx, sa, sw, (bf16*)C, (const bf16*)R, M, N, K,
                    ldc, ldr, status, stages, height);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
@@ -617,7 +624,7 @@ static int gemm_fp8_launch(const void* A8, const float* sa, const void* W8, cons
     if (K <= 0 || K % 16 || N % 16 || (epilogue != EPI_RS && ldc % 8) || (epilogue == EPI_RESIDUAL && ldr % 8))
         return (int)cudaErrorInvalidValue;
     if (epilogue == EPI_SWIGLU && N % 32) return (int)cudaErrorInvalidValue;
-    if (fp8_skinny_takes(M, N, K, num_sms)) {
+    if (fp8_skinny_takes(M, N, K)) {
         if (epilogue == EPI_STORE) return launch_fp8_skinny<EPI_STORE>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
         if (epilogue == EPI_RESIDUAL) return launch_fp8_skinny<EPI_RESIDUAL>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
         if (epilogue == EPI_SWIGLU) return launch_fp8_skinny<EPI_SWIGLU>(A8, sa, W8, sw, C, R, M, N, K, ldc, ldr, status, num_sms, st);
