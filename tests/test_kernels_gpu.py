@@ -958,3 +958,36 @@ def test_rope_kvwrite_splits_of_blocks(d, hq, hkv):
         close(kv[0], kv[1], 3e-2)
         one = torch.cat([norm(packed, kv[2], slice(t, t + 1)) for t in range(n)])
         assert torch.equal(one, got) and torch.equal(kv[2], kv[0])
+
+
+@pytest.mark.parametrize("parts", [1, 2, 7, 8, 9, 31, 32, 33, 40, 64, 65, 129])
+@pytest.mark.parametrize("d,group", [(64, 1), (128, 4), (256, 2)])
+def test_merge_of_decode_parts(parts, d, group):
+    """Parts of split requests, added up eight and weighed 32 at a time: counts around both, requests of one part (left alone) and of none
+    beside them, parts without a visible key, a plan that ends before the last part, sinks. Against 64 bits: one rounding to bf16 (2^-9)."""
+    import ctypes as C
+    from pie_b200.ops import _lib
+    hkv, max_items = 2, 2 * parts + 2
+    hq = hkv * group
+    g = torch.Generator(device=DEV).manual_seed(parts * 7 + d)
+    counts = [parts, 1, 0, parts, 3]                              # the last one's parts lie beyond max_items in part
+    indptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    o = torch.randn(int(indptr[-1]), hq, d, generator=g, device=DEV)
+    lse = torch.randn(int(indptr[-1]), hq, generator=g, device=DEV) * 4
+    lse[torch.rand(lse.shape, generator=g, device=DEV) < 0.2] = -float("inf")
+    sinks = torch.randn(hq, generator=g, device=DEV)
+    out = torch.full((len(counts), hq, d), 7.0, dtype=torch.bfloat16, device=DEV)
+    ip = torch.from_numpy(indptr).to(DEV)
+    merge = _lib.declare("pie_decode_merge", [C.c_void_p] * 4 + [C.c_int] * 4 + [C.c_void_p, C.c_int, C.c_void_p])
+    assert merge(o.data_ptr(), lse.data_ptr(), ip.data_ptr(), out.data_ptr(), len(counts), hq, hkv, d, sinks.data_ptr(), max_items,
+                 torch.cuda.current_stream().cuda_stream) == 0
+    for r in range(len(counts)):
+        a, b = int(indptr[r]), min(int(indptr[r + 1]), max_items)
+        if b - a <= 1:
+            assert bool((out[r] == 7.0).all())
+            continue
+        w = torch.exp2(lse[a:b].double())
+        total = w.sum(0) + torch.exp2(sinks.double())
+        want = (w[..., None] * o[a:b].double()).sum(0) / total[:, None]
+        want[w.sum(0) == 0] = 0.0
+        torch.testing.assert_close(out[r].double(), want, rtol=2 ** -8, atol=1e-5)
