@@ -256,8 +256,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 // shared memory, four K blocks at a time and seven such chunks ahead.
 //
 // Weights cold, at 8 / 24 / 48 / 64 rows (us): 5120 x 25600 (20.6 at the memory's rate) with two CTAs per SM, block by block,
-// 65 / 74 / 89 / 98, by the kernel above 74 / 74 / 75 / 75, like this 48 / 51 / 56 / 66; 10240 x 5120 17 / 19 / 21 / 23 and 13 / 14 / 15 / 16;
-// 51200 x 5120 42 / 43 / 51 / 57 and 41 / 42 / 45 / 48 (6.4 to 5.5 TB/s); 24576 x 4096 18.1 / 18.8 / 21.8 / 24.2 and 19.0 / 20.1 / 22.2 / 24.4.
+// 65 / 74 / 89 / 98, by the kernel above 74 / 74 / 75 / 75, like this 47 / 51 / 57 / 64; 10240 x 5120 17 / 19 / 21 / 23 and 13 / 14 / 15 / 16;
+// 51200 x 5120 42 / 43 / 51 / 57 and 41 / 42 / 44 / 46 (6.4 to 5.8 TB/s); 24576 x 4096 18.1 / 18.8 / 21.8 / 24.2 and 18.9 / 20.1 / 22.0 / 24.2.
 constexpr int F8S_THREADS = 64 + 256, F8S_CHUNK = 4;
 constexpr uint32_t F8S_MMA_BYTES = GEMM_BM * F8_BK;          // what an MMA reads from a slot's start on
 constexpr uint32_t F8S_BUFS = 2;                               // groups of F8S_CHUNK blocks in tensor memory
@@ -595,7 +595,7 @@ static int fp8_skinny_height(int N, int num_sms) {
 }
 
 // Up to 64 rows run here: the bits of the kernel above in less time wherever measured (1 to 64 rows, 1280 to 51200 features, K from 1024
-// on: 5120 x 1024 4.6 to 6.0 us against 7.2). Fewer features or a shorter K are not worth the set-up.
+// on: 5120 x 1024 3.8 to 5.3 us against 7.2). Fewer features or a shorter K are not worth the set-up.
 static bool fp8_skinny_takes(int M, int N, int K) { return M <= 64 && N >= 128 && K >= 512; }
 
 template <int EPI>
