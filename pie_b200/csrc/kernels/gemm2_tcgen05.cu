@@ -13,11 +13,15 @@
 // gemm_tcgen05.cu; every wait on an mbarrier is bounded. The two cluster-wide barriers (start, end)
 // are reached by every thread on every path.
 //
-// Tiles are whole in K and as wide as makes the rounds of the machine short (plan_pairs), where K used to be split over pairs with the
-// parts parked in global memory: no workspace, one order of sums. (Walking the tiles in bands of row blocks, for operands that L2 holds
-// together, measured no faster.) Weights cold, before and now (us): 512 x 4096 x 14336 80 and 53, 512 x 4096 x 4096 26.4 (on single CTAs)
-// and 18.5, 200 x 2048 x 4096 23.4 and 13.5, 1536 x 4096 x 14336 201 and 137, 3661 x 4096 x 4096 129 and 103; 8300 x 28672 x 4096 1.45 ms
-// either way: 1.3 PFLOP/s, what the power limit allows.
+// Tiles whole in K are as wide as makes the rounds of the machine short (plan_pairs). (Walking them in bands of row blocks, for operands
+// that L2 holds together, measured no faster.) Back to back, weights cold, in tiles of 256 columns or on single CTAs and now (us):
+// 512 x 4096 x 4096 26.4 and 18.5, 200 x 2048 x 4096 23.4 and 13.5, 200 x 49152 x 4096 86 and 82, 300 x 24576 x 4096 86 and 69;
+// 8300 x 28672 x 4096 1.45 ms either way: 1.3 PFLOP/s, what the power limit allows.
+//
+// Large products whose last round of 256-column tiles would be short have K split over the pairs instead, the parts parked in global
+// memory. Whole tiles of another width are faster there (512 x 4096 x 14336 48 us against 62, 1536 x 4096 x 14336 124 against 174), but
+// the tensor cores cut every addition off, and the error of a sum grows with the chain: 1.1e-9 of the result's norm for each of K, of
+// 14336 1.6e-5 whole and 3.1e-6 to 6.0e-6 in parts, 4 to 7 times as much at 4 to 6 parts. 32-bit streams keep that difference.
 #include <algorithm>
 
 #include "gemm_common.cuh"
@@ -36,7 +40,7 @@ template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                   bf16* __restrict__ C, const bf16* __restrict__ R, int M, int N, int K, int ldc, int ldr,
-                  int* status, const __grid_constant__ TpArgs tp, int bn, int stages, const __grid_constant__ EpiArgs ex) {
+                  int* status, const __grid_constant__ TpArgs tp, const StreamKArgs sk, int bn, int stages, const __grid_constant__ EpiArgs ex) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t ring = (raw + 1023u) & ~1023u;
@@ -89,11 +93,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             int s = 0;
             const uint32_t leader_full0 = map_to_cta(full_bar(0), 0);
             pdl_wait();
-            for (int tile = pid; tile < num_tiles && ok; tile += npairs) {
-                const int m_blk = tile % tiles_m, n_blk = tile / tiles_m;
+            SegmentWalk walk(sk.enabled != 0, num_tiles, num_kb, pid, npairs);
+            Segment seg;
+            while (ok && walk.next(seg)) {
+                const int m_blk = seg.tile % tiles_m, n_blk = seg.tile / tiles_m;
                 const int a_row = m_blk * PAIR_M + (int)crank * GEMM_BM, b_row = n_blk * bn + (int)crank * (bn / 2);
                 if (tp.gated && !ag_gate_wait_rows(tp, status, a_row, GEMM_BM, seen)) break;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                for (int kb = seg.kb0; kb < seg.kb1; ++kb, ++it) {
                     if (!mbar_wait_cluster(empty_bar(s), ph ^ 1u, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
                     // both CTAs' loads complete on the leader's barrier, armed for the pair's bytes
                     if (leader) mbar_arrive_expect_tx(full_bar(s), 2 * stage_bytes);
@@ -118,12 +124,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             uint32_t ph = 0, tcount = 0;
             int s = 0;
             bool ok = true;
-            for (int tile = pid; tile < num_tiles && ok; tile += npairs, ++tcount) {
+            SegmentWalk walk(sk.enabled != 0, num_tiles, num_kb, pid, npairs);
+            Segment seg;
+            for (; ok && walk.next(seg); ++tcount) {
                 const uint32_t acc = tcount & 1u, aph = (tcount >> 1) & 1u;
                 if (!mbar_wait_cluster(tempty_bar(acc), aph ^ 1u, status, PIE_ERR_WAIT_EPILOGUE)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * 256;
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
                     if (!mbar_wait_cluster(full_bar(s), ph, status, PIE_ERR_WAIT_TMA)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = ring + s * stage_bytes;
@@ -131,7 +139,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
                     const uint64_t bdesc = make_smem_desc_sw128(a_addr + PAIR_A_BYTES);
 #pragma unroll
                     for (int k = 0; k < GEMM_BK / 16; ++k)
-                        umma_bf16_2cta(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0);
+                        umma_bf16_2cta(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, ((kb - seg.kb0) | k) != 0);
                     umma_commit_2cta(empty_bar(s), 3);   // slot s is free in both CTAs
                     if (++s == stages) { s = 0; ph ^= 1u; }
                 }
@@ -142,25 +150,74 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         // ----------------------------------------------------------- epilogue (own 128 rows)
         const int q = warp & 3, chunks = (bn + 63) / 64;
         uint8_t* stage = ring_ptr + PAIR_RING + 512 + (warp - 2) * 4096;
-        pdl_wait();          // outputs and residual may still be in use by the previous kernel
+        pdl_wait();          // outputs, residual and workspace may still be in use by the previous kernel
         const XieluCoef act(EPI == EPI_XIELU ? ex.act : nullptr);
         const uint32_t leader_tempty0 = map_to_cta(tempty_bar(0), 0);
         const uint32_t leader_tempty1 = map_to_cta(tempty_bar(1), 0);
+        const long long total_units = (long long)num_tiles * num_kb;
+        SegmentWalk walk(sk.enabled != 0, num_tiles, num_kb, pid, npairs);
+        Segment seg;
         uint32_t tcount = 0;
-        for (int tile = pid; tile < num_tiles; tile += npairs, ++tcount) {
-            const int m_blk = tile % tiles_m, n_blk = tile / tiles_m;
+        for (; walk.next(seg); ++tcount) {
+            const int m_blk = seg.tile % tiles_m, n_blk = seg.tile / tiles_m;
             const uint32_t acc = tcount & 1u, aph = (tcount >> 1) & 1u;
             const bool got = mbar_wait_cluster(tfull_bar(acc), aph, status, PIE_ERR_WAIT_MMA);
             if (!__all_sync(0xffffffffu, got)) break;
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256;
             const int row0 = m_blk * PAIR_M + (int)crank * GEMM_BM + q * 32, col0 = n_blk * bn, n_end = min(N, col0 + bn);
+            // Part of a tile: parked in the workspace, and the last pair to arrive for these 32 rows (nobody waits) adds up the tile's
+            // parts, its own among them, in the order of the pairs. Layout of a slot and warp: [chunk of 32 columns][float4][lane].
+            const bool partial = seg.kb0 != 0 || seg.kb1 != num_kb;
+            const size_t slot_floats4 = (size_t)PAIR_M * bn / 4, mine4 = (size_t)((int)crank * 4 + q) * (32 * bn / 4) + lane;
+            bool finalise = true;
+            int c_first = 0, c_last = -1;
+            if (partial) {
+                uint4* park = reinterpret_cast<uint4*>(sk.ws) + (pid + seg.tile) * slot_floats4 + mine4;
 #pragma unroll 1
-            for (int c = 0; c < chunks; ++c) {
+                for (int c = 0; c < bn / 32; ++c) {
+                    uint32_t v[32];
+                    tmem_ld_32x32(t_row + c * 32, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) park[(c * 8 + j) * 32] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                }
+                __threadfence();
+                __syncwarp();
+                c_first = streamk_cta_of((long long)seg.tile * num_kb, total_units, npairs);
+                c_last = streamk_cta_of((long long)(seg.tile + 1) * num_kb - 1, total_units, npairs);
+                int last = 0;
+                if (lane == 0) {
+                    int* ctr = sk.cnt + seg.tile * 8 + (int)crank * 4 + q;
+                    last = atomicAdd(ctr, 1) == c_last - c_first;
+                    if (last) *ctr = 0;
+                }
+                finalise = __shfl_sync(0xffffffffu, last, 0) != 0;
+                if (finalise) __threadfence();
+            }
+#pragma unroll 1
+            for (int c = 0; finalise && c < chunks; ++c) {
                 uint32_t v0[32], v1[32];
                 tmem_ld_32x32(t_row + c * 64, v0);
                 tmem_ld_32x32(t_row + c * 64 + 32, v1);
                 tmem_ld_wait();
+                if (partial) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v0[j] = v1[j] = 0u;
+                    for (int cc = c_first; cc <= c_last; ++cc) {
+                        const float4* part = reinterpret_cast<const float4*>(sk.ws) + (cc + seg.tile) * slot_floats4 + mine4 + (size_t)c * 16 * 32;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float4 a4 = __ldcg(part + j * 32), b4 = __ldcg(part + (8 + j) * 32);
+                            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                v0[4 * j + e] = __float_as_uint(__uint_as_float(v0[4 * j + e]) + a[e]);
+                                v1[4 * j + e] = __float_as_uint(__uint_as_float(v1[4 * j + e]) + b[e]);
+                            }
+                        }
+                    }
+                }
                 epilogue_store_64<EPI>(v0, v1, stage, row0, col0 + c * 64, M, N, C, ldc, R, ldr, tp, n_end, ex, &act);
             }
             tc_fence_before();
@@ -169,7 +226,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
                 if (leader) mbar_arrive(tempty_bar(acc));
                 else mbar_arrive_cluster(acc ? leader_tempty1 : leader_tempty0);
             }
-            if (EPI == EPI_RS) {
+            if (EPI == EPI_RS && finalise) {
                 __threadfence_system();
                 __syncwarp();
                 if (lane == 0) rs_publish_arrival(tp, num_tiles * 8);
@@ -192,6 +249,12 @@ using namespace pie;
 
 extern "C" int pie_make_tma_2d_bf16(CUtensorMap* map, const void* ptr, long rows, long cols, long ld, int box_rows);
 
+// Products whose K is split over pairs, if at all: from 2e10 multiplications on, from 1e10 with a long K. Below, single CTAs may split it.
+bool pie_gemm2_large(int M, int N, int K) {
+    const double macs = (double)M * N * K;
+    return M > GEMM_BM && N >= 128 && (macs >= 2.0e10 || (macs >= 1.0e10 && K >= 8192));
+}
+
 // Tuning aid: tile width of every following launch of more than 128 rows (0: as planned; -1: pairs with the planned width, also where
 // the other kernel would be chosen).
 static int g_pair_bn = 0;
@@ -210,9 +273,26 @@ extern "C" __attribute__((visibility("default"))) int pie_gemm_set_pair_width(in
 //   257 to 384 rows, whose pairs' tiles are up to half empty: 300 x 12352 x 4096 41.7 / 36.0, 320 x 9216 x 512 8.8 / 7.8, but
 //     300 x 4096 x 4096 17.6 / 19.8 and 300 x 5120 x 25600 98 / 134
 //   one row of tiles, and more than one round of them: 200 x 28672 x 4096 83 / 67, but 200 x 18432 x 4096 (one round) 33 / 37
-static bool plan_pairs(int M, int N, int K, int pairs_max, int& width, int& pairs) {
+// Where K is split - on pairs here, or on single CTAs (single_splits: their plan does so) - is a matter of the error of sums and of their
+// order, and stays as it is whatever is the faster way.
+struct PairPlan {
+    int width, pairs, streamk;
+};
+static bool plan_pairs(int M, int N, int K, int pairs_max, long ws_floats, int cnt_ints, bool single_splits, PairPlan& p) {
     if (M <= GEMM_BM || N < 128) return false;
     const long num_kb = (K + GEMM_BK - 1) / GEMM_BK, tiles_m = (M + PAIR_M - 1) / PAIR_M;
+    if (g_pair_bn == 0) {
+        const bool large = pie_gemm2_large(M, N, K);
+        if (!large && single_splits) return false;
+        const int bn = N >= 256 ? 256 : 128;
+        const long tiles = tiles_m * ((N + bn - 1) / bn), rounds = (tiles + pairs_max - 1) / pairs_max;
+        const long pairs = std::min<long>(tiles * num_kb / 16, pairs_max);         // 16 k-blocks per pair or more
+        if (large && pairs >= 1 && tiles % pairs != 0 && tiles <= 2L * pairs_max && (double)tiles / pairs + 0.12 < 0.92 * rounds &&
+            (pairs + tiles) * PAIR_M * bn <= ws_floats && tiles * 8 <= cnt_ints) {
+            p = PairPlan{bn, (int)pairs, 1};
+            return true;
+        }
+    }
     long best = -1, rounds = 0;
     for (int bn = 256; bn >= 64; bn -= 16) {
         if (g_pair_bn > 0 && bn != g_pair_bn) continue;
@@ -221,8 +301,7 @@ static bool plan_pairs(int M, int N, int K, int pairs_max, int& width, int& pair
         if (best >= 0 && cost >= best) continue;
         best = cost;
         rounds = r;
-        width = bn;
-        pairs = (int)std::min<long>(pairs_max, tiles);
+        p = PairPlan{bn, (int)std::min<long>(pairs_max, tiles), 0};
     }
     if (g_pair_bn) return true;
     const long low = tiles_m * ((N + 63) / 64);            // tiles of the least width
@@ -233,39 +312,51 @@ static bool plan_pairs(int M, int N, int K, int pairs_max, int& width, int& pair
 
 template <int EPI>
 static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, void* C, const void* R, int M, int N,
-                        int K, int ldc, int ldr, int* status, int pairs, int bn, cudaStream_t st, const TpArgs& tp,
-                        const EpiArgs& ex) {
+                        int K, int ldc, int ldr, int* status, const PairPlan& p, float* ws, int* cnt, cudaStream_t st,
+                        const TpArgs& tp, const EpiArgs& ex) {
     auto kern = gemm2_bf16_kernel<EPI>;
-    const int stages = std::min<int>(PAIR_MAX_STAGES, PAIR_RING / (PAIR_A_BYTES + bn * GEMM_BK));
+    const int stages = std::min<int>(PAIR_MAX_STAGES, PAIR_RING / (PAIR_A_BYTES + p.width * GEMM_BK));
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM);
     if (e != cudaSuccess) return (int)e;
-    e = launch_pdl(kern, dim3(2 * pairs), dim3(GEMM_THREADS), PAIR_SMEM, st, ta, tb, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
-                   status, tp, bn, stages, ex);
+    const StreamKArgs sk{ws, cnt, p.streamk, 0, nullptr};
+    e = launch_pdl(kern, dim3(2 * p.pairs), dim3(GEMM_THREADS), PAIR_SMEM, st, ta, tb, (bf16*)C, (const bf16*)R, M, N, K, ldc, ldr,
+                   status, tp, sk, p.width, stages, ex);
     return (int)(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+// The plan of a launch: out = {width of the tiles, pairs, K split}. False where the single-CTA kernel takes the product.
+bool pie_gemm2_plan(int M, int N, int K, int num_sms, long ws_floats, int cnt_ints, bool single_splits, int* out) {
+    PairPlan p{};
+    if (num_sms < 2 || !plan_pairs(M, N, K, num_sms / 2, ws_floats, cnt_ints, single_splits, p)) return false;
+    out[0] = p.width;
+    out[1] = p.pairs;
+    out[2] = p.streamk;
+    return true;
 }
 
 // CTA-pair GEMM entry used by the public GEMM functions. Sets *handled = 0 (and launches nothing)
 // when the shape is better served by the single-CTA kernel.
 int pie_gemm2_dispatch(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda,
                        int ldw, int ldc, int ldr, int epilogue, int* status, int num_sms, cudaStream_t st,
-                       const TpArgs* tp_in, int* handled, const EpiArgs& ex) {
+                       const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, bool single_splits, int* handled,
+                       const EpiArgs& ex) {
     *handled = 0;
     if (num_sms < 2) return 0;
-    int bn = 0, pairs = 0;
-    if (!plan_pairs(M, N, K, num_sms / 2, bn, pairs)) return 0;
+    PairPlan p{};
+    if (!plan_pairs(M, N, K, num_sms / 2, ws ? ws_floats : 0, cnt_ints, single_splits, p)) return 0;
     CUtensorMap ta, tb;
     if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
-    if (pie_make_tma_2d_bf16(&tb, W, N, K, ldw, bn / 2) != 0) return (int)cudaErrorInvalidValue;
+    if (pie_make_tma_2d_bf16(&tb, W, N, K, ldw, p.width / 2) != 0) return (int)cudaErrorInvalidValue;
     const TpArgs tp = tp_in ? *tp_in : TpArgs{};
     *handled = 1;
     switch (epilogue) {
-        case EPI_STORE: return launch_gemm2<EPI_STORE>(ta, tb, C, R, M, N, K, ldc, ldr, status, pairs, bn, st, tp, ex);
-        case EPI_RESIDUAL: return launch_gemm2<EPI_RESIDUAL>(ta, tb, C, R, M, N, K, ldc, ldr, status, pairs, bn, st, tp, ex);
-        case EPI_SWIGLU: return launch_gemm2<EPI_SWIGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, pairs, bn, st, tp, ex);
-        case EPI_GEGLU: return launch_gemm2<EPI_GEGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, pairs, bn, st, tp, ex);
-        case EPI_XIELU: return launch_gemm2<EPI_XIELU>(ta, tb, C, R, M, N, K, ldc, ldr, status, pairs, bn, st, tp, ex);
-        case EPI_STREAM: return launch_gemm2<EPI_STREAM>(ta, tb, C, R, M, N, K, ldc, ldr, status, pairs, bn, st, tp, ex);
-        case EPI_RS: return launch_gemm2<EPI_RS>(ta, tb, C, R, M, N, K, ldc, ldr, status, pairs, bn, st, tp, ex);
+        case EPI_STORE: return launch_gemm2<EPI_STORE>(ta, tb, C, R, M, N, K, ldc, ldr, status, p, ws, cnt, st, tp, ex);
+        case EPI_RESIDUAL: return launch_gemm2<EPI_RESIDUAL>(ta, tb, C, R, M, N, K, ldc, ldr, status, p, ws, cnt, st, tp, ex);
+        case EPI_SWIGLU: return launch_gemm2<EPI_SWIGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, p, ws, cnt, st, tp, ex);
+        case EPI_GEGLU: return launch_gemm2<EPI_GEGLU>(ta, tb, C, R, M, N, K, ldc, ldr, status, p, ws, cnt, st, tp, ex);
+        case EPI_XIELU: return launch_gemm2<EPI_XIELU>(ta, tb, C, R, M, N, K, ldc, ldr, status, p, ws, cnt, st, tp, ex);
+        case EPI_STREAM: return launch_gemm2<EPI_STREAM>(ta, tb, C, R, M, N, K, ldc, ldr, status, p, ws, cnt, st, tp, ex);
+        case EPI_RS: return launch_gemm2<EPI_RS>(ta, tb, C, R, M, N, K, ldc, ldr, status, p, ws, cnt, st, tp, ex);
         default: *handled = 0; return (int)cudaErrorInvalidValue;
     }
 }

@@ -120,7 +120,7 @@ struct SegmentWalk {
     long long u, u_end;
     int t, t_step, num_tiles, num_kb;
     bool sk;
-    // worker = CTA index, workers = how many share the problem
+    // worker = CTA (or CTA pair) index, workers = how many share the problem
     __device__ SegmentWalk(bool streamk, int num_tiles_, int num_kb_, int worker, int workers)
         : num_tiles(num_tiles_), num_kb(num_kb_), sk(streamk) {
         if (sk) {

@@ -429,7 +429,10 @@ PIE_API int pie_gemm_set_swap(int max_m) { g_gemm_swap_max_m = max_m; return 0; 
 
 int pie_gemm2_dispatch(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda,
                        int ldw, int ldc, int ldr, int epilogue, int* status, int num_sms, cudaStream_t st,
-                       const TpArgs* tp_in, int* handled, const EpiArgs& ex = EpiArgs());
+                       const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, bool single_splits, int* handled,
+                       const EpiArgs& ex = EpiArgs());
+bool pie_gemm2_large(int M, int N, int K);
+bool pie_gemm2_plan(int M, int N, int K, int num_sms, long ws_floats, int cnt_ints, bool single_splits, int* out);
 
 int pie_gemm_skinny_rows(int N, int K, int num_sms);
 int pie_gemm_skinny(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda, int ldw, int ldc, int ldr,
@@ -526,6 +529,21 @@ PIE_API int pie_gemm_plan(int M, int N, int K, int num_sms, int with_workspace, 
     return 0;
 }
 
+// Which kernel a product of more than 128 rows runs on and how (introspection, tests): out = {1 CTA pairs / 0 single CTAs, tile width,
+// pairs or CTAs, K split}.
+PIE_API int pie_gemm_route(int M, int N, int K, int num_sms, int with_workspace, int* out) {
+    GemmWorkspace w{};
+    if (with_workspace) {
+        w.ws = reinterpret_cast<float*>(16);
+        w.ws_floats = 3L * num_sms * 128 * 256;
+        w.cnt_ints = 2 * num_sms * 4;
+    }
+    const GemmPlan p = plan_gemm(M, N, K, num_sms, 0, w, !pie_gemm2_large(M, N, K));
+    out[0] = pie_gemm2_plan(M, N, K, num_sms, w.ws_floats, w.cnt_ints, p.streamk, out + 1);
+    if (!out[0]) { out[1] = p.bn; out[2] = p.grid; out[3] = p.streamk; }
+    return 0;
+}
+
 // Rows of a tile: the batch spread evenly over its 128-row tiles, whole where one tile holds it.
 static int tile_rows(int M) {
     if (M <= GEMM_BM) return M;
@@ -568,16 +586,17 @@ static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M
     if ((epilogue == EPI_SWIGLU || epilogue == EPI_GEGLU) && N % 32) return (int)cudaErrorInvalidValue;
     GemmWorkspace w;
     if (int rc = current_workspace(&w)) return rc;
-    if (g_gemm_pairs && force_bn == 0) {
+    bool allow_sk = true;
+    if (g_gemm_pairs && force_bn == 0 && M > GEMM_BM) {
+        allow_sk = !pie_gemm2_large(M, N, K);
         int handled = 0;
-        const int rc = pie_gemm2_dispatch(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, status, num_sms, st,
-                                          nullptr, &handled, ex);
+        const int rc = pie_gemm2_dispatch(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, status, num_sms, st, nullptr, w.ws,
+                                          w.ws_floats, w.cnt, w.cnt_ints, plan_gemm(M, N, K, num_sms, 0, w, allow_sk).streamk, &handled, ex);
         if (handled || rc) return rc;
     }
     if (force_bn == 0 && M <= GEMM_BM &&
         (g_gemm_swap_max_m >= 1000 || (M <= g_gemm_swap_max_m && N >= 128 && K >= 512 && M <= pie_gemm_skinny_rows(N, K, num_sms))))
         return pie_gemm_skinny(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, status, num_sms, st, ex);
-    bool allow_sk = true;
     if (force_bn < 0) { allow_sk = false; force_bn = -force_bn == 1 ? 0 : -force_bn; }  // negative: whole-tile only
     if (force_bn > 256 || force_bn % 16) return (int)cudaErrorInvalidValue;
     const GemmPlan plan = plan_gemm(M, N, K, num_sms, force_bn, w, allow_sk);
@@ -665,14 +684,16 @@ PIE_API int pie_gemm_bf16_tp(const void* A, const void* W, void* C, int M, int N
     if (epilogue == EPI_RS && (rows_per_rank % 32 || rows_per_rank <= 0)) return (int)cudaErrorInvalidValue;
     GemmWorkspace w;
     if (int rc = current_workspace(&w)) return rc;
-    if (g_gemm_pairs && force_bn == 0) {
+    bool allow_sk = true;
+    if (g_gemm_pairs && force_bn == 0 && M > GEMM_BM) {
+        allow_sk = !pie_gemm2_large(M, N, K);
         int handled = 0;
-        const int rc = pie_gemm2_dispatch(A, W, C, nullptr, M, N, K, lda, ldw, ldc, 0, epilogue, status, num_sms,
-                                          st, &tp, &handled);
+        const int rc = pie_gemm2_dispatch(A, W, C, nullptr, M, N, K, lda, ldw, ldc, 0, epilogue, status, num_sms, st, &tp, w.ws,
+                                          w.ws_floats, w.cnt, w.cnt_ints, plan_gemm(M, N, K, num_sms, 0, w, allow_sk).streamk, &handled);
         if (handled || rc) return rc;
     }
     if (force_bn < 0 || force_bn > 256 || force_bn % 16) return (int)cudaErrorInvalidValue;
-    const GemmPlan plan = plan_gemm(M, N, K, num_sms, force_bn, w);
+    const GemmPlan plan = plan_gemm(M, N, K, num_sms, force_bn, w, allow_sk);
     const int bn = plan.bn_t(), bm = M < GEMM_BM ? M : GEMM_BM;       // tiles of 128 rows: owners hold multiples of 32
     CUtensorMap ta, tb;
     if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, bm) != 0) return (int)cudaErrorInvalidValue;

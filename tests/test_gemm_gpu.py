@@ -37,11 +37,13 @@ def test_gemm_plain(m, n, k, bn):
 
 
 @pytest.mark.parametrize("m,n,k", [(512, 6144, 4096), (512, 4096, 14336), (512, 768, 4096), (64, 4096, 4096),
-                                   (300, 2048, 8192), (512, 28672, 4096)])
+                                   (300, 2048, 8192), (512, 28672, 4096), (200, 1024, 4096), (1024, 512, 4096)])
 @pytest.mark.parametrize("epi", ["store", "residual", "swiglu"])
 def test_gemm_stream_k_matches_whole_tile_and_reference(m, n, k, epi):
-    """Skinny shapes take the stream-K schedule (split tiles fixed up through the workspace);
-    force_bn=-1 forces whole-tile scheduling of the same kernel."""
+    """Skinny shapes take the stream-K schedule (split tiles fixed up through the workspace), on pairs or on single CTAs;
+    force_bn=-1 is whole-tile scheduling of the single CTAs."""
+    if m > 128 and n <= 4096:
+        assert route(m, n, k)[3] == 1
     x, w = bf(m, k, seed=11), bf(n, k, scale=0.03, seed=12)
     r = bf(m, n, seed=13) if epi == "residual" else None
     e = {"store": ops.EPI_STORE, "residual": ops.EPI_RESIDUAL, "swiglu": ops.EPI_SWIGLU}[epi]
@@ -55,6 +57,65 @@ def test_gemm_stream_k_matches_whole_tile_and_reference(m, n, k, epi):
         want = ref.swiglu_interleaved(want)
     check(y, want, k)
     check(y_dp, want, k)
+
+
+def route(m, n, k):
+    """(CTA pairs or single CTAs, tile width, pairs or CTAs, K split) of a product of more than 128 rows."""
+    out = (ctypes.c_int * 4)()
+    assert _lib.declare("pie_gemm_route", [ctypes.c_int] * 5 + [ctypes.c_void_p])(m, n, k, ops.num_sms(DEV), 1, out) == 0
+    return tuple(out)
+
+
+def product32(x, w, out=None, width=0):
+    """out (0 if not given) + x @ w.T in 32 bits; `width`: in whole tiles of that width on CTA pairs."""
+    out = torch.zeros(x.shape[0], w.shape[0], device=DEV) if out is None else out
+    fn = _lib.declare("pie_gemm_bf16_stream", [ctypes.c_void_p] * 5 + [ctypes.c_int, ctypes.c_void_p] + [ctypes.c_int] * 6 +
+                      [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p])
+    set_width = _lib.declare("pie_gemm_set_pair_width", [ctypes.c_int])
+    ops.ensure_gemm_workspace(DEV)
+    set_width(width)
+    try:
+        assert fn(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), out.data_ptr(), out.stride(0), None, x.shape[0], w.shape[0], x.shape[1],
+                  x.stride(0), w.stride(0), 0, ops.kernel_status(DEV).data_ptr(), ops.num_sms(DEV),
+                  torch.cuda.current_stream().cuda_stream) == 0
+    finally:
+        set_width(0)
+    return out
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 4096, 14336), (256, 5120, 8192), (1030, 6144, 4096), (200, 28672, 4096), (385, 10240, 5120)])
+def test_gemm_pairs_add_up_the_parts_of_a_split_k_in_order(m, n, k):
+    """Large products whose last round of tiles would be short: K split evenly over the pairs. Bit for bit the sum of the parts, each a
+    chain of its own, in their order - the order these products have always had."""
+    assert route(m, n, k) == (1, 256, 74, 1)
+    x, w = bf(m, k, seed=61), bf(n, k, scale=k ** -0.5, seed=62)
+    got = [product32(x, w) for _ in range(2)]              # twice: the arrival counters must be back at zero
+    assert torch.equal(*got)
+    tiles_m, tiles_n, blocks = -(-m // 256), -(-n // 256), -(-k // 64)
+    total = tiles_m * tiles_n * blocks
+    starts = [total * p // 74 for p in range(75)]
+    for tile in {0, tiles_m * tiles_n // 2, tiles_m * tiles_n - 1}:
+        r, c = tile % tiles_m * 256, tile // tiles_m * 256
+        cuts = sorted({tile * blocks, (tile + 1) * blocks, *(s for s in starts if tile * blocks < s < (tile + 1) * blocks)})
+        want = None
+        for a, b in zip(cuts, cuts[1:]):
+            a, b = (a - tile * blocks) * 64, min(k, (b - tile * blocks) * 64)
+            want = product32(x[:, a:b], w[c:c + 256, a:b], want, width=256)
+        assert torch.equal(got[0][r:r + 256, c:c + 256], want[r:r + 256]), tile
+    ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 4096, 14336), (256, 7168, 8192), (129, 4096, 14336), (300, 1024, 8192), (1024, 3072, 8192),
+                                   (640, 512, 4096)])
+def test_gemm_split_k_keeps_the_error_of_its_shorter_chains(m, n, k):
+    """Additions of the tensor cores are cut off, so a sum's error grows with its chain. Products whose K is split, on pairs or on single
+    CTAs, have chains of less than half of K and keep 0.6 of the whole chain's error or less; 300 x 1024 x 8192 has 0.14."""
+    assert route(m, n, k)[3] == 1
+    x, w = bf(m, k, seed=63), bf(n, k, scale=k ** -0.5, seed=64)
+    want = x.double() @ w.double().t()
+    err = [float((y.double() - want).norm()) for y in (product32(x, w), product32(x, w, width=128))]
+    assert err[0] <= 0.6 * err[1]
+    ops.check_kernel_status()
 
 
 def test_gemm_residual():
