@@ -228,7 +228,8 @@ class Capabilities:
         return Capabilities(**d)
 
 
-_SEED_MIX = np.int64(0x9E3779B97F4A7C15 - (1 << 64))
+_SEED_MIX_INT = 0x9E3779B97F4A7C15 - (1 << 64)
+_SEED_MIX = np.int64(_SEED_MIX_INT)
 
 
 def position_seed(seed, position):
@@ -239,3 +240,9 @@ def position_seed(seed, position):
     with np.errstate(over="ignore"):
         out = (np.asarray(seed, dtype=np.int64) * _SEED_MIX) ^ (np.asarray(position, dtype=np.int64) * np.int64(0x632BE5AB))
     return np.where(out == 0, 1, out)
+
+
+def position_seed_of(seed: int, position: int) -> int:
+    """`position_seed` of one seed, in Python's numbers."""
+    mixed = (seed * _SEED_MIX_INT ^ position * 0x632BE5AB) & (1 << 64) - 1
+    return (mixed - (1 << 64) if mixed >> 63 else mixed) or 1

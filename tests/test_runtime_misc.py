@@ -336,3 +336,56 @@ def test_sampler_parameters_of_a_fire_equal_those_worked_out_slot_by_slot():
                 s = drv.slab
                 assert (s.h("temperature", np.float32)[j], s.h("top_k")[j], s.h("top_p", np.float32)[j], s.h("min_p", np.float32)[j],
                         s.h("seeds", np.int64)[j]) == want
+
+
+def _sampler_params_of(specs, rows, positions):
+    from pie_b200.driver.executor import TorchDriver, _Slab
+    from pie_b200.driver.schema import ForwardRequest
+
+    drv = TorchDriver.__new__(TorchDriver)
+    drv.max_rows, drv.rng = 64, np.random.default_rng(7)
+    drv.slab = _Slab({"temperature": 64, "top_k": 64, "top_p": 64, "min_p": 64, "seeds": 128}, "cpu")
+    req = ForwardRequest(tokens=np.zeros(40, np.int32), positions=positions, qo_indptr=np.array([0, 40]), kv_page_indices=None,
+                         kv_page_indptr=None, kv_last_page_lens=None, slot_row=rows, slot_samplers=specs)
+    return drv, req
+
+
+def test_sampler_parameters_of_few_slots_take_few_calls():
+    """A prompt's fire has one token slot: its parameters cost no more calls into numpy than its fields (arrays of them took over thirty)."""
+    import sys
+    from pie_b200.driver.schema import SamplerKind, SamplerSpec
+
+    for seed, most in ((0, 14), (9, 14)):
+        drv, req = _sampler_params_of([SamplerSpec(SamplerKind.TOP_P, 0.8, 0, 0.9, seed=seed)], np.zeros(1, np.int32), np.arange(40, dtype=np.int32))
+        drv._sampler_params(req, None)
+        calls = []
+        sys.setprofile(lambda frame, event, arg: calls.append(arg) if event == "c_call" else None)
+        try:
+            drv._sampler_params(req, None)
+        finally:
+            sys.setprofile(None)
+        assert len(calls) <= most, calls
+
+
+@pytest.mark.parametrize("count", [1, 3, 4, 15, 16, 17, 33])
+def test_sampler_seeds_of_few_and_of_many_slots(count):
+    """Seeds mixed one by one and as an array, drawn one by one and together, are the same; a spec without a seed (None) draws one; only
+    slots with a seed to mix need a row."""
+    from pie_b200.driver.schema import SamplerKind, SamplerSpec, position_seed
+
+    rng = np.random.default_rng(count)
+    positions, rows = rng.integers(0, 1 << 30, 40).astype(np.int32), rng.integers(-3, 45, count).astype(np.int32)
+    given = [int(v) for v in rng.integers(-(2 ** 63), 2 ** 63 - 1, count)]
+    drv, req = _sampler_params_of([SamplerSpec(SamplerKind.MULTINOMIAL, seed=v) for v in given], rows, positions)
+    drv._sampler_params(req, None)
+    want = [int(position_seed(v, int(positions[r]) if 0 <= r < 40 else 0)) for v, r in zip(given, rows)]
+    assert drv.slab.h("seeds", np.int64)[:count].tolist() == want
+    drv, req = _sampler_params_of([SamplerSpec(SamplerKind.MULTINOMIAL, seed=5)] + [SamplerSpec(SamplerKind.MULTINOMIAL, seed=None)] * count,
+                                  rows[:1], positions)
+    drv._sampler_params(req, None)
+    draw = np.random.default_rng(7)
+    want = [int(position_seed(5, int(positions[rows[0]]) if 0 <= rows[0] < 40 else 0))] + [int(draw.integers(1, 2 ** 62)) for _ in range(count)]
+    assert drv.slab.h("seeds", np.int64)[:count + 1].tolist() == want
+    with pytest.raises(OverflowError):
+        drv, req = _sampler_params_of([SamplerSpec(SamplerKind.MULTINOMIAL, seed=2 ** 63)], rows, positions)
+        drv._sampler_params(req, None)
