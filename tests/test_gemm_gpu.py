@@ -37,13 +37,11 @@ def test_gemm_plain(m, n, k, bn):
 
 
 @pytest.mark.parametrize("m,n,k", [(512, 6144, 4096), (512, 4096, 14336), (512, 768, 4096), (64, 4096, 4096),
-                                   (300, 2048, 8192), (512, 28672, 4096), (200, 1024, 4096), (1024, 512, 4096)])
+                                   (300, 2048, 8192), (512, 28672, 4096)])
 @pytest.mark.parametrize("epi", ["store", "residual", "swiglu"])
 def test_gemm_stream_k_matches_whole_tile_and_reference(m, n, k, epi):
-    """Skinny shapes take the stream-K schedule (split tiles fixed up through the workspace), on pairs or on single CTAs;
-    force_bn=-1 is whole-tile scheduling of the single CTAs."""
-    if m > 128 and n <= 4096:
-        assert route(m, n, k)[3] == 1
+    """Skinny shapes take the stream-K schedule (split tiles fixed up through the workspace);
+    force_bn=-1 forces whole-tile scheduling of the same kernel."""
     x, w = bf(m, k, seed=11), bf(n, k, scale=0.03, seed=12)
     r = bf(m, n, seed=13) if epi == "residual" else None
     e = {"store": ops.EPI_STORE, "residual": ops.EPI_RESIDUAL, "swiglu": ops.EPI_SWIGLU}[epi]
@@ -64,6 +62,41 @@ def route(m, n, k):
     out = (ctypes.c_int * 4)()
     assert _lib.declare("pie_gemm_route", [ctypes.c_int] * 5 + [ctypes.c_void_p])(m, n, k, ops.num_sms(DEV), 1, out) == 0
     return tuple(out)
+
+
+@pytest.mark.parametrize("m,n,k,taken", [(200, 1024, 4096, True), (512, 768, 4096, True), (300, 2048, 8192, True), (1024, 512, 4096, True),
+                                         (257, 1536, 4104, True), (512, 4096, 14336, False), (64, 4096, 4096, False)])
+@pytest.mark.parametrize("epi", ["store", "residual", "swiglu"])
+def test_gemm_single_ctas_split_k(m, n, k, taken, epi):
+    """K split evenly over single CTAs, several row tiles or one, parts of two and more CTAs per tile, ragged ends: against the fp32
+    reference and whole tiles of the same kernel. `taken`: the products that run like this by themselves. 32-bit sums of one product
+    differ by their order alone: one rounding to bf16 (2^-9), or two with a GLU's own error, of values near 1."""
+    plan = (ctypes.c_int * 3)()
+    assert _lib.declare("pie_gemm_plan", [ctypes.c_int] * 5 + [ctypes.c_void_p])(m, n, k, ops.num_sms(DEV), 1, plan) == 0
+    assert plan[2] == 1
+    assert not taken or route(m, n, k) == (0, *plan)
+    x, w = bf(m, k, seed=71), bf(n, k, scale=k ** -0.5, seed=72)
+    r = bf(m, n, seed=73) if epi == "residual" else None
+    e = {"store": ops.EPI_STORE, "residual": ops.EPI_RESIDUAL, "swiglu": ops.EPI_SWIGLU}[epi]
+    default = ops.gemm(x, w, residual=r, epilogue=e)
+    ops.set_gemm_pairs(False)
+    ops.set_gemm_swap(0)
+    try:
+        got = [ops.gemm(x, w, residual=r, epilogue=e) for _ in range(3)]        # again: the arrival counters must be back at zero
+        whole = ops.gemm(x, w, residual=r, epilogue=e, force_bn=-1)
+    finally:
+        ops.set_gemm_pairs(True)
+        ops.set_gemm_swap(128)
+    ops.check_kernel_status()
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    assert not taken or torch.equal(got[0], default)
+    want = x.float() @ w.float().t()
+    if epi == "residual":
+        want = want + r.float()
+    if epi == "swiglu":
+        want = ref.swiglu_interleaved(want)
+    for y in (got[0], whole):
+        torch.testing.assert_close(y.float(), want, rtol=2 ** -8, atol=2e-3)
 
 
 def product32(x, w, out=None, width=0):
