@@ -266,20 +266,22 @@ extern "C" __attribute__((visibility("default"))) int pie_gemm_set_pair_width(in
 
 // Width of the tiles: the one whose rounds of the machine take the least time together. A k-block of a tile takes a time that grows with
 // bn + 62 (the 256 rows of A are there whatever the width), a round 500 such units and the last tile's epilogue 10 bn: within 1.5 % of
-// the best of eleven widths over 96 shapes of 200 to 3661 rows. False where single CTAs are the faster ones (us, pairs against single
-// CTAs, weights cold):
-//   few tiles of a long K, which single CTAs split: 200 x 1024 x 4096 12.9 / 11.7, but 320 x 1024 x 4096 (32 tiles) 12.9 / 14.1
-//   two to four tiles of a short K: 200 x 128 x 512 4.5 / 4.1
-//   257 to 384 rows, whose pairs' tiles are up to half empty: 300 x 12352 x 4096 41.7 / 36.0, 320 x 9216 x 512 8.8 / 7.8, but
-//     300 x 4096 x 4096 17.6 / 19.8 and 300 x 5120 x 25600 98 / 134
-//   one row of tiles, and more than one round of them: 200 x 28672 x 4096 83 / 67, but 200 x 18432 x 4096 (one round) 33 / 37
+// the best of thirteen widths over 96 shapes of 200 to 3661 rows.
+//
+// Pairs or single CTAs (in tiles of their plan, `single_bn`): what should take less time, by a fit to 2941 products of 129 to 2305 rows,
+// 128 to 128256 features and a K of 128 to 14336. The faster kernel to 0.5 % in the mean over them, to 2 % for 94 of 100; over 399 more of
+// any size, odd ones among them, 1.2 % and 88 of 100. Pairs against single CTAs, weights cold, back to back (us):
+//   a short K, whose rounds are all start and epilogue: 640 x 65536 x 256 39.8 / 28.4, 1024 x 9216 x 128 11.3 / 8.8, 512 x 9216 x 512 9.0 / 8.3
+//   257 to 384 rows, whose pairs' tiles are up to half empty: 300 x 12288 x 4096 37.9 / 34.2, but 300 x 4096 x 4096 15.7 / 17.4
+//   a last round of either kind that is nearly empty: 640 x 7168 x 2048 18.8 / 16.6, 129 x 24576 x 4096 46.5 / 61.9
 // Where K is split - on pairs here, or on single CTAs (single_splits: their plan does so) - is a matter of the error of sums and of their
 // order, and stays as it is whatever is the faster way.
 struct PairPlan {
     int width, pairs, streamk;
 };
-static bool plan_pairs(int M, int N, int K, int pairs_max, long ws_floats, int cnt_ints, bool single_splits, PairPlan& p) {
+static bool plan_pairs(int M, int N, int K, int num_sms, long ws_floats, int cnt_ints, int single_bn, bool single_splits, PairPlan& p) {
     if (M <= GEMM_BM || N < 128) return false;
+    const int pairs_max = num_sms / 2;
     const long num_kb = (K + GEMM_BK - 1) / GEMM_BK, tiles_m = (M + PAIR_M - 1) / PAIR_M;
     if (g_pair_bn == 0) {
         const bool large = pie_gemm2_large(M, N, K);
@@ -304,10 +306,9 @@ static bool plan_pairs(int M, int N, int K, int pairs_max, long ws_floats, int c
         p = PairPlan{bn, (int)std::min<long>(pairs_max, tiles), 0};
     }
     if (g_pair_bn) return true;
-    const long low = tiles_m * ((N + 63) / 64);            // tiles of the least width
-    if ((K >= 4096 && low <= 16) || (K <= 512 && low <= 4)) return false;
-    if (M > PAIR_M && M <= 3 * GEMM_BM && N >= 6144 && !(rounds == 1 && K >= 8192)) return false;
-    return !(M <= PAIR_M && rounds == 2 && K >= 4096);
+    const long tiles_1 = (long)((M + GEMM_BM - 1) / GEMM_BM) * ((N + single_bn - 1) / single_bn), rounds_1 = (tiles_1 + num_sms - 1) / num_sms;
+    const double single_ns = rounds_1 * (num_kb * (single_bn + 180.) + 800. + 1.5 * single_bn) + 6. * single_bn + 1200.;
+    return rounds * (num_kb * (p.width + 80.) + 1660.) + 20. * p.width < single_ns;
 }
 
 template <int EPI>
@@ -325,9 +326,9 @@ static int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, void* C, c
 }
 
 // The plan of a launch: out = {width of the tiles, pairs, K split}. False where the single-CTA kernel takes the product.
-bool pie_gemm2_plan(int M, int N, int K, int num_sms, long ws_floats, int cnt_ints, bool single_splits, int* out) {
+bool pie_gemm2_plan(int M, int N, int K, int num_sms, long ws_floats, int cnt_ints, int single_bn, bool single_splits, int* out) {
     PairPlan p{};
-    if (num_sms < 2 || !plan_pairs(M, N, K, num_sms / 2, ws_floats, cnt_ints, single_splits, p)) return false;
+    if (num_sms < 2 || !plan_pairs(M, N, K, num_sms, ws_floats, cnt_ints, single_bn, single_splits, p)) return false;
     out[0] = p.width;
     out[1] = p.pairs;
     out[2] = p.streamk;
@@ -338,12 +339,12 @@ bool pie_gemm2_plan(int M, int N, int K, int num_sms, long ws_floats, int cnt_in
 // when the shape is better served by the single-CTA kernel.
 int pie_gemm2_dispatch(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda,
                        int ldw, int ldc, int ldr, int epilogue, int* status, int num_sms, cudaStream_t st,
-                       const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, bool single_splits, int* handled,
-                       const EpiArgs& ex) {
+                       const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, int single_bn, bool single_splits,
+                       int* handled, const EpiArgs& ex) {
     *handled = 0;
     if (num_sms < 2) return 0;
     PairPlan p{};
-    if (!plan_pairs(M, N, K, num_sms / 2, ws ? ws_floats : 0, cnt_ints, single_splits, p)) return 0;
+    if (!plan_pairs(M, N, K, num_sms, ws ? ws_floats : 0, cnt_ints, single_bn, single_splits, p)) return 0;
     CUtensorMap ta, tb;
     if (pie_make_tma_2d_bf16(&ta, A, M, K, lda, GEMM_BM) != 0) return (int)cudaErrorInvalidValue;
     if (pie_make_tma_2d_bf16(&tb, W, N, K, ldw, p.width / 2) != 0) return (int)cudaErrorInvalidValue;

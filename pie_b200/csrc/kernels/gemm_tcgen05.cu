@@ -429,10 +429,10 @@ PIE_API int pie_gemm_set_swap(int max_m) { g_gemm_swap_max_m = max_m; return 0; 
 
 int pie_gemm2_dispatch(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda,
                        int ldw, int ldc, int ldr, int epilogue, int* status, int num_sms, cudaStream_t st,
-                       const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, bool single_splits, int* handled,
-                       const EpiArgs& ex = EpiArgs());
+                       const TpArgs* tp_in, float* ws, long ws_floats, int* cnt, int cnt_ints, int single_bn, bool single_splits,
+                       int* handled, const EpiArgs& ex = EpiArgs());
 bool pie_gemm2_large(int M, int N, int K);
-bool pie_gemm2_plan(int M, int N, int K, int num_sms, long ws_floats, int cnt_ints, bool single_splits, int* out);
+bool pie_gemm2_plan(int M, int N, int K, int num_sms, long ws_floats, int cnt_ints, int single_bn, bool single_splits, int* out);
 
 int pie_gemm_skinny_rows(int N, int K, int num_sms);
 int pie_gemm_skinny(const void* A, const void* W, void* C, const void* R, int M, int N, int K, int lda, int ldw, int ldc, int ldr,
@@ -539,7 +539,7 @@ PIE_API int pie_gemm_route(int M, int N, int K, int num_sms, int with_workspace,
         w.cnt_ints = 2 * num_sms * 4;
     }
     const GemmPlan p = plan_gemm(M, N, K, num_sms, 0, w, !pie_gemm2_large(M, N, K));
-    out[0] = pie_gemm2_plan(M, N, K, num_sms, w.ws_floats, w.cnt_ints, p.streamk, out + 1);
+    out[0] = pie_gemm2_plan(M, N, K, num_sms, w.ws_floats, w.cnt_ints, p.bn, p.streamk, out + 1);
     if (!out[0]) { out[1] = p.bn; out[2] = p.grid; out[3] = p.streamk; }
     return 0;
 }
@@ -589,9 +589,10 @@ static int gemm_bf16(const void* A, const void* W, void* C, const void* R, int M
     bool allow_sk = true;
     if (g_gemm_pairs && force_bn == 0 && M > GEMM_BM) {
         allow_sk = !pie_gemm2_large(M, N, K);
+        const GemmPlan single = plan_gemm(M, N, K, num_sms, 0, w, allow_sk);
         int handled = 0;
         const int rc = pie_gemm2_dispatch(A, W, C, R, M, N, K, lda, ldw, ldc, ldr, epilogue, status, num_sms, st, nullptr, w.ws,
-                                          w.ws_floats, w.cnt, w.cnt_ints, plan_gemm(M, N, K, num_sms, 0, w, allow_sk).streamk, &handled, ex);
+                                          w.ws_floats, w.cnt, w.cnt_ints, single.bn, single.streamk, &handled, ex);
         if (handled || rc) return rc;
     }
     if (force_bn == 0 && M <= GEMM_BM &&
@@ -687,9 +688,10 @@ PIE_API int pie_gemm_bf16_tp(const void* A, const void* W, void* C, int M, int N
     bool allow_sk = true;
     if (g_gemm_pairs && force_bn == 0 && M > GEMM_BM) {
         allow_sk = !pie_gemm2_large(M, N, K);
+        const GemmPlan single = plan_gemm(M, N, K, num_sms, 0, w, allow_sk);
         int handled = 0;
         const int rc = pie_gemm2_dispatch(A, W, C, nullptr, M, N, K, lda, ldw, ldc, 0, epilogue, status, num_sms, st, &tp, w.ws,
-                                          w.ws_floats, w.cnt, w.cnt_ints, plan_gemm(M, N, K, num_sms, 0, w, allow_sk).streamk, &handled);
+                                          w.ws_floats, w.cnt, w.cnt_ints, single.bn, single.streamk, &handled);
         if (handled || rc) return rc;
     }
     if (force_bn < 0 || force_bn > 256 || force_bn % 16) return (int)cudaErrorInvalidValue;
