@@ -248,6 +248,97 @@ def test_gemm_pair_tile_widths(bn, m, n, k, epi):
     torch.testing.assert_close(y.float(), want, rtol=2 ** -8, atol=2e-3)
 
 
+@pytest.mark.parametrize("bn", [64, 80, 112, 144, 176, 208, 256])
+@pytest.mark.parametrize("m,n,k", [(129, 128, 64), (257, 1056, 520), (700, 2080, 1096), (2305, 544, 136)])
+@pytest.mark.parametrize("epi", ["geglu", "xielu", "stream"])
+def test_gemm_pair_tile_widths_of_the_other_epilogues(bn, m, n, k, epi):
+    """As above for the epilogues with an activation or a bias and for the 32-bit stream, whose 128-byte pieces end inside a chunk. Sums of
+    1096 or fewer in 32 bits: 69 additions cut off at 2^-23 of partial sums below 4 are 3.3e-5; bf16 results are one rounding (2^-9), or
+    two with an activation's own error, of values near 1."""
+    from pie_b200.ops import latent as lops
+    x, w, b = bf(m, k, seed=54), bf(n, k, scale=k ** -0.5, seed=55), bf(n, seed=56)
+    act = torch.tensor([0.3, -0.2], dtype=torch.bfloat16, device=DEV)
+    stream = torch.randn(m, n, device=DEV, generator=torch.Generator(device=DEV).manual_seed(57))
+    z = x.double() @ w.double().t()
+    width = _lib.declare("pie_gemm_set_pair_width", [ctypes.c_int])
+    width(bn)
+    try:
+        if epi == "geglu":
+            y, want = ops.gemm(x, w, epilogue=ops.EPI_GEGLU), ref.glu_interleaved(z.float(), "gelu_tanh").double()
+        elif epi == "xielu":
+            y = lops.gemm_xielu(x, w, b, act, torch.full((m, n), 7.0, dtype=torch.bfloat16, device=DEV))
+            z = z + b.double()
+            pos, neg = torch.nn.functional.softplus(act.double())
+            want = torch.where(z > 0, pos * z * z, (0.5 + neg) * (torch.expm1(z) - z)) + 0.5 * z
+        else:
+            y, copy = lops.gemm_stream(x, w, b, stream.clone(), copy=True)
+            want = stream.double() + z + b.double()
+    finally:
+        width(0)
+    ops.check_kernel_status()
+    if epi == "stream":
+        torch.testing.assert_close(y.double(), want, rtol=2 ** -22, atol=3.3e-5)
+        assert torch.equal(copy, y.to(torch.bfloat16))
+    else:
+        torch.testing.assert_close(y.double(), want, rtol=2 ** -8, atol=2e-3)
+
+
+def tp_args(world, rank, rows, n, epoch):
+    """Arguments of a tensor-parallel product on one GPU: every rank's receive buffer and flags are buffers of this GPU, and the flags that
+    the gate looks at are already raised."""
+    t = dict(recv=torch.full((world, world, rows, n), 7.0, dtype=torch.bfloat16, device=DEV),
+             rs_flags=torch.zeros(world, 8, dtype=torch.int32, device=DEV), ag_flags=torch.full((8,), epoch, dtype=torch.int32, device=DEV),
+             counters=torch.tensor([0, 0, 0, epoch], dtype=torch.int32, device=DEV))       # rs_done, rs_epoch, -, ag_epoch
+    blob = ctypes.create_string_buffer(_lib.declare("pie_tp_args_size", [])())
+    fill = _lib.declare("pie_tp_fill_args", [ctypes.c_void_p] * 7 + [ctypes.c_int] * 4)
+    each = lambda x: (ctypes.c_void_p * world)(*[x[i].data_ptr() for i in range(world)])
+    c = t["counters"].data_ptr()
+    assert fill(blob, t["ag_flags"].data_ptr(), c + 12, each(t["recv"]), each(t["rs_flags"]), c, c + 4, world, rank, rows, 0) == 0
+    return blob, t
+
+
+def gemm_tp(x, w, out, epilogue, blob, rows, gated):
+    fn = _lib.declare("pie_gemm_bf16_tp", [ctypes.c_void_p] * 3 + [ctypes.c_int] * 7 + [ctypes.c_void_p] + [ctypes.c_int] * 3 +
+                      [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p])
+    ops.ensure_gemm_workspace(DEV)
+    assert fn(x.data_ptr(), w.data_ptr(), None if out is None else out.data_ptr(), x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0),
+              0 if out is None else out.stride(0), epilogue, blob, rows, gated, 0, ops.kernel_status(DEV).data_ptr(), ops.num_sms(DEV),
+              torch.cuda.current_stream().cuda_stream) == 0
+
+
+@pytest.mark.parametrize("bn,m,n,k", [(64, 129, 128, 64), (80, 700, 1032, 520), (112, 1025, 2080, 264), (176, 385, 4096, 1096), (208, 2305, 520, 136),
+                                      (256, 300, 1000, 512), (0, 512, 4096, 14336), (0, 200, 28672, 4096), (0, 512, 4096, 4096), (0, 200, 1024, 4096)])
+@pytest.mark.parametrize("world", [1, 3])
+def test_gemm_pairs_scatter_rows_to_owners_and_wait_at_the_gate(bn, m, n, k, world):
+    """The tensor-parallel forms on pairs, whole tiles of many widths and K split (width 0: as planned), right behind the product that
+    writes their activations: the rows of every owner are those of the plain product bit for bit, in their place and nowhere else, the
+    last arrival resets its counter and raises the flags; a gate whose flags are up lets the plain product through."""
+    rank, rows = world - 1, -(-m // world // 32) * 32 + 32
+    first, square, w = bf(m, 256, seed=74), bf(k, 256, scale=1 / 16, seed=75), bf(n, k, scale=k ** -0.5, seed=76)
+    blob, t = tp_args(world, rank, rows, n, 5)
+    width = _lib.declare("pie_gemm_set_pair_width", [ctypes.c_int])
+    width(bn)
+    try:
+        want = ops.gemm(ops.gemm(first, square), w)
+        torch.cuda.synchronize()
+        for turn in range(2):
+            gemm_tp(ops.gemm(first, square), w, None, 3, blob, rows, 0)
+        gated = [torch.empty_like(want) for _ in range(2)]
+        for out, owned in zip(gated, (rows, 0)):
+            gemm_tp(ops.gemm(first, square), w, out, ops.EPI_STORE, blob, owned, 1)
+    finally:
+        width(0)
+    torch.cuda.synchronize()
+    ops.check_kernel_status()
+    assert torch.equal(gated[0], want) and torch.equal(gated[1], want)
+    expect = torch.full_like(t["recv"], 7.0)
+    for o in range(world):
+        mine = want[o * rows:(o + 1) * rows]
+        expect[o, rank, :len(mine)] = mine
+    assert torch.equal(t["recv"], expect)
+    assert t["counters"].tolist() == [0, 2, 0, 5] and t["rs_flags"][:, rank].tolist() == [2] * world
+
+
 @pytest.mark.parametrize("m", [1, 7, 64, 65, 100, 128])
 @pytest.mark.parametrize("n,k", [(6144, 4096), (4096, 14336), (1000, 512), (28672, 4096)])
 @pytest.mark.parametrize("epi", ["store", "residual", "swiglu"])
