@@ -583,15 +583,19 @@ PIE_API int pie_gemm_fp8_blockscaled_tp(const void* A8, const float* sa, const v
 
 // Weight rows of a tile: where one round of the machine will do, as many as leave 64 tiles or so - what a round takes hardly depends on
 // its tiles' rows, and more CTAs ask L2 for the same rows of the batch - else as few as leave the rounds as few. Whole quarters of 32 (two
-// warps each), or halves of them where that would end at 128. Measured at 4 / 48 rows (us): 5120 x 25600 in tiles of 24 rows (two rounds)
+// warps each), or parts of them where that would end at 128. Measured at 4 / 48 rows (us): 5120 x 25600 in tiles of 24 rows (two rounds)
 // 91 / 110, of 40 49 / 57, of 64 48 / 56; 6144 x 4096 of 48 12.6 / 13.0, of 64 11.4 / 12.3, of 96 10.1 / 11.6; 8192 x 8192 of 64 19.3 / 21.0, of
-// 128 17.2 / 20.8; 28672 x 4096 of 112 20.5 / 23.1, of 128 21.5 / 23.9; 51200 x 5120 of 88 (four rounds) 42.0 / 50.5, of 128 41.5 / 44.2.
+// 128 17.2 / 20.8; 51200 x 5120 of 88 (four rounds) 42.0 / 50.5, of 128 41.5 / 44.2. At 1 / 64 rows: 28672 x 5120 of 104 24.4 / 29.9, of 112
+// 24.7 / 29.9, of 128 25.8 / 30.2; 57344 x 5120 (four rounds) of 104 45.9 / 55.9, of 112 47.8 / 56.1, of 128 49.1 / 57.9; 24576 x 5120 of 88
+// 22.6 / 29.4, of 96 22.4 / 28.8.
 static int fp8_skinny_height(int N, int num_sms) {
     const int rounds = ((N + GEMM_BM - 1) / GEMM_BM + num_sms - 1) / num_sms;
     int least = (N + rounds * num_sms - 1) / (rounds * num_sms);
     if (rounds == 1) least = std::min(GEMM_BM, std::max(least, (N + 63) / 64));
     const int height = (least + 31) / 32 * 32;
-    return height < GEMM_BM ? height : (least + 15) / 16 * 16;
+    if (height < GEMM_BM) return height;
+    const int step = rounds > 1 ? 8 : 16;
+    return (least + step - 1) / step * step;
 }
 
 // Up to 64 rows run here: the bits of the kernel above in less time wherever measured (1 to 64 rows, 1280 to 51200 features, K from 1024
