@@ -598,9 +598,14 @@ static int fp8_skinny_height(int N, int num_sms) {
     return (least + step - 1) / step * step;
 }
 
-// Up to 64 rows run here: the bits of the kernel above in less time wherever measured (1 to 64 rows, 1280 to 51200 features, K from 1024
-// on: 5120 x 1024 3.8 to 5.3 us against 7.2). Fewer features or a shorter K are not worth the set-up.
-static bool fp8_skinny_takes(int M, int N, int K) { return M <= 64 && N >= 128 && K >= 512; }
+// Up to 64 rows run here, with the bits of the kernel above. Measured over 128 to 51200 features and a K of 512 to 25600, quantiser and
+// product (us, here / above): 1 x 1024 x 1024 4.5 / 6.7, 64 x 1024 x 1024 5.9 / 6.5, 64 x 5120 x 1024 6.5 / 8.1, 16 x 2048 x 8192
+// 19.4 / 21.4, 48 x 2048 x 8192 21.7 / 21.9. With few features a launch takes what one tile's sums over K take, and from 49 rows on these are
+// the longer ones here: 56 x 1024 x 4096 13.7 / 13.3, 64 x 1536 x 2048 9.2 / 8.8, 64 x 2048 x 8192 24.4 / 22.5, and 24.8 / 24.4 with 2560
+// features. Fewer features or a shorter K are not worth the set-up.
+static bool fp8_skinny_takes(int M, int N, int K) {
+    return M <= 64 && N >= 128 && K >= 512 && !(M > 48 && N <= 2048 && K >= 2048);
+}
 
 template <int EPI>
 static int launch_fp8_skinny(const void* A8, const float* sa, const void* W8, const float* sw, void* C, const void* R, int M, int N, int K,

@@ -875,6 +875,19 @@ def test_fp8_gemm_of_small_batches_in_tiles_of_every_height(m, n, k, epi):
     test_fp8_gemm_of_small_batches(m, n, k, epi)
 
 
+@pytest.mark.parametrize("n,k", [(2048, 2048), (2064, 2048), (128, 2064), (2048, 2032)])
+def test_fp8_gemm_rows_are_the_same_on_either_side_of_the_small_batches(n, k):
+    """48 / 49 and 64 / 65 rows, features and K around which products change kernels: a row's bits do not depend on the kernel."""
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    w8 = (torch.randn(n, k, device=DEV, generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    q = ops.Fp8Linear(w8, (torch.rand(n, (k + 127) // 128, device=DEV, generator=g) + 0.5) / 50 * k ** -0.5)
+    x = torch.randn(65, k, device=DEV, generator=g).to(torch.bfloat16)
+    want = ops.gemm_fp8w(x, q, mode="fused")
+    for m in (1, 48, 49, 64):
+        assert torch.equal(ops.gemm_fp8w(x[:m], q, mode="fused"), want[:m]), m
+    ops.check_kernel_status()
+
+
 @pytest.mark.parametrize("vocab", [1024, 32000, 128256, 151936])
 @pytest.mark.parametrize("k,base", [(0, None), (0, 0.3), (0, 0.03), (3000, 0.02)])
 def test_sample_does_not_depend_on_the_batch_or_the_run(vocab, k, base):
