@@ -481,53 +481,78 @@ paged_decode_attn_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
 }
 
 // Merge the partial results of requests that were split into several items, a block per (request, query head), a thread per dimension.
-// Bound by the latency of its loads: part by part the sums took 0.27 us of every part of the longest request. A warp's lanes now load and
-// weigh 32 parts at a time, and eight parts' values are on their way while the eight before are added up, in the parts' order.
-// Attention and merge of one request of 16000 tokens in 63 parts 36 -> 25 us, of 4400 tokens in 18 parts 15.5 -> 12.3 us (8 heads of 128).
+// Bound by the latency of its loads: part by part the sums took 0.27 us of every part of the longest request. A warp's lanes load and
+// weigh 32 parts at a time, and eight parts' values are on their way while the eight before are added up, in the parts' order. Up to four
+// parts are all requested at once and weighed by every thread: with many requests their launch is bound by what a warp issues and by the
+// warps in flight, and the registers of eight parts ahead would halve these (hence ten blocks of 128 per SM).
+// Part by part / 32 at a time without a bound on registers / like this (us; 32 heads of 128): 300 requests of 2 parts 10.5 / 11.6 / 10.6, of 4
+// 12.9 / 13.2 / 11.5, of 8 23.0 / 15.5 / 14.4, 64 of 18 13.5 / 7.2 / 6.3, 1 of 63 12.8 / 4.7 / 4.5; 512 of 2 parts, 8 heads of 256, 8.5 / 10.9 / 7.6.
 template <int D>
-__global__ void __launch_bounds__(D)
+__global__ void __launch_bounds__(D, 1280 / D)
 paged_decode_merge_kernel(const float* __restrict__ o_part, const float* __restrict__ lse_part,
                           const int* __restrict__ req_item_indptr, bf16* __restrict__ out, int hq, int hkv, int group,
                           const float* __restrict__ sinks_log2, int max_items) {
-    constexpr int AHEAD = 8;
+    constexpr int AHEAD = 8, FEW = 4;
     const int req = blockIdx.x, qh = blockIdx.y, lane = threadIdx.x & 31, dim = threadIdx.x;
     pdl_trigger();
     pdl_wait();
     const int a = req_item_indptr[req], n = min(req_item_indptr[req + 1], max_items) - a;
     if (n <= 1) return;
-    const int kvh = qh / group, row = qh - kvh * group;
-    const size_t heads = (size_t)hkv * group, first = (size_t)a * heads + (size_t)kvh * group + row;
-    float next[AHEAD];
-    auto request = [&](int i0) {
+    const int kvh = qh / group, heads = hkv * group;
+    const size_t first = (size_t)a * heads + (size_t)kvh * group + (qh - kvh * group);
+    const float *lse = lse_part + first, *o = o_part + first * D + dim;
+    float M = -INFINITY, L = 0.f, O = 0.f;
+    if (n <= FEW) {
+        float l[FEW], v[FEW];
 #pragma unroll
-        for (int u = 0; u < AHEAD; ++u) next[u] = i0 + u < n ? o_part[(first + (i0 + u) * heads) * D + dim] : 0.f;
-    };
-    request(0);
-    const float lse0 = lane < n ? lse_part[first + lane * heads] : -INFINITY;
-    float M = lse0;
-    for (int i = lane + 32; i < n; i += 32) M = fmaxf(M, lse_part[first + i * heads]);
-    M = warp_max(M);
-    float L = 0.f, O = 0.f;
-    if (M != -INFINITY) {
-        for (int i0 = 0; i0 < n; i0 += 32) {
-            const float lse = i0 == 0 ? lse0 : (i0 + lane < n ? lse_part[first + (i0 + lane) * heads] : -INFINITY);
-            const float weight = exp2f(lse - M);
-            for (int j0 = 0; j0 < 32 && i0 + j0 < n; j0 += AHEAD) {
-                float now[AHEAD];
+        for (int i = 0; i < FEW; ++i) {
+            l[i] = i < n ? lse[(size_t)i * heads] : -INFINITY;
+            v[i] = i < n ? o[(size_t)i * heads * D] : 0.f;
+            M = fmaxf(M, l[i]);
+        }
+        if (M != -INFINITY) {
 #pragma unroll
-                for (int u = 0; u < AHEAD; ++u) now[u] = next[u];
-                if (i0 + j0 + AHEAD < n) request(i0 + j0 + AHEAD);
+            for (int i = 0; i < FEW; ++i) {
+                if (i >= n) break;
+                const float sc = exp2f(l[i] - M);
+                L += sc;
+                O += v[i] * sc;
+            }
+        }
+    } else {
+        float next[AHEAD];
+        auto request = [&](int i0) {
 #pragma unroll
-                for (int u = 0; u < AHEAD; ++u) {
-                    if (i0 + j0 + u >= n) break;
-                    const float sc = __shfl_sync(0xffffffffu, weight, j0 + u);
-                    L += sc;
-                    O += now[u] * sc;
+            for (int u = 0; u < AHEAD; ++u) next[u] = i0 + u < n ? o[(size_t)(i0 + u) * heads * D] : 0.f;
+        };
+        request(0);
+        const float lse0 = lane < n ? lse[(size_t)lane * heads] : -INFINITY;
+        M = lse0;
+#pragma unroll 1
+        for (int i = lane + 32; i < n; i += 32) M = fmaxf(M, lse[(size_t)i * heads]);
+        M = warp_max(M);
+        if (M != -INFINITY) {
+#pragma unroll 1
+            for (int i0 = 0; i0 < n; i0 += 32) {
+                const float weight = exp2f((i0 == 0 ? lse0 : i0 + lane < n ? lse[(size_t)(i0 + lane) * heads] : -INFINITY) - M);
+#pragma unroll 1
+                for (int j0 = 0; j0 < 32 && i0 + j0 < n; j0 += AHEAD) {
+                    float now[AHEAD];
+#pragma unroll
+                    for (int u = 0; u < AHEAD; ++u) now[u] = next[u];
+                    if (i0 + j0 + AHEAD < n) request(i0 + j0 + AHEAD);
+#pragma unroll
+                    for (int u = 0; u < AHEAD; ++u) {
+                        if (i0 + j0 + u >= n) break;
+                        const float sc = __shfl_sync(0xffffffffu, weight, j0 + u);
+                        L += sc;
+                        O += now[u] * sc;
+                    }
                 }
             }
         }
-        if (sinks_log2) L += exp2f(sinks_log2[qh] - M);
     }
+    if (M != -INFINITY && sinks_log2) L += exp2f(sinks_log2[qh] - M);
     out[((size_t)req * hq + qh) * D + dim] = __float2bfloat16(L > 0.f ? O / L : 0.f);
 }
 

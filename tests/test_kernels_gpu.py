@@ -1014,3 +1014,36 @@ def test_merge_of_decode_parts(parts, d, group):
         want = (w[..., None] * o[a:b].double()).sum(0) / total[:, None]
         want[w.sum(0) == 0] = 0.0
         torch.testing.assert_close(out[r].double(), want, rtol=2 ** -8, atol=1e-5)
+
+
+@pytest.mark.parametrize("parts,cut", [(2, 1), (7, 3), (9, 1), (31, 3), (32, 1), (33, 8), (40, 5), (65, 33), (129, 3)])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_merge_of_decode_parts_of_a_plan_that_ends_inside_a_request(parts, cut, sinks):
+    """A plan that holds all but the last parts of a request, also inside 8 and 32 of them: what it holds is merged, and what lies beyond
+    (here numbers that would show) is neither added nor weighed. Against 64 bits: one rounding to bf16 (2^-9)."""
+    import ctypes as C
+    from pie_b200.ops import _lib
+    hkv, group, d = 2, 4, 128
+    hq = hkv * group
+    counts = [parts, 1, 0, parts, parts + 5]
+    indptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    max_items = int(indptr[-1]) - cut
+    g = torch.Generator(device=DEV).manual_seed(parts * 7 + cut)
+    o = torch.randn(int(indptr[-1]), hq, d, generator=g, device=DEV)
+    lse = torch.randn(int(indptr[-1]), hq, generator=g, device=DEV) * 4
+    o[max_items:], lse[max_items:] = 1e30, 100.0
+    sink = torch.randn(hq, generator=g, device=DEV) if sinks else None
+    out = torch.full((len(counts), hq, d), 7.0, dtype=torch.bfloat16, device=DEV)
+    ip = torch.from_numpy(indptr).to(DEV)
+    merge = _lib.declare("pie_decode_merge", [C.c_void_p] * 4 + [C.c_int] * 4 + [C.c_void_p, C.c_int, C.c_void_p])
+    assert merge(o.data_ptr(), lse.data_ptr(), ip.data_ptr(), out.data_ptr(), len(counts), hq, hkv, d, sink.data_ptr() if sinks else None,
+                 max_items, torch.cuda.current_stream().cuda_stream) == 0
+    for r in range(len(counts)):
+        a, b = int(indptr[r]), min(int(indptr[r + 1]), max_items)
+        if b - a <= 1:
+            assert bool((out[r] == 7.0).all())
+            continue
+        w = torch.exp2(lse[a:b].double())
+        total = w.sum(0) + (torch.exp2(sink.double()) if sinks else 0.0)
+        want = (w[..., None] * o[a:b].double()).sum(0) / total[:, None]
+        torch.testing.assert_close(out[r].double(), want, rtol=2 ** -8, atol=1e-5)
