@@ -99,9 +99,11 @@ def test_gemm_single_ctas_split_k(m, n, k, taken, epi):
         torch.testing.assert_close(y.float(), want, rtol=2 ** -8, atol=2e-3)
 
 
-@pytest.mark.parametrize("m,n,k,pairs", [(640, 65536, 256, 0), (1024, 49152, 256, 0), (640, 7168, 128, 0), (385, 18944, 128, 0), (2305, 28672, 256, 0),
+@pytest.mark.parametrize("m,n,k,pairs", [(640, 65536, 256, 0), (1024, 49152, 256, 0), (640, 7168, 128, 0), (385, 18944, 128, 0),
+                                         (2305, 28672, 256, 0),
                                          (512, 9216, 512, 0), (640, 7168, 2048, 0), (300, 12288, 4096, 0), (257, 12288, 2048, 0),
-                                         (129, 24576, 4096, 1), (200, 20480, 4096, 1), (129, 24576, 5120, 1), (300, 4096, 4096, 1), (300, 16384, 4096, 1),
+                                         (129, 24576, 4096, 1), (200, 20480, 4096, 1), (129, 24576, 5120, 1), (300, 4096, 4096, 1),
+                                         (300, 16384, 4096, 1),
                                          (512, 512, 1024, 1), (512, 4096, 4096, 1), (2305, 28672, 4096, 1), (200, 49152, 2048, 1)])
 def test_gemm_products_run_on_the_kernel_that_takes_less_time(m, n, k, pairs):
     """Shapes at which one of the two kernels for more than 128 rows was measured 8 to 40 % faster on 148 SMs; either gives the same bits."""
@@ -306,8 +308,9 @@ def gemm_tp(x, w, out, epilogue, blob, rows, gated):
               torch.cuda.current_stream().cuda_stream) == 0
 
 
-@pytest.mark.parametrize("bn,m,n,k", [(64, 129, 128, 64), (80, 700, 1032, 520), (112, 1025, 2080, 264), (176, 385, 4096, 1096), (208, 2305, 520, 136),
-                                      (256, 300, 1000, 512), (0, 512, 4096, 14336), (0, 200, 28672, 4096), (0, 512, 4096, 4096), (0, 200, 1024, 4096)])
+@pytest.mark.parametrize("bn,m,n,k", [(64, 129, 128, 64), (80, 700, 1032, 520), (112, 1025, 2080, 264), (176, 385, 4096, 1096),
+                                      (208, 2305, 520, 136), (256, 300, 1000, 512), (0, 512, 4096, 14336), (0, 200, 28672, 4096),
+                                      (0, 512, 4096, 4096), (0, 200, 1024, 4096)])
 @pytest.mark.parametrize("world", [1, 3])
 def test_gemm_pairs_scatter_rows_to_owners_and_wait_at_the_gate(bn, m, n, k, world):
     """The tensor-parallel forms on pairs, whole tiles of many widths and K split (width 0: as planned), right behind the product that
