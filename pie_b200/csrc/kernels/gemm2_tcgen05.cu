@@ -15,7 +15,7 @@
 //
 // Tiles whole in K are as wide as makes the rounds of the machine short (plan_pairs). (Walking them in bands of row blocks, for operands
 // that L2 holds together, measured no faster.) Back to back, weights cold, in tiles of 256 columns or on single CTAs and now (us):
-// 512 x 4096 x 4096 26.4 and 18.5, 200 x 2048 x 4096 23.4 and 13.5, 200 x 49152 x 4096 86 and 82, 300 x 24576 x 4096 86 and 69;
+// 512 x 4096 x 4096 23.7 and 16.3, 200 x 2048 x 4096 26.1 and 15.2, 200 x 49152 x 4096 92 and 86;
 // 8300 x 28672 x 4096 1.45 ms either way: 1.3 PFLOP/s, what the power limit allows.
 //
 // Large products whose last round of 256-column tiles would be short have K split over the pairs instead, the parts parked in global

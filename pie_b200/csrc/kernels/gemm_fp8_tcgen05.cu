@@ -255,9 +255,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 // per SM, which also halves the CTAs that ask L2 for the same rows of the batch. The scales of features and tokens come through
 // shared memory, four K blocks at a time and seven such chunks ahead.
 //
-// Weights cold, at 8 / 24 / 48 / 64 rows (us): 5120 x 25600 (20.6 at the memory's rate) with two CTAs per SM, block by block,
-// 65 / 74 / 89 / 98, by the kernel above 74 / 74 / 75 / 75, like this 47 / 51 / 57 / 64; 10240 x 5120 17 / 19 / 21 / 23 and 13 / 14 / 15 / 16;
-// 51200 x 5120 42 / 43 / 51 / 57 and 41 / 42 / 44 / 46 (6.4 to 5.8 TB/s); 24576 x 4096 18.1 / 18.8 / 21.8 / 24.2 and 18.9 / 20.1 / 22.0 / 24.2.
+// Weights cold, at 8 / 24 / 48 / 64 rows (us), with two CTAs per SM and block by block, or by the kernel above where that ran, and like this:
+// 5120 x 25600 (20.6 at the memory's rate) 79 / 87 / 88 / 88 and 47 / 50 / 56 / 64; 10240 x 5120 22 / 29 / 27 / 27 and 13 / 14 / 15 / 16;
+// 51200 x 5120 43 / 46 / 54 / 60 and 42 / 43 / 44 / 45 (6.3 to 5.8 TB/s); 24576 x 4096 18.8 / 20.2 / 23.6 / 25.8 and 19.2 / 20.2 / 22.0 / 24.1.
+// Up to 16 rows in two rounds of tiles are slower than they were by 2 % (24576 x 5120, one row: 22.1 and 22.7) to 4 % (27648 x 2560: 13.8 and
+// 14.3).
 constexpr int F8S_THREADS = 64 + 256, F8S_CHUNK = 4;
 constexpr uint32_t F8S_MMA_BYTES = GEMM_BM * F8_BK;          // what an MMA reads from a slot's start on
 constexpr uint32_t F8S_BUFS = 2;                               // groups of F8S_CHUNK blocks in tensor memory
