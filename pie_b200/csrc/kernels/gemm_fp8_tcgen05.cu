@@ -589,9 +589,12 @@ PIE_API int pie_gemm_fp8_blockscaled_tp(const void* A8, const float* sa, const v
 // 91 / 110, of 40 49 / 57, of 64 48 / 56; 6144 x 4096 of 48 12.6 / 13.0, of 64 11.4 / 12.3, of 96 10.1 / 11.6; 8192 x 8192 of 64 19.3 / 21.0, of
 // 128 17.2 / 20.8; 51200 x 5120 of 88 (four rounds) 42.0 / 50.5, of 128 41.5 / 44.2. At 1 / 64 rows: 28672 x 5120 of 104 24.4 / 29.9, of 112
 // 24.7 / 29.9, of 128 25.8 / 30.2; 57344 x 5120 (four rounds) of 104 45.9 / 55.9, of 112 47.8 / 56.1, of 128 49.1 / 57.9; 24576 x 5120 of 88
-// 22.6 / 29.4, of 96 22.4 / 28.8.
-static int fp8_skinny_height(int N, int num_sms) {
+// 22.6 / 29.4, of 96 22.4 / 28.8. Several rounds of a short K are most of all their tiles' starts and ends, and want few tiles: 27648 x 512 of
+// 96 5.2 / 7.3, of 128 4.8 / 6.2, 27648 x 2048 12.0 / 14.5 and 10.9 / 14.0, 57344 x 1536 of 104 15.6 / 21.2, of 128 15.5 / 20.3, but 57344 x 2048
+// 20.6 / 26.5 and 21.1 / 25.7.
+static int fp8_skinny_height(int N, int K, int num_sms) {
     const int rounds = ((N + GEMM_BM - 1) / GEMM_BM + num_sms - 1) / num_sms;
+    if (rounds > 1 && K <= (rounds == 2 ? 2048 : 1536)) return GEMM_BM;
     int least = (N + rounds * num_sms - 1) / (rounds * num_sms);
     if (rounds == 1) least = std::min(GEMM_BM, std::max(least, (N + 63) / 64));
     const int height = (least + 31) / 32 * 32;
@@ -612,7 +615,7 @@ static bool fp8_skinny_takes(int M, int N, int K) {
 template <int EPI>
 static int launch_fp8_skinny(const void* A8, const float* sa, const void* W8, const float* sw, void* C, const void* R, int M, int N, int K,
                              int ldc, int ldr, int* status, int num_sms, cudaStream_t st) {
-    const int height = fp8_skinny_height(N, num_sms);
+    const int height = fp8_skinny_height(N, K, num_sms);
     CUtensorMap tw, tx;
     if (make_tma_2d_u8(&tw, W8, N, K, K, height) != 0) return (int)cudaErrorInvalidValue;
     if (make_tma_2d_u8(&tx, A8, M, K, K, M) != 0) return (int)cudaErrorInvalidValue;      // the box ends with the batch

@@ -865,11 +865,12 @@ def test_fp8_gemm_of_small_batches(m, n, k, epi):
     torch.testing.assert_close(y.float(), want, rtol=2 ** -8, atol=1e-3)
 
 
-@pytest.mark.parametrize("m,n,k", [(33, 28672, 640), (8, 57344, 512), (33, 7008, 640), (64, 14336, 1168), (24, 4096, 1024),
-                                   (50, 4000, 528), (3, 8192, 1664), (64, 6144, 912), (1, 24576, 528)])
+@pytest.mark.parametrize("m,n,k", [(33, 28672, 2064), (8, 57344, 1552), (33, 7008, 640), (60, 28672, 528), (64, 14336, 1168), (24, 4096, 1024),
+                                   (50, 4000, 528), (3, 8192, 1664), (64, 6144, 912),
+                                   (1, 24576, 2064)])
 @pytest.mark.parametrize("epi", ["store", "residual", "swiglu"])
 def test_fp8_gemm_of_small_batches_in_tiles_of_every_height(m, n, k, epi):
-    """Tiles of 104 and 112 rows (the last quarter live in part, MMA rows that overlap the batch's), of 64 (two quarters) and 96, one to four
+    """Tiles of 104 and 112 rows (the last quarter live in part, MMA rows that overlap the batch's), of 64 (two quarters), 96 and 128, one to four
     per CTA, a last one that is not whole, K blocks that are no multiple of a group: as above, one rounding to bf16 (2^-9) of 32-bit sums in another
     order."""
     test_fp8_gemm_of_small_batches(m, n, k, epi)
